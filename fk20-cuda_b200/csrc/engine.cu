@@ -36,6 +36,7 @@
 #include "consts.cuh"
 #include "launch.h"
 #include "layout.cuh"
+#include "proj_plan.cuh"
 
 using namespace fk;
 
@@ -126,6 +127,75 @@ int current_device_ready() {
     int dev;
     if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return FK20_ENODEV; }
     return ensure_device(dev);
+}
+
+}  // namespace
+
+namespace {
+
+// ---- projection plans (proj_plan.cuh): built once per process and length, then
+// uploaded once per device; kept for the life of the process (0.3 MB at m = 512)
+struct HostPlan {
+    ProjPlan plan;
+    std::vector<uint32_t> progs;  // [muls][PROG_WORDS]
+    double alg_dbl = 0, alg_add = 0;
+    int programs = 0;             // products that are not 0 or +-1
+};
+struct DevPlan {
+    ProjTask *tasks = nullptr;
+    uint32_t *progs = nullptr;
+    uint16_t *out = nullptr;
+};
+
+const HostPlan &host_plan(int log_m, bool half) {
+    static HostPlan plans[2][3];
+    static std::once_flag once[2][3];
+    HostPlan &h = plans[half][log_m - 7];
+    std::call_once(once[half][log_m - 7], [&] {
+        h.plan = host::build_proj_plan(log_m, half);
+        h.progs.resize((size_t)h.plan.muls * PROG_WORDS);
+        for (int k = 0; k < h.plan.muls; k++) {
+            uint32_t *p = &h.progs[(size_t)k * PROG_WORDS];
+            host::make_program(p, h.plan.scalars[k].data());
+            int d = 0, a = 0;
+            host::program_cost(p, &d, &a);
+            h.alg_dbl += d, h.alg_add += a;
+            h.programs += !(p[0] & 0x300u);
+        }
+    });
+    return h;
+}
+
+std::mutex g_plan_mu;
+DevPlan g_dev_plan[64][2][3];
+
+// the plan on the current device `dev`
+int device_plan(int dev, int log_m, bool half, DevPlan *out) {
+    if (dev < 0 || dev >= 64) return FK20_ENODEV;
+    const HostPlan &h = host_plan(log_m, half);
+    std::lock_guard<std::mutex> lk(g_plan_mu);
+    DevPlan &d = g_dev_plan[dev][half][log_m - 7];
+    if (!d.out) {
+        DevPlan n;
+        const size_t tb = h.plan.tasks.size() * sizeof(ProjTask), pb = h.progs.size() * sizeof(uint32_t),
+                     ob = h.plan.out.size() * sizeof(uint16_t);
+        cudaError_t e = cudaMalloc((void **)&n.tasks, tb);
+        if (e == cudaSuccess) e = cudaMalloc((void **)&n.progs, pb);
+        if (e == cudaSuccess) e = cudaMalloc((void **)&n.out, ob);
+        if (e == cudaSuccess) e = cudaMemcpy(n.tasks, h.plan.tasks.data(), tb, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(n.progs, h.progs.data(), pb, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(n.out, h.plan.out.data(), ob, cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            cudaFree(n.tasks);
+            cudaFree(n.progs);
+            cudaFree(n.out);
+            return e == cudaErrorMemoryAllocation ? FK20_ENOMEM : (int)e;
+        }
+        d = n;
+    }
+    *out = d;
+    return 0;
 }
 
 }  // namespace
@@ -373,7 +443,8 @@ struct fk20_ctx {
     int msm_threads = 128;      // MSM block size (64, 128, 256)
     int test_check = 0;         // checked build: MSM launches record a planted failure (tests)
     int fft_blocks_per_sm = 0;  // persistent FFT grid: blocks per SM (0 = as many as fit)
-    int fused_occupancy = 1;    // blocks of the persistent FFT kernel that fit on one SM
+    int fused_occupancy = 1;    // blocks of the cohorts' persistent FFT kernel that fit on one SM
+    int proj_occupancy = 1;     // blocks of the persistent projection kernel that fit on one SM
     unsigned wait_limit = FUSED_SPIN_LIMIT;  // polls before a persistent wait gives up
     unsigned unpublished = 0xffffffffu;      // test hook: a task whose completion is not published
     std::mutex mu;
@@ -392,6 +463,7 @@ namespace {
 
 Tables *tables_for(fk20_ctx *ctx, int log_m) { return (log_m >= 7 && log_m <= 9) ? &ctx->tab[log_m - 7] : nullptr; }
 
+size_t scal_group(int log_m) { return (size_t)(1 << log_m) * L_COLS * SCAL_Q * 32; }  // uint4
 size_t tile_bytes(int G, int m) { return (size_t)G * m * TILE_Q * 32 * sizeof(uint4); }
 size_t scal_bytes(int G, int m) { return (size_t)G * m * L_COLS * SCAL_Q * 32 * sizeof(uint4); }
 
@@ -481,33 +553,24 @@ Work msm_products(int W, int log_m, bool times_m) {
     return w;
 }
 
-// inverse DIF stages 0..L-2, middle (last inverse + zero upper half + first
-// forward stage, optionally times 1/m), forward DIT stages 1..L-1
-int run_hext_to_hfft(Profiler &pf, uint4 *D, int G, int rows, int log_m, int scale, cudaStream_t st) {
-    const int m = 1 << log_m;
-    for (int s = 0; s < log_m - 1; s++) {
-        const Work w = stage_products(rows, log_m, s, 0);
-        pf.begin(FK20_K_STAGE_INV, w.alg, w.exe, st);
-        launch_g1_stage(D, G, log_m, s, 0, st);
-        pf.end(st);
-        CKL();
-    }
-    const Work mid = (Work(ADD_P) + (scale ? prog_products(512 + log_m) : Work())) * ((double)rows * (m / 2));
-    pf.begin(FK20_K_MIDDLE, mid.alg, mid.exe, st);
-    launch_g1_middle(D, G, log_m, scale, st);
-    pf.end(st);
-    CKL();
-    for (int s = 1; s < log_m; s++) {
-        const Work w = stage_products(rows, log_m, s, 1);
-        pf.begin(FK20_K_STAGE_FWD, w.alg, w.exe, st);
-        launch_g1_stage(D, G, log_m, s, 1, st);
-        pf.end(st);
-        CKL();
-    }
-    return 0;
+// the map hext_fft -> h_fft of one row: counted algorithmically as the FFTs it
+// stands for (inverse DIF stages 0..L-2, last inverse butterfly + zeroing +
+// first forward one, forward DIT stages 1..L-1); executed, two instances of
+// the plan's products and additions
+Work proj_products(int log_m, bool half) {
+    Work w;
+    for (int s = 0; s < log_m - 1; s++) w += stage_products(1, log_m, s, 0) + stage_products(1, log_m, s + 1, 1);
+    w += Work(ADD_P) * (double)(1 << (log_m - 1));
+    const HostPlan &h = host_plan(log_m, half);
+    w.exe = 2 * (h.programs * (37.0 * MP + 16.0 * MS_X) + (h.alg_dbl - h.programs) * (2 * MP + 5 * MS_X) +
+                 (h.alg_add - 3 * h.programs) * (8 * MP + 3 * MS_X) + h.plan.lin_products * MP);
+    return w;
 }
 
-int output_launch(Profiler &pf, uint64_t *dst, const uint4 *D, const size_t *row_off, int rows, int log_m,
+size_t arena_bytes(const ProjArena &a) { return (size_t)a.G * a.slots * TILE_Q * 32 * sizeof(uint4); }
+size_t ready_bytes(const ProjArena &a) { return (size_t)a.G * (a.slots + 1) * sizeof(unsigned); }
+
+int output_launch(Profiler &pf, uint64_t *dst, const TileView &D, const size_t *row_off, int rows, int log_m,
                   int bitrev_out, cudaStream_t st) {
     pf.begin(FK20_K_OUTPUT, (double)rows * (1 << log_m) * 3 * MP, (double)rows * (1 << log_m) * 3 * MP, st);
     launch_tile_to_ref(dst, D, row_off, rows, log_m, bitrev_out, st);
@@ -552,6 +615,8 @@ int build_tables(fk20_ctx *ctx, int log_m, const uint64_t *xext, cudaStream_t st
     const int W = (GLV_TABLE_BITS + cb - 1) / cb;
     T->ready = false;
     T->gen++;
+    DevPlan plan;  // the pipeline's plan goes to the device with the tables
+    CKR(device_plan(ctx->device, log_m, false, &plan));
     if (xext != (const uint64_t *)T->xext.p) {  // keep the bases for rebuilds at another window
         CKR(T->xext.reserve((size_t)L_COLS * m * sizeof(g1p_t)));
         CK(cudaMemcpyAsync(T->xext.p, xext, (size_t)L_COLS * m * sizeof(g1p_t), cudaMemcpyDeviceToDevice, st));
@@ -582,7 +647,7 @@ int fingerprint(fk20_ctx *ctx, const void *p, size_t words, unsigned long long *
 
 int msm_launch(fk20_ctx *ctx, Tables *T, uint4 *D, const uint4 *S, int G, int rows, int times_m, cudaStream_t st) {
     MsmArgs a{};
-    a.seg[0] = MsmSeg{D, S, (const uint4 *)T->table.p, G, T->log_m, rows, T->cb, T->W, 0};
+    a.seg[0] = MsmSeg{D, S, (const uint4 *)T->table.p, G, T->log_m, rows, T->cb, T->W, 0, {}, scal_group(T->log_m)};
     a.nseg = 1;
     a.times_m = times_m;
     a.test_check = ctx->test_check;
@@ -610,59 +675,141 @@ constexpr size_t SYNC_HDR = 256;  // persistent-launch header: task counter at 0
 // products), two products to affine, two conversions out of Montgomery form
 constexpr double PROOF_OUT_MP = 575.0;
 
+// Arena slots of the pipeline's plan: the scalar tiles of a row group lie
+// behind the input slots of its (first) group, where nothing is written
+// before the MSM has read them.
+int pipeline_slots(int log_m) {
+    const int need = (int)((scal_group(log_m) + TILE_Q * 32 - 1) / (TILE_Q * 32));
+    return std::max(host_plan(log_m, false).plan.slots, (1 << (log_m - 1)) + need);
+}
+
 struct SegLayout {
     size_t s_off[MAX_SEGS], d_off[MAX_SEGS], r_off[MAX_SEGS];
+    ProjArena arena[MAX_SEGS];
     size_t s_bytes = 0, d_bytes = 0, r_bytes = 0;
+    size_t s_stride[MAX_SEGS];
+    // a segment's arena, scalars inside, and its ready counters (full), or its scalar and point tiles
+    void add(int k, int log_m, unsigned rows, bool full) {
+        const int m = 1 << log_m, G = (int)((rows + 31) / 32);
+        arena[k] = full ? proj_arena(pipeline_slots(log_m), rows) : ProjArena{0, G, 0};
+        s_stride[k] = full ? (size_t)arena[k].slots * TILE_Q * 32 : scal_group(log_m);
+        s_off[k] = s_bytes;
+        if (!full) s_bytes += scal_bytes(G, m);
+        d_off[k] = d_bytes;
+        if (full) s_off[k] = d_bytes + ((size_t)m / 2) * TILE_Q * 32 * sizeof(uint4);
+        d_bytes += full ? arena_bytes(arena[k]) : tile_bytes(G, m);
+        r_off[k] = r_bytes;
+        r_bytes += full ? (ready_bytes(arena[k]) + 255) / 256 * 256 : 0;
+    }
 };
 
-int segment_layout(fk20_ctx *ctx, const Seg *sg, int nseg, SegLayout &lay) {
-    if (nseg < 1 || nseg > MAX_SEGS) return FK20_EINVAL;
+int segment_layout(fk20_ctx *ctx, const Seg *sg, int nseg, bool full, SegLayout &lay) {
+    if (nseg < 1 || nseg > MAX_PROJ_SEGS) return FK20_EINVAL;
     for (int k = 0; k < nseg; k++) {
         Tables *T = tables_for(ctx, sg[k].log_m);
         if (!T) return FK20_EINVAL;
         if (!T->ready) return FK20_ENOSETUP;
-        const int m = 1 << sg[k].log_m, G = (int)((sg[k].rows + 31) / 32);
-        lay.s_off[k] = lay.s_bytes;
-        lay.s_bytes += scal_bytes(G, m);
-        lay.d_off[k] = lay.d_bytes;
-        lay.d_bytes += tile_bytes(G, m);
-        lay.r_off[k] = lay.r_bytes;
-        lay.r_bytes += (size_t)G * m * sizeof(unsigned);
+        lay.add(k, sg[k].log_m, sg[k].rows, full);
     }
     return 0;
 }
 
+// Rows of one segment that one pass takes: an arena holds 24 MB for every 32
+// rows of 4096 coefficients, so longer batches run in passes through one
+// workspace.  1024 rows (780 MB) fill the chip 55 times over in the products.
+constexpr unsigned PASS_ROWS = 1024;
+
 // device buffers of a segment call (a no-op once they are large enough)
 int reserve_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, bool full) {
     SegLayout lay;
-    CKR(segment_layout(ctx, sg, nseg, lay));
+    Seg part[MAX_SEGS];
+    if (nseg < 1 || nseg > MAX_PROJ_SEGS) return FK20_EINVAL;
+    for (int k = 0; k < nseg; k++) part[k] = sg[k], part[k].rows = std::min(sg[k].rows, PASS_ROWS);
+    CKR(segment_layout(ctx, part, nseg, full, lay));
     CKR(ws.init());
-    CKR(ws.S.reserve(lay.s_bytes));
+    if (!full) CKR(ws.S.reserve(lay.s_bytes));
     CKR(ws.D.reserve(lay.d_bytes));
     if (full) CKR(ws.sync.reserve(SYNC_HDR + lay.r_bytes));
     return 0;
 }
 
+// The projection of the arenas D + d_off[k] (inputs stored) on st: one
+// persistent launch, or (staged) one launch per run of independent tasks.
+// `first` clears the error word too; a later pass of the same call keeps it.
+int run_projection(fk20_ctx *ctx, Workspace &ws, const SegLayout &lay, const int *log_m, const unsigned *rows, int nseg,
+                   bool half, bool first, int bps, cudaStream_t st) {
+    ProjArgs p{};
+    const ProjPlan *plans[MAX_PROJ_SEGS];
+    int G[MAX_PROJ_SEGS];
+    Work prod;
+    for (int k = 0; k < nseg; k++) {
+        const HostPlan &h = host_plan(log_m[k], half);
+        DevPlan d;
+        CKR(device_plan(ctx->device, log_m[k], half, &d));
+        plans[k] = &h.plan;
+        G[k] = lay.arena[k].G;
+        p.seg[k] = ProjSeg{(uint4 *)ws.D.p + lay.d_off[k] / sizeof(uint4),
+                           (unsigned *)((char *)ws.sync.p + SYNC_HDR + lay.r_off[k]), d.tasks, d.progs, lay.arena[k],
+                           (int)h.plan.tasks.size(), h.plan.muls, h.plan.muls};
+        prod += proj_products(log_m[k], half) * (double)rows[k];
+    }
+    if (!host::build_proj_runs(p.runs, plans, G, nseg)) return FK20_EINVAL;
+    p.nseg = nseg;
+    p.next = (unsigned *)ws.sync.p;
+    p.err = (int *)((char *)ws.sync.p + 128);
+    p.spin_limit = ctx->wait_limit;
+    p.unpublished = ctx->unpublished;
+    // persistent grid: the context's setting, or the caller's share of the SMs (server packs)
+    int per_sm = ctx->proj_occupancy;
+    const int want = bps > 0 ? bps : ctx->fft_blocks_per_sm;
+    if (want > 0 && want < per_sm) per_sm = want;
+    const auto blocks = [&](unsigned tasks) {
+        return (int)std::min<unsigned>((unsigned)(ctx->sms * per_sm), (tasks + FFT_WARPS - 1) / FFT_WARPS);
+    };
+    if (first) {
+        CK(cudaMemsetAsync(ws.sync.p, 0, SYNC_HDR + lay.r_bytes, st));
+    } else {
+        CK(cudaMemsetAsync(ws.sync.p, 0, 128, st));
+        CK(cudaMemsetAsync((char *)ws.sync.p + SYNC_HDR, 0, lay.r_bytes, st));
+    }
+    ctx->prof.begin(FK20_K_FFT_FUSED, prod.alg, prod.exe, st);
+    if (ctx->fused_fft) {
+        p.first = 0;
+        p.last = p.runs.total;
+        launch_proj(p, blocks(p.runs.total), st);
+        CKL();
+    } else {
+        for (int r = 0; r < p.runs.n; r++) {
+            p.first = p.runs.run[r].start;
+            p.last = r + 1 < p.runs.n ? p.runs.run[r + 1].start : p.runs.total;
+            CK(cudaMemsetAsync(p.next, 0, sizeof(unsigned), st));
+            launch_proj(p, blocks(p.last - p.first), st);
+            CKL();
+        }
+    }
+    ctx->prof.end(st);
+    CK(cudaMemcpyAsync(ws.err_host, p.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    return 0;
+}
+
 // Enqueues the FK20 pipeline of the segments on st: the toeplitz Fr FFTs (one
 // launch per segment), ONE fixed-base MSM launch over all segments, then
-// (full) the G1 inverse + forward transforms as ONE persistent launch over all
-// segments -- or stage by stage when the fused FFT is off -- and the h_fft
-// outputs; or (!full) the hext_fft outputs times m.  The tables are the
-// context's; the workspace is the caller's.  Allocates only when `ws` is too
-// small (reserve_segments first makes the enqueue allocation-free).
-int run_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, const fr_t *polys, void *out, bool full,
-                 cudaStream_t st, bool proofs = false, int fft_bps = 0) {
+// (full) the map hext_fft -> h_fft as ONE persistent launch over all segments
+// -- or level by level when the fused FFT is off -- and the h_fft outputs; or
+// (!full) the hext_fft outputs times m.  The tables are the context's; the
+// workspace is the caller's.  Allocates only when `ws` is too small
+// (reserve_segments first makes the enqueue allocation-free).
+int run_pass(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, const fr_t *polys, void *out, bool full,
+             cudaStream_t st, bool proofs, int fft_bps, bool first) {
     SegLayout lay;
-    CKR(segment_layout(ctx, sg, nseg, lay));
-    CKR(reserve_segments(ctx, ws, sg, nseg, full));
-    if (*ws.err_host) return launch_error(*ws.err_host);  // a previous persistent launch stopped: results invalid
-    uint4 *S = (uint4 *)ws.S.p, *D = (uint4 *)ws.D.p;
+    CKR(segment_layout(ctx, sg, nseg, full, lay));
+    uint4 *D = (uint4 *)ws.D.p, *S = full ? D : (uint4 *)ws.S.p;
     const size_t U = sizeof(uint4);
     for (int k = 0; k < nseg; k++) {
         Tables *T = tables_for(ctx, sg[k].log_m);
         const Work w = fr_fft_products(sg[k].log_m) * ((double)sg[k].rows * L_COLS);
         ctx->prof.begin(FK20_K_TC_FFT, w.alg, w.exe, st);
-        launch_tc_fft(S + lay.s_off[k] / U, (const uint64_t *)polys, sg[k].poly_off, (int)T->n, sg[k].log_m,
+        launch_tc_fft(S + lay.s_off[k] / U, lay.s_stride[k], (const uint64_t *)polys, sg[k].poly_off, (int)T->n, sg[k].log_m,
                       sg[k].rows, st);
         ctx->prof.end(st);
         CKL();
@@ -674,7 +821,8 @@ int run_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, const fr
         Tables *T = tables_for(ctx, sg[k].log_m);
         const int m = 1 << sg[k].log_m, G = (int)((sg[k].rows + 31) / 32);
         a.seg[k] = MsmSeg{D + lay.d_off[k] / U, S + lay.s_off[k] / U, (const uint4 *)T->table.p, G, sg[k].log_m,
-                          (int)sg[k].rows, T->cb, T->W, warps};
+                          (int)sg[k].rows, T->cb, T->W, warps, full ? lay.arena[k] : ProjArena{},
+                          lay.s_stride[k]};
         warps += (unsigned)G * m;
         prod += msm_products(T->W, sg[k].log_m, !full) * ((double)sg[k].rows * m);
     }
@@ -686,56 +834,59 @@ int run_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, const fr
     launch_msm(a, ctx->msm_threads, st);
     ctx->prof.end(st);
     CKL();
-    if (full && ctx->fused_fft) {
-        FusedPlan p{};
-        unsigned widest = 0;
-        prod = Work();
-        for (int k = 0; k < nseg; k++) {
-            const int log_m = sg[k].log_m, m = 1 << log_m, G = (int)((sg[k].rows + 31) / 32);
-            p.seg[k] = FusedSeg{D + lay.d_off[k] / U, (unsigned *)((char *)ws.sync.p + SYNC_HDR + lay.r_off[k])};
-            p.blk.G[k] = G;
-            p.blk.log_m[k] = log_m;
-            widest += (unsigned)G * (m / 2);
-            for (int s = 0; s < log_m - 1; s++)
-                prod += stage_products((int)sg[k].rows, log_m, s, 0) + stage_products((int)sg[k].rows, log_m, s + 1, 1);
-            prod += Work((double)sg[k].rows * (m / 2) * ADD_P);
-        }
-        p.blk.nseg = nseg;
-        fused_blocks_build(p.blk);
-        p.next = (unsigned *)ws.sync.p;
-        p.err = (int *)((char *)ws.sync.p + 128);
-        p.epoch = 1;  // counters are cleared before every launch
-        p.spin_limit = ctx->wait_limit;
-        p.unpublished = ctx->unpublished;
-        // persistent grid: the context's setting, or the caller's share of the SMs (server packs)
-        int per_sm = ctx->fused_occupancy;
-        const int want = fft_bps > 0 ? fft_bps : ctx->fft_blocks_per_sm;
-        if (want > 0 && want < per_sm) per_sm = want;
-        const unsigned max_blocks = (widest + FFT_WARPS - 1) / FFT_WARPS;
-        p.blocks = (int)std::min<unsigned>((unsigned)(ctx->sms * per_sm), max_blocks);
-        CK(cudaMemsetAsync(ws.sync.p, 0, SYNC_HDR + lay.r_bytes, st));
-        ctx->prof.begin(FK20_K_FFT_FUSED, prod.alg, prod.exe, st);
-        launch_g1_fused(p, st);
-        ctx->prof.end(st);
-        CKL();
-        CK(cudaMemcpyAsync(ws.err_host, p.err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    } else if (full) {
-        for (int k = 0; k < nseg; k++)
-            CKR(run_hext_to_hfft(ctx->prof, D + lay.d_off[k] / U, (int)((sg[k].rows + 31) / 32), (int)sg[k].rows,
-                                 sg[k].log_m, 0, st));
+    if (full) {
+        int log_m[MAX_PROJ_SEGS];
+        unsigned rows[MAX_PROJ_SEGS];
+        for (int k = 0; k < nseg; k++) log_m[k] = sg[k].log_m, rows[k] = sg[k].rows;
+        CKR(run_projection(ctx, ws, lay, log_m, rows, nseg, false, first, fft_bps, st));
     }
     for (int k = 0; k < nseg; k++) {
+        TileView v{D + lay.d_off[k] / U, nullptr, lay.arena[k]};
+        if (full) {
+            DevPlan d;
+            CKR(device_plan(ctx->device, sg[k].log_m, false, &d));
+            v.out = d.out;
+        }
         if (proofs) {  // compressed, data-availability order (kernels_out.cu)
             const double po = (double)sg[k].rows * (1 << sg[k].log_m) * PROOF_OUT_MP * MP;
             ctx->prof.begin(FK20_K_OUTPUT, po, po, st);
-            launch_tile_to_proofs((uint8_t *)out, D + lay.d_off[k] / U, sg[k].out_off, (int)sg[k].rows,
+            launch_tile_to_proofs((uint8_t *)out, v, sg[k].out_off, (int)sg[k].rows,
                                   sg[k].log_m, st);
             ctx->prof.end(st);
             CKL();
         } else {
-            CKR(output_launch(ctx->prof, (uint64_t *)out, D + lay.d_off[k] / U, sg[k].out_off, (int)sg[k].rows,
+            CKR(output_launch(ctx->prof, (uint64_t *)out, v, sg[k].out_off, (int)sg[k].rows,
                               sg[k].log_m, 0, st));
         }
+    }
+    return 0;
+}
+
+// run_pass over at most PASS_ROWS rows of each segment at a time
+int run_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, const fr_t *polys, void *out, bool full,
+                 cudaStream_t st, bool proofs = false, int fft_bps = 0) {
+    CKR(reserve_segments(ctx, ws, sg, nseg, full));
+    if (*ws.err_host) return launch_error(*ws.err_host);  // a previous persistent launch stopped: results invalid
+    unsigned most = 0;
+    for (int k = 0; k < nseg; k++) most = std::max(most, sg[k].rows);
+    for (unsigned r0 = 0; r0 < most; r0 += PASS_ROWS) {
+        Seg part[MAX_PROJ_SEGS];
+        int np = 0;
+        const fr_t *in = polys;
+        char *to = (char *)out;
+        for (int k = 0; k < nseg; k++) {
+            if (r0 >= sg[k].rows) continue;
+            Seg s = sg[k];
+            s.rows = std::min(s.rows - r0, PASS_ROWS);
+            const size_t m = (size_t)1 << s.log_m;
+            // contiguous rows come as the only segment of a call
+            if (s.poly_off) s.poly_off += r0;
+            else in += (size_t)r0 * m * (L_COLS / 2);
+            if (s.out_off) s.out_off += r0;
+            else to += (size_t)r0 * m * (proofs ? 48 : sizeof(g1p_t));
+            part[np++] = s;
+        }
+        CKR(run_pass(ctx, ws, part, np, in, to, full, st, proofs, fft_bps, r0 == 0));
     }
     return 0;
 }
@@ -842,7 +993,7 @@ int setup2xext(fk20_ctx *ctx, g1p_t *xext_fft, const g1p_t *setup, unsigned n, c
         launch_g1_stage(D, 1, log_m, s, 1, st);
         CKL();
     }
-    launch_tile_to_ref((uint64_t *)xext_fft, D, nullptr, L_COLS, log_m, 0, st);
+    launch_tile_to_ref((uint64_t *)xext_fft, TileView{D, nullptr, {}}, nullptr, L_COLS, log_m, 0, st);
     CKL();
     return 0;
 }
@@ -860,7 +1011,7 @@ int g1_transform(fk20_ctx *ctx, g1p_t *out, const g1p_t *in, int log_m, unsigned
             launch_g1_stage(D, G, log_m, s, 1, st);
             CKL();
         }
-        launch_tile_to_ref((uint64_t *)out, D, nullptr, (int)count, log_m, 0, st);
+        launch_tile_to_ref((uint64_t *)out, TileView{D, nullptr, {}}, nullptr, (int)count, log_m, 0, st);
         CKL();
     } else {  // natural load, DIF inverse -> bit-reversed, times 1/m, reorder on store
         launch_ref_to_tile(D, (const uint64_t *)in, (int)count, G, log_m, 0, 0, st);
@@ -871,7 +1022,7 @@ int g1_transform(fk20_ctx *ctx, g1p_t *out, const g1p_t *in, int log_m, unsigned
         }
         launch_g1_scale(D, G, log_m, 512 + log_m, st);
         CKL();
-        launch_tile_to_ref((uint64_t *)out, D, nullptr, (int)count, log_m, 1, st);
+        launch_tile_to_ref((uint64_t *)out, TileView{D, nullptr, {}}, nullptr, (int)count, log_m, 1, st);
         CKL();
     }
     return 0;
@@ -895,9 +1046,8 @@ int fk20_test_fail_allocations(int count) {
 int fk20_check_status(int *compiled) {
     if (compiled) *compiled = FK_CHECKED;
     if (cudaDeviceSynchronize() != cudaSuccess) return (int)cudaGetLastError();
-    int v = check_take_msm();
-    const int f = check_take_fft();
-    return v ? v : f;
+    const int v = check_take_msm(), f = check_take_fft(), p = check_take_proj();
+    return v ? v : f ? f : p;
 }
 
 int fk20_ctx_create(fk20_ctx **out, int device, int window) {
@@ -918,6 +1068,7 @@ int fk20_ctx_create(fk20_ctx **out, int device, int window) {
     {
         DeviceGuard dg(device);
         c->fused_occupancy = std::max(1, fused_blocks_per_sm());
+        c->proj_occupancy = std::max(1, proj_blocks_per_sm());
         const int rc = c->ws.init();
         if (rc) {
             delete c;
@@ -1102,7 +1253,8 @@ int fk20_ctx_msm(fk20_ctx *ctx, g1p_t *hext_fft, const fr_t *tc_fft, unsigned ro
     launch_ref_to_scalars((uint4 *)ctx->ws.S.p, (const uint64_t *)tc_fft, (int)rows, log_m, st);
     CKL();
     CKR(msm_launch(ctx, T, (uint4 *)ctx->ws.D.p, (const uint4 *)ctx->ws.S.p, G, (int)rows, 1, st));
-    CKR(output_launch(ctx->prof, (uint64_t *)hext_fft, (const uint4 *)ctx->ws.D.p, nullptr, (int)rows, log_m, 0, st));
+    CKR(output_launch(ctx->prof, (uint64_t *)hext_fft, TileView{(const uint4 *)ctx->ws.D.p, nullptr, {}}, nullptr, (int)rows,
+                      log_m, 0, st));
     return 0;
 }
 
@@ -1347,8 +1499,8 @@ int autotune(fk20_ctx *ctx, int log_m, unsigned rows, size_t max_table_bytes, fk
     // 2. MSM block size, 3. persistent FFT grid, 4. fused vs staged FFT
     for (int t : {64, 128, 256})
         if (!rc && t != best.threads) rc = consider(Cfg{best.window, t, best.bps, best.fused});
-    for (int b = 1; b <= ctx->fused_occupancy && !rc; b++)
-        if (b != (best.bps ? best.bps : ctx->fused_occupancy)) rc = consider(Cfg{best.window, best.threads, b, 1});
+    for (int b = 1; b <= ctx->proj_occupancy && !rc; b++)
+        if (b != (best.bps ? best.bps : ctx->proj_occupancy)) rc = consider(Cfg{best.window, best.threads, b, 1});
     if (!rc) rc = consider(Cfg{best.window, best.threads, best.bps, best.fused ? 0 : 1});
     apply(best);
     cudaStreamSynchronize(st);
@@ -1546,14 +1698,28 @@ int fk20_hext_fft2h_fft(g1p_t *h_fft, const g1p_t *hext_fft, unsigned rows, void
     std::lock_guard<std::mutex> lk(ctx->mu);
     cudaStream_t st = S_(stream);
     const int log_m = 9, m = 512;
-    const int G = (int)((rows + 31) / 32);
-    CKR(ctx->D2.reserve(tile_bytes(G, m)));
-    uint4 *D = (uint4 *)ctx->D2.p;
-    launch_ref_to_tile(D, (const uint64_t *)hext_fft, (int)rows, G, log_m, 0, 0, st);
-    CKL();
-    CKR(run_hext_to_hfft(ctx->prof, D, G, (int)rows, log_m, 1, st));
-    launch_tile_to_ref((uint64_t *)h_fft, D, nullptr, (int)rows, log_m, 0, st);
-    CKL();
+    Workspace &ws = ctx->ws;
+    CKR(ws.init());
+    if (*ws.err_host) return launch_error(*ws.err_host);
+    DevPlan d;
+    CKR(device_plan(ctx->device, log_m, true, &d));
+    const int slots = host_plan(log_m, true).plan.slots;
+    const ProjArena most = proj_arena(slots, std::min(rows, PASS_ROWS));
+    CKR(ws.D.reserve(arena_bytes(most)));
+    CKR(ws.sync.reserve(SYNC_HDR + ready_bytes(most)));
+    for (unsigned r0 = 0; r0 < rows; r0 += PASS_ROWS) {
+        const unsigned n = std::min(rows - r0, PASS_ROWS);
+        SegLayout lay;
+        lay.arena[0] = proj_arena(slots, n);
+        lay.d_off[0] = lay.r_off[0] = 0;
+        lay.r_bytes = ready_bytes(lay.arena[0]);
+        launch_ref_to_arena((uint4 *)ws.D.p, lay.arena[0], (const uint64_t *)(hext_fft + (size_t)r0 * m), (int)n, log_m, st);
+        CKL();
+        CKR(run_projection(ctx, ws, lay, &log_m, &n, 1, true, r0 == 0, 0, st));
+        const TileView v{(const uint4 *)ws.D.p, d.out, lay.arena[0]};
+        launch_tile_to_ref((uint64_t *)(h_fft + (size_t)r0 * m), v, nullptr, (int)n, log_m, 0, st);
+        CKL();
+    }
     return 0;
 }
 
@@ -1756,16 +1922,27 @@ int pinned_reserve(void **p, size_t *have, size_t need) {
     return 0;
 }
 
-// device bytes of a pack with cnt[k] requests of log_m = 7 + k
-size_t pack_bytes(const unsigned cnt[3]) {
-    size_t b = SYNC_HDR + 2 * sizeof(size_t) * (cnt[0] + cnt[1] + cnt[2]);
+// device bytes of a pack with cnt[k] requests of log_m = 7 + k, or of a slot's
+// buffers once it has taken that pack
+size_t pack_bytes(const unsigned cnt[3], const Slot *sl = nullptr) {
+    size_t in = 0, out = 0;
+    SegLayout lay;
     for (int k = 0; k < 3; k++) {
         if (!cnt[k]) continue;
-        const int m = 128 << k, G = (int)((cnt[k] + 31) / 32);
-        b += (size_t)cnt[k] * ((size_t)m * 8 * sizeof(fr_t) + (size_t)m * sizeof(g1p_t));
-        b += scal_bytes(G, m) + tile_bytes(G, m) + (size_t)G * m * sizeof(unsigned);
+        const int m = 128 << k;
+        in += (size_t)cnt[k] * m * 8 * sizeof(fr_t);
+        out += (size_t)cnt[k] * m * sizeof(g1p_t);
+        lay.add(k, 7 + k, std::min(cnt[k], PASS_ROWS), true);
     }
-    return b;
+    size_t offs = 2 * sizeof(size_t) * (cnt[0] + cnt[1] + cnt[2]), sync = SYNC_HDR + lay.r_bytes, D = lay.d_bytes;
+    if (sl) {  // buffers only grow
+        in = std::max(in, sl->dpoly.bytes);
+        out = std::max(out, sl->dout.bytes);
+        offs = std::max(offs, sl->ws.offs.bytes);
+        sync = std::max(sync, sl->ws.sync.bytes);
+        D = std::max(D, sl->ws.D.bytes);
+    }
+    return in + out + offs + sync + D;
 }
 
 }  // namespace
@@ -1870,11 +2047,11 @@ int enqueue_pack(fk20_server *s, Slot &sl, bool latency) {
         // time); a throughput-mode pack takes 1/slots of the SMs, so packs of
         // different slots run side by side and hide each other's dependency
         // waits.
-        int share = ctx->fused_occupancy;
+        int share = ctx->proj_occupancy;
         if (s->cfg.fft_blocks_per_sm)
-            share = std::min((int)s->cfg.fft_blocks_per_sm, ctx->fused_occupancy);
+            share = std::min((int)s->cfg.fft_blocks_per_sm, ctx->proj_occupancy);
         else if (!latency)
-            share = std::max(1, ctx->fused_occupancy / (int)s->slots.size());
+            share = std::max(1, ctx->proj_occupancy / (int)s->slots.size());
         CKR(run_segments(ctx, sl.ws, sg, nseg, (const fr_t *)sl.dpoly.p, (g1p_t *)sl.dout.p, true, sl.st, false,
                          share));
     }
@@ -1959,7 +2136,7 @@ void server_main(fk20_server *s) {
                 const int k = log_m_for_n(r.n) - 7;
                 unsigned c2[3] = {cnt[0], cnt[1], cnt[2]};
                 c2[k]++;
-                const size_t need = std::max(fs->bytes(), pack_bytes(c2));
+                const size_t need = pack_bytes(c2, fs);
                 if (need > fs->bytes() && !asked) {
                     asked = true;
                     size_t fr = 0, tot = 0;
@@ -1999,6 +2176,16 @@ void server_main(fk20_server *s) {
                 // for one of them to complete; alone, it never fits
                 bool busy = false;
                 for (Slot &sl : s->slots) busy |= !sl.reqs.empty();
+                // ... unless idle slots hold buffers grown for other packs:
+                // they are given back first
+                bool held = false;
+                if (!busy)
+                    for (Slot &sl : s->slots) {
+                        held |= sl.bytes() > 0;
+                        sl.ws.D.release(), sl.ws.offs.release(), sl.ws.sync.release();
+                        sl.dpoly.release(), sl.dout.release();
+                    }
+                if (held) continue;
                 if (!busy) {
                     s->finished[s->queue.front().ticket] = FK20_ENOMEM;
                     s->nomem++;
@@ -2070,11 +2257,11 @@ int cohort_msm(fk20_server *s, const std::vector<int> &fresh) {
         const int m = 1 << c.log_m, n = m * 8;
         Tables *T = tables_for(ctx, c.log_m);
         CK(cudaMemcpyAsync(b.dpoly.p, b.hpoly, (size_t)c.rows * n * sizeof(fr_t), cudaMemcpyHostToDevice, st));
-        launch_tc_fft((uint4 *)b.S.p, (const uint64_t *)b.dpoly.p, nullptr, n, c.log_m, (unsigned)c.rows, st);
+        launch_tc_fft((uint4 *)b.S.p, scal_group(c.log_m), (const uint64_t *)b.dpoly.p, nullptr, n, c.log_m, (unsigned)c.rows, st);
         CKL();
         CK(cudaMemsetAsync(b.ready.p, 0, (size_t)c.G * m * sizeof(unsigned), st));
         a.seg[k] = MsmSeg{(uint4 *)b.D.p, (const uint4 *)b.S.p, (const uint4 *)T->table.p, c.G, c.log_m, c.rows,
-                          T->cb, T->W, warps};
+                          T->cb, T->W, warps, {}, scal_group(c.log_m)};
         warps += (unsigned)c.G << c.log_m;
     }
     a.nseg = (int)fresh.size();
@@ -2127,7 +2314,7 @@ int cohort_launch(fk20_server *s, const std::vector<int> &act) {
         c.stage = p.blk.s_hi[k];
         if (c.stage < 2 * c.log_m - 1) continue;
         const int m = 1 << c.log_m;
-        launch_tile_to_ref((uint64_t *)b.dout.p, (const uint4 *)b.D.p, nullptr, c.rows, c.log_m, 0, st);
+        launch_tile_to_ref((uint64_t *)b.dout.p, TileView{(const uint4 *)b.D.p, nullptr, {}}, nullptr, c.rows, c.log_m, 0, st);
         CKL();
         CK(cudaMemcpyAsync(b.hout, b.dout.p, (size_t)c.rows * m * sizeof(g1p_t), cudaMemcpyDeviceToHost, st));
         CK(cudaEventRecord(b.out_done, st));
@@ -2481,14 +2668,8 @@ int fk20_server_create(fk20_server **out, fk20_ctx *ctx, const fk20_server_confi
                 if (!rc) rc = sl.ws.offs.reserve(2 * (size_t)(cap + 64) * sizeof(size_t));
                 if (!rc) {
                     SegLayout lay;
-                    for (int k = 0; k < 3 && !rc; k++) {
-                        const int m = 1 << sg[k].log_m, G = (int)((sg[k].rows + 31) / 32);
-                        lay.s_bytes += scal_bytes(G, m);
-                        lay.d_bytes += tile_bytes(G, m);
-                        lay.r_bytes += (size_t)G * m * sizeof(unsigned);
-                    }
-                    rc = sl.ws.S.reserve(lay.s_bytes);
-                    if (!rc) rc = sl.ws.D.reserve(lay.d_bytes);
+                    for (int k = 0; k < 3; k++) lay.add(k, sg[k].log_m, std::min(sg[k].rows, PASS_ROWS), true);
+                    rc = sl.ws.D.reserve(lay.d_bytes);
                     if (!rc) rc = sl.ws.sync.reserve(SYNC_HDR + lay.r_bytes);
                 }
             }

@@ -523,7 +523,7 @@ FK_HD void f_pow(Elem<F> &r, const Elem<F> &a, const uint32_t *e, int nw) {
 
 // inverse by Fermat's little theorem, a^(m-2); inv(0) = 0
 template <class F>
-FK_HD void f_inv(Elem<F> &r, const Elem<F> &a) {
+FK_HD void f_inv_pow(Elem<F> &r, const Elem<F> &a) {
     uint32_t e[F::N];
     uint64_t br = 2;
 #pragma unroll
@@ -533,6 +533,123 @@ FK_HD void f_inv(Elem<F> &r, const Elem<F> &a) {
         br = d >> 63;
     }
     f_pow<F>(r, a, e, F::N);
+}
+
+// Fp inverse by division steps (Bernstein and Yang, "Fast constant-time gcd
+// computation and modular inversion", 2019): 30 steps at a time on the low
+// words give a 2 x 2 matrix, which then updates f, g (the gcd pair, starting
+// at p and a) and d, e (f = d a / c, g = e a / c mod p throughout, starting
+// at 0 and c) by exact divisions by 2^30.  Numbers are 13 signed limbs of 30
+// bits.  c = R^2 makes the result a^-1 R for a Montgomery-form input a R.
+// Theorem 11.2 of the paper: g = 0 after (49 * 381 + 57) / 17 = 1101 steps, 37
+// rounds; the loop ends as soon as g is 0 (25 rounds on average).  |d| and |e|
+// grow by at most p / 2 a round and fit.  About 20,000 instructions against
+// 320,000 for a^(p-2) (381 squares and ~190 products): one inverse per point
+// of an output costs less than sharing a slow one did.
+struct Limbs30 {
+    int32_t v[13];
+};
+FK_HD int32_t l30_word(const uint32_t *w, int i) {  // bits 30 i .. 30 i + 29 of 12 words
+    const int bit = 30 * i, k = bit >> 5, s = bit & 31;
+    uint64_t x = w[k];
+    if (k + 1 < 12) x |= (uint64_t)w[k + 1] << 32;
+    return (int32_t)((uint32_t)(x >> s) & 0x3fffffffu);
+}
+FK_HD void l30_matrix(int32_t &delta, uint32_t f, uint32_t g, int32_t t[4]) {
+    int32_t u = 1, v = 0, q = 0, r = 1;
+#pragma unroll 1
+    for (int i = 0; i < 30; i++) {
+        const bool odd = g & 1, swap = odd && delta > 0;
+        const uint32_t f0 = f, g0 = g;
+        const int32_t u0 = u, v0 = v, q0 = q, r0 = r;
+        f = swap ? g0 : f0;
+        u = swap ? q0 : u0;
+        v = swap ? r0 : v0;
+        g = odd ? g0 + (swap ? 0u - f0 : f0) : g0;
+        q = odd ? q0 + (swap ? -u0 : u0) : q0;
+        r = odd ? r0 + (swap ? -v0 : v0) : r0;
+        delta = (swap ? -delta : delta) + 1;
+        g >>= 1;
+        u = (int32_t)((uint32_t)u << 1);
+        v = (int32_t)((uint32_t)v << 1);
+    }
+    t[0] = u, t[1] = v, t[2] = q, t[3] = r;
+}
+FK_HD void fp_inv_steps(Elem<FpDesc> &res, const Elem<FpDesc> &a) {
+    constexpr int32_t M = 0x3fffffff;
+    Limbs30 f, g, d, e, p;
+    uint32_t pw[12], cw[12];
+#pragma unroll
+    for (int i = 0; i < 12; i++) pw[i] = FpDesc::mod(i), cw[i] = FpDesc::r2(i);
+#pragma unroll
+    for (int i = 0; i < 13; i++) {
+        p.v[i] = f.v[i] = l30_word(pw, i);
+        g.v[i] = l30_word(a.w, i);
+        d.v[i] = 0;
+        e.v[i] = l30_word(cw, i);
+    }
+    int32_t delta = 1;
+#pragma unroll 1
+    for (int round = 0; round < 37; round++) {
+        int32_t t[4];
+        // the low 30 bits decide 30 steps
+        l30_matrix(delta, (uint32_t)f.v[0] | ((uint32_t)f.v[1] << 30), (uint32_t)g.v[0] | ((uint32_t)g.v[1] << 30), t);
+        const int64_t u = t[0], v = t[1], q = t[2], r = t[3];
+        int64_t cf = u * f.v[0] + v * g.v[0], cg = q * f.v[0] + r * g.v[0];
+        cf >>= 30;
+        cg >>= 30;
+        int64_t cd = u * d.v[0] + v * e.v[0], ce = q * d.v[0] + r * e.v[0];
+        // the multiples of p (centred) that make the low 30 bits vanish
+        int32_t md = (int32_t)(((uint32_t)cd * FpDesc::M0) << 2) >> 2, me = (int32_t)(((uint32_t)ce * FpDesc::M0) << 2) >> 2;
+        cd = (cd + (int64_t)md * p.v[0]) >> 30;
+        ce = (ce + (int64_t)me * p.v[0]) >> 30;
+        int32_t any = 0;
+#pragma unroll
+        for (int i = 1; i < 13; i++) {
+            cf += u * f.v[i] + v * g.v[i];
+            cg += q * f.v[i] + r * g.v[i];
+            cd += u * d.v[i] + v * e.v[i] + (int64_t)md * p.v[i];
+            ce += q * d.v[i] + r * e.v[i] + (int64_t)me * p.v[i];
+            f.v[i - 1] = (int32_t)cf & M;
+            g.v[i - 1] = (int32_t)cg & M;
+            d.v[i - 1] = (int32_t)cd & M;
+            e.v[i - 1] = (int32_t)ce & M;
+            any |= g.v[i - 1];
+            cf >>= 30, cg >>= 30, cd >>= 30, ce >>= 30;
+        }
+        f.v[12] = (int32_t)cf, g.v[12] = (int32_t)cg, d.v[12] = (int32_t)cd, e.v[12] = (int32_t)ce;
+        if ((any | g.v[12]) == 0) break;
+    }
+    // f = +-1 (or a = 0: f = +-p, d = 0 mod p): the inverse is f d, brought into [0, p)
+    int32_t neg = f.v[12] >> 31;
+#pragma unroll 1
+    for (int k = 0; k < 96; k++) {
+        int64_t c = 0;
+        Limbs30 s;
+#pragma unroll
+        for (int i = 0; i < 13; i++) {
+            // first -d where f < 0, then d + p while negative, d - p while that is not negative
+            c += k == 0 ? (neg ? -(int64_t)d.v[i] : (int64_t)d.v[i]) : (int64_t)d.v[i] + (d.v[12] < 0 ? p.v[i] : -p.v[i]);
+            s.v[i] = i < 12 ? (int32_t)c & M : (int32_t)c;
+            c >>= 30;
+        }
+        const bool done = k > 0 && d.v[12] >= 0 && s.v[12] < 0;  // 0 <= d < p
+        if (done) break;
+        d = s;
+    }
+#pragma unroll
+    for (int i = 0; i < 12; i++) {
+        const int bit = 32 * i, k = bit / 30, sft = bit % 30;
+        uint64_t x = (uint64_t)(uint32_t)d.v[k] >> sft;
+        x |= (uint64_t)(uint32_t)d.v[k + 1] << (30 - sft);
+        if (k + 2 < 13) x |= (uint64_t)(uint32_t)d.v[k + 2] << (60 - sft);
+        res.w[i] = (uint32_t)x;
+    }
+}
+template <class F>
+FK_HD void f_inv(Elem<F> &r, const Elem<F> &a) {
+    if constexpr (F::N == 12) fp_inv_steps(r, a);
+    else f_inv_pow<F>(r, a);
 }
 
 }  // namespace fk

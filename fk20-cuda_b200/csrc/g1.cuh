@@ -158,6 +158,63 @@ FK_HD void g1_add_q(G1P &R, const G1P &P, const QT &Q, bool negQ) {
 // R = P + Q (RCB Algorithm 7, 12 M + 2 m_3b)
 FK_HD void g1_add(G1P &R, const G1P &P, const G1P &Q) { g1_add_q(R, P, RegPoint{Q}, false); }
 
+// P + Q and P - Q together: Algorithm 7 twice with the products that do not
+// depend on Q's sign shared (X1X2, Y1Y2, Z1Z2, X1Z2 + X2Z1 and the Y
+// coordinate, which is the same for both): 18 M instead of 24.  Each result
+// coordinate goes to st(0 sum / 1 difference, coordinate, value) as soon as it
+// is known.
+template <class QT, class ST>
+FK_HD void g1_addsub_q(const G1P &P, const QT &Q, const ST &st) {
+    Fp t0, t1, t2, a, b, c, d, s, q, t;
+    Q.get(0, q);
+    fp_mul(t0, P.x, q);
+    fp_mul(b, P.y, q);
+    Q.get(2, t);
+    fp_mul(t2, P.z, t);
+    fp_mul(c, P.y, t);
+    f_add(q, q, t);
+    f_add(t, P.x, P.z);
+    fp_mul(s, t, q);
+    f_sub(s, s, t0);
+    f_sub(s, s, t2);         // X1 Z2 + X2 Z1
+    Q.get(1, q);
+    fp_mul(t1, P.y, q);
+    fp_mul(a, P.x, q);
+    fp_mul(d, P.z, q);
+    f_mul12(s, s);
+    f_add(t, t0, t0);
+    f_add(t0, t, t0);        // 3 X1 X2
+    f_mul12(t2, t2);
+    f_add(q, t1, t2);        // Y1 Y2 + b3 Z1 Z2
+    f_sub(t1, t1, t2);       // Y1 Y2 - b3 Z1 Z2
+    fp_mul(t, t1, q);
+    fp_mul(t2, s, t0);
+    f_add(t, t, t2);
+    st(0, 1, t);
+    st(1, 1, t);
+    f_sub(t2, b, a);
+    f_add(a, b, a);          // X1 Y2 + X2 Y1 (t2: its counterpart for -Q)
+    f_sub(b, c, d);
+    f_add(c, c, d);          // Y1 Z2 + Y2 Z1 (b: its counterpart for -Q)
+    fp_mul(t, a, t1);
+    fp_mul(d, c, s);
+    f_sub(t, t, d);
+    st(0, 0, t);
+    fp_mul(t, q, c);
+    fp_mul(d, t0, a);
+    f_add(t, t, d);
+    st(0, 2, t);
+    fp_mul(t, t2, q);
+    fp_mul(d, b, s);
+    f_add(t, t, d);
+    f_neg(t, t);
+    st(1, 0, t);
+    fp_mul(t, t0, t2);
+    fp_mul(d, t1, b);
+    f_sub(t, t, d);
+    st(1, 2, t);
+}
+
 // R = P + (qx, qy) with Q affine and not infinity (RCB Algorithm 8, 11 M + 2 m_3b)
 FK_HD void g1_madd(G1P &R, const G1P &P, const Fp &qx, const Fp &qy) {
     Fp t0, t1, t2, t3, t4, X3, Y3, Z3;
@@ -375,6 +432,19 @@ FK_HD constexpr uint32_t beta_mont(int i) {
     return i == 0 ? 0x8671f071u : i == 1 ? 0xcd03c9e4u : i == 2 ? 0x1fcda5d2u : i == 3 ? 0x5dab2246u
          : i == 4 ? 0xd3851b95u : i == 5 ? 0x587042afu : i == 6 ? 0x01bacb9eu : i == 7 ? 0x8eb60ebeu
          : i == 8 ? 0x83d050d2u : i == 9 ? 0x03f97d6eu : i == 10 ? 0x54638741u : 0x18f02065u;
+}
+
+// beta^2 = -1 - beta (Montgomery form)
+FK_HD void fp_mul_beta(Fp &r, const Fp &x, int power) {
+    Fp beta, t;
+#pragma unroll
+    for (int i = 0; i < 12; i++) beta.w[i] = beta_mont(i);
+    fp_mul(t, x, beta);
+    if (power == 2) {
+        f_add(t, t, x);
+        f_neg(t, t);
+    }
+    r = t;
 }
 
 FK_HD void g1_phi(G1P &R, const G1P &P) {

@@ -243,34 +243,6 @@ void launch_g1_fused(const FusedPlan &p, cudaStream_t st) {
     k_g1_fused<<<p.blocks, FFT_THREADS, 0, st>>>(p);
 }
 
-// last DIF stage + zeroing of the upper half + first DIT stage: pairs
-// (2q, 2q+1) -> both = a + b, optionally times 2^-log_m
-template <bool SCALE>
-__global__ void __launch_bounds__(FFT_THREADS) k_g1_middle(uint4 *__restrict__ D, int G, int log_m) {
-    // the program scratch (SCALE), whose point 1 also holds b for the sum;
-    // without SCALE one point of scratch
-    __shared__ uint32_t slots[SCALE ? PROG_SLOT_WORDS : 36][FFT_THREADS];
-    const int m = 1 << log_m;
-    const int warp = blockIdx.x * (FFT_THREADS / 32) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    const int g = warp % G, q = warp / G;
-    if (q >= (m >> 1)) return;
-    uint4 *p0 = D + tile_index(g, m, 2 * q);
-    uint4 *p1 = D + tile_index(g, m, 2 * q + 1);
-    const StridedPoint sv{&slots[SCALE ? 36 : 0][threadIdx.x], FFT_THREADS};
-    G1P x;
-    tile_to_slot(sv, p1, lane);
-    tile_load(x, p0, lane);
-    g1_add_q(x, x, sv, false);
-    if (SCALE) {
-        const ProgSlots slot{&slots[0][threadIdx.x], FFT_THREADS};
-        slot[0].put(x);
-        g1_mul_prog(x, slot, c_prog[512 + log_m]);
-    }
-    tile_store(p0, lane, x);
-    tile_store(p1, lane, x);
-}
-
 // every point of the tiles times program `prog`
 __global__ void __launch_bounds__(FFT_THREADS) k_g1_scale(uint4 *__restrict__ D, int G, int log_m, int prog) {
     __shared__ uint32_t slots[PROG_SLOT_WORDS][FFT_THREADS];
@@ -304,9 +276,10 @@ __global__ void k_ref_to_tile(uint4 *__restrict__ D, const uint64_t *__restrict_
     }
 }
 
-// tiles -> reference g1p_t rows, natural order; row r is written at
-// dst + 18 * (row_off ? row_off[r] : r * m)
-__global__ void k_tile_to_ref(uint64_t *__restrict__ dst, const uint4 *__restrict__ D, const size_t *__restrict__ row_off,
+// tiles -> reference g1p_t rows, natural order, normalised (x, y, 1): the
+// words do not depend on the order of additions that led to a point.  Row r is
+// written at dst + 18 * (row_off ? row_off[r] : r * m).
+__global__ void k_tile_to_ref(uint64_t *__restrict__ dst, const TileView V, const size_t *__restrict__ row_off,
                               int rows, int log_m, int bitrev_out) {
     const int m = 1 << log_m;
     const size_t total = (size_t)rows * m;
@@ -314,7 +287,8 @@ __global__ void k_tile_to_ref(uint64_t *__restrict__ dst, const uint4 *__restric
         const int row = (int)(e / m), i = (int)(e % m);
         const int pos = bitrev_out ? (int)bitrev((unsigned)i, log_m) : i;
         G1P p;
-        tile_load(p, D + tile_index(row >> 5, m, pos), row & 31);
+        view_load(p, V, row, pos, m);
+        g1_normalize(p);
         const size_t base = row_off ? row_off[row] : (size_t)row * m;
         g1p_to_ref(dst + 18 * (base + i), p);
     }
@@ -353,11 +327,6 @@ void launch_g1_stage(uint4 *D, int G, int log_m, int s, int kind, cudaStream_t s
     if (kind == 0) k_g1_stage<0><<<blocks, FFT_THREADS, 0, st>>>(D, G, log_m, s);
     else k_g1_stage<1><<<blocks, FFT_THREADS, 0, st>>>(D, G, log_m, s);
 }
-void launch_g1_middle(uint4 *D, int G, int log_m, int scale, cudaStream_t st) {
-    const unsigned blocks = blocks_for((size_t)G * ((1u << log_m) / 2), FFT_THREADS / 32);
-    if (scale) k_g1_middle<true><<<blocks, FFT_THREADS, 0, st>>>(D, G, log_m);
-    else k_g1_middle<false><<<blocks, FFT_THREADS, 0, st>>>(D, G, log_m);
-}
 void launch_g1_scale(uint4 *D, int G, int log_m, int prog, cudaStream_t st) {
     k_g1_scale<<<blocks_for((size_t)G * (1u << log_m), FFT_THREADS / 32), FFT_THREADS, 0, st>>>(D, G, log_m, prog);
 }
@@ -366,9 +335,9 @@ void launch_ref_to_tile(uint4 *D, const uint64_t *src, int rows, int G, int log_
     k_ref_to_tile<<<grid_stride_blocks((size_t)G * 32 * (1u << log_m)), 256, 0, st>>>(D, src, rows, G, log_m,
                                                                                    bitrev_in, zero_upper);
 }
-void launch_tile_to_ref(uint64_t *dst, const uint4 *D, const size_t *row_off, int rows, int log_m, int bitrev_out,
+void launch_tile_to_ref(uint64_t *dst, const TileView &v, const size_t *row_off, int rows, int log_m, int bitrev_out,
                         cudaStream_t st) {
-    k_tile_to_ref<<<grid_stride_blocks((size_t)rows << log_m), 256, 0, st>>>(dst, D, row_off, rows, log_m, bitrev_out);
+    k_tile_to_ref<<<blocks_for((size_t)rows << log_m, 64), 64, 0, st>>>(dst, v, row_off, rows, log_m, bitrev_out);
 }
 void launch_hext2h_ref(uint64_t *h, int rows, int log_m, cudaStream_t st) {
     k_hext2h_ref<<<grid_stride_blocks((size_t)rows << (log_m - 1)), 256, 0, st>>>(h, rows, log_m);

@@ -65,8 +65,9 @@ __device__ __forceinline__ void store_scalar(uint4 *dst, const uint32_t v[8]) {
     dst[32] = make_uint4(s2[0], s2[1], s2[2], s2[3]);
 }
 
-// grid (rows, 16), block m/2: toeplitz -> FFT -> scalar tiles S[g][c][i][q][lane]
-__global__ void __launch_bounds__(256) k_tc_fft(uint4 *__restrict__ S, const uint64_t *__restrict__ poly,
+// grid (rows, 16), block m/2: toeplitz -> FFT -> scalar tiles S[g][c][i][q][lane],
+// group g at S + g * stride
+__global__ void __launch_bounds__(256) k_tc_fft(uint4 *__restrict__ S, size_t stride, const uint64_t *__restrict__ poly,
                                                const size_t *__restrict__ row_off, int n, int log_m) {
     __shared__ uint32_t sm[512][8];
     const int m = 1 << log_m;
@@ -87,7 +88,7 @@ __global__ void __launch_bounds__(256) k_tc_fft(uint4 *__restrict__ S, const uin
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const int c = tid + h * (m >> 1);
-        store_scalar(S + ((((size_t)g * m + c) * L_COLS + i) * SCAL_Q) * 32 + lane, sm[c]);
+        store_scalar(S + g * stride + (((size_t)c * L_COLS + i) * SCAL_Q) * 32 + lane, sm[c]);
     }
 }
 
@@ -156,9 +157,9 @@ __global__ void k_ref_to_scalars(uint4 *__restrict__ S, const uint64_t *__restri
     }
 }
 
-void launch_tc_fft(uint4 *S, const uint64_t *poly, const size_t *row_off, int n, int log_m, unsigned rows,
+void launch_tc_fft(uint4 *S, size_t stride, const uint64_t *poly, const size_t *row_off, int n, int log_m, unsigned rows,
                    cudaStream_t st) {
-    k_tc_fft<<<dim3(rows, L_COLS), (1u << log_m) / 2, 0, st>>>(S, poly, row_off, n, log_m);
+    k_tc_fft<<<dim3(rows, L_COLS), (1u << log_m) / 2, 0, st>>>(S, stride, poly, row_off, n, log_m);
 }
 void launch_fr_fft_ref(uint64_t *out, const uint64_t *in, int log_m, unsigned count, int inverse, cudaStream_t st) {
     k_fr_fft_ref<<<count, (1u << log_m) / 2, 0, st>>>(out, in, log_m, inverse);

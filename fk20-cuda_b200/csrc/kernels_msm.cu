@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(MSM_MAX_THREADS, FK_MSM_MINB) k_msm(const __gr
 #pragma unroll 1
         for (int i = 0; i < L_COLS; i++) {
             uint32_t s[9];
-            const uint4 v = a.S[((((size_t)g * m + c) * L_COLS + i) * SCAL_Q + half) * 32 + lane];
+            const uint4 v = a.S[g * a.s_stride + (((size_t)c * L_COLS + i) * SCAL_Q + half) * 32 + lane];
             s[0] = v.x; s[1] = v.y; s[2] = v.z; s[3] = v.w;
 #pragma unroll
             for (int k = 4; k < 9; k++) s[k] = 0;
@@ -216,7 +216,13 @@ __global__ void __launch_bounds__(MSM_MAX_THREADS, FK_MSM_MINB) k_msm(const __gr
     if (args.times_m) {
         for (int t = 0; t < a.log_m; t++) g1_dbl(acc, acc);
     }
-    tile_store(a.D + tile_index(g, m, c), lane, acc);
+    if (a.arena.slots == 0) {
+        tile_store(a.D + tile_index(g, m, c), lane, acc);
+    } else if (!a.arena.paired || row < 16) {
+        int ga, la;
+        proj_lane(a.arena, row, proj_in_inst(c), ga, la);
+        tile_store(a.D + proj_tile(a.arena, ga, proj_in_slot(c, a.log_m)), la, acc);
+    }
 }
 
 // ---------------------------------------------------------------- KZG commitments

@@ -71,14 +71,14 @@ __global__ void k_h_fft_to_proofs(uint8_t *__restrict__ out, const uint64_t *__r
 
 // pipeline tiles (h_fft, natural order) -> proofs in data-availability order;
 // row r's proofs start at proof index (out_off ? out_off[r] : r * m)
-__global__ void k_tile_to_proofs(uint8_t *__restrict__ out, const uint4 *__restrict__ D,
+__global__ void k_tile_to_proofs(uint8_t *__restrict__ out, const TileView V,
                                  const size_t *__restrict__ out_off, int rows, int log_m) {
     const int m = 1 << log_m;
     const size_t total = (size_t)rows * m;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
         const int row = (int)(e >> log_m), i = (int)(e & (m - 1));
         G1P p;
-        tile_load(p, D + tile_index(row >> 5, m, (int)bitrev((unsigned)i, log_m)), row & 31);
+        view_load(p, V, row, (int)bitrev((unsigned)i, log_m), m);
         uint32_t w[12];
         g1_compress48(w, p);
         const size_t base = out_off ? out_off[row] : (size_t)row * m;
@@ -92,9 +92,9 @@ void launch_g1p_compress(uint8_t *out, const uint64_t *p, size_t count, cudaStre
 void launch_h_fft_to_proofs(uint8_t *out, const uint64_t *h, int rows, int log_m, cudaStream_t st) {
     k_h_fft_to_proofs<<<grid_stride_blocks((size_t)rows << log_m), 128, 0, st>>>(out, h, rows, log_m);
 }
-void launch_tile_to_proofs(uint8_t *out, const uint4 *D, const size_t *out_off, int rows, int log_m,
+void launch_tile_to_proofs(uint8_t *out, const TileView &v, const size_t *out_off, int rows, int log_m,
                            cudaStream_t st) {
-    k_tile_to_proofs<<<grid_stride_blocks((size_t)rows << log_m), 128, 0, st>>>(out, D, out_off, rows, log_m);
+    k_tile_to_proofs<<<blocks_for((size_t)rows << log_m, 64), 64, 0, st>>>(out, v, out_off, rows, log_m);
 }
 
 }  // namespace fk

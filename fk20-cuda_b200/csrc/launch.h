@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "fused_plan.cuh"
+#include "proj_task.cuh"
 
 namespace fk {
 
@@ -21,6 +22,8 @@ struct MsmSeg {
     const uint4 *table;
     int G, log_m, rows, cb, W;
     unsigned warp_start;  // first warp (of the launch) that works on this segment
+    ProjArena arena;      // slots > 0: D is an arena (proj_task.cuh), else point tiles [G][m]
+    size_t s_stride;      // uint4 from one row group's scalars to the next
 };
 struct MsmArgs {
     MsmSeg seg[MAX_SEGS];
@@ -50,6 +53,39 @@ struct FusedPlan {
 };
 constexpr unsigned FUSED_SPIN_LIMIT = 1u << 24;  // default spin_limit
 
+// Persistent projection launch (kernels_proj.cu): per segment its arena,
+// ready[G][slots + 1] (slot versions, then the count of finished products),
+// the plan's tasks and the products' programs.
+struct ProjSeg {
+    uint4 *D;
+    unsigned *ready;
+    const ProjTask *tasks;
+    const uint32_t *progs;
+    ProjArena arena;
+    int ntasks, nprog, nprod;  // nprod: products per group
+};
+struct ProjArgs {
+    ProjSeg seg[MAX_PROJ_SEGS];
+    ProjRuns runs;
+    int nseg;
+    unsigned first, last;  // launch indices to run
+    unsigned *next;        // task counter (zeroed before the launch)
+    int *err;              // 0 = ok, else 1000 + phase that timed out, 2000 a failed check
+    unsigned spin_limit;   // polls before a wait gives up
+    unsigned unpublished;  // as FusedPlan::unpublished
+};
+int proj_blocks_per_sm();
+void launch_proj(const ProjArgs &p, int blocks, cudaStream_t st);
+void launch_ref_to_arena(uint4 *D, const ProjArena &A, const uint64_t *src, int rows, int log_m, cudaStream_t st);
+
+// Points read by the output kernels: natural tiles [G][m], or (out != null) an
+// arena whose slot out[k] holds position 2k + instance
+struct TileView {
+    const uint4 *D;
+    const uint16_t *out;
+    ProjArena arena;
+};
+
 // per-module constant upload (one per translation unit)
 cudaError_t upload_consts_fr();
 cudaError_t upload_consts_msm();
@@ -58,7 +94,7 @@ cudaError_t upload_consts_tables();
 cudaError_t upload_consts_misc();
 
 // kernels_fr.cu
-void launch_tc_fft(uint4 *S, const uint64_t *poly, const size_t *row_off, int n, int log_m, unsigned rows,
+void launch_tc_fft(uint4 *S, size_t stride, const uint64_t *poly, const size_t *row_off, int n, int log_m, unsigned rows,
                    cudaStream_t st);
 void launch_fr_fft_ref(uint64_t *out, const uint64_t *in, int log_m, unsigned count, int inverse, cudaStream_t st);
 void launch_toeplitz_ref(uint64_t *tc, const uint64_t *poly, int n, int log_m, unsigned rows, cudaStream_t st);
@@ -70,6 +106,7 @@ void launch_msm(const MsmArgs &a, int threads, cudaStream_t st);  // threads: 64
 // MSM / persistent-FFT translation units (0: none)
 int check_take_msm();
 int check_take_fft();
+int check_take_proj();
 // KZG commitments: polynomial lengths are multiples of COMMIT_CHUNK; pass 1
 // has commit_parts(rows, n) warps per 32 rows, and part holds as many tiles
 constexpr int COMMIT_CHUNK = 32;
@@ -79,13 +116,12 @@ void launch_commit(uint64_t *out, uint4 *part, const uint64_t *poly, const uint4
 
 // kernels_fft.cu
 void launch_g1_stage(uint4 *D, int G, int log_m, int s, int kind, cudaStream_t st);
-void launch_g1_middle(uint4 *D, int G, int log_m, int scale, cudaStream_t st);
 int fused_blocks_per_sm();
 void launch_g1_fused(const FusedPlan &p, cudaStream_t st);
 void launch_g1_scale(uint4 *D, int G, int log_m, int prog, cudaStream_t st);
 void launch_ref_to_tile(uint4 *D, const uint64_t *src, int rows, int G, int log_m, int bitrev_in, int zero_upper,
                         cudaStream_t st);
-void launch_tile_to_ref(uint64_t *dst, const uint4 *D, const size_t *row_off, int rows, int log_m, int bitrev_out,
+void launch_tile_to_ref(uint64_t *dst, const TileView &v, const size_t *row_off, int rows, int log_m, int bitrev_out,
                         cudaStream_t st);
 void launch_hext2h_ref(uint64_t *h, int rows, int log_m, cudaStream_t st);
 void launch_setup_to_tile(uint4 *D, const uint64_t *setup, int n, int log_m, cudaStream_t st);
@@ -93,7 +129,7 @@ void launch_setup_to_tile(uint4 *D, const uint64_t *setup, int n, int log_m, cud
 // kernels_out.cu: 48-byte compressed proofs, data-availability order
 void launch_g1p_compress(uint8_t *out, const uint64_t *p, size_t count, cudaStream_t st);
 void launch_h_fft_to_proofs(uint8_t *out, const uint64_t *h, int rows, int log_m, cudaStream_t st);
-void launch_tile_to_proofs(uint8_t *out, const uint4 *D, const size_t *out_off, int rows, int log_m,
+void launch_tile_to_proofs(uint8_t *out, const TileView &v, const size_t *out_off, int rows, int log_m,
                            cudaStream_t st);
 
 // kernels_pairing.cu: op 0 pairing values, op 1 pairing checks; G2 element-wise ops

@@ -18,6 +18,7 @@
 //   ((b * W + w) * E + e) * 6.
 #pragma once
 #include "g1.cuh"
+#include "launch.h"
 
 namespace fk {
 
@@ -43,6 +44,17 @@ FK_D void tile_store(uint4 *__restrict__ base, int lane, const G1P &p) {
     for (int k = 0; k < 12; k++) { w[k] = p.x.w[k]; w[12 + k] = p.y.w[k]; w[24 + k] = p.z.w[k]; }
 #pragma unroll
     for (int q = 0; q < TILE_Q; q++) base[q * 32 + lane] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+}
+
+// the point of (row, position i) of an output view
+FK_D void view_load(G1P &p, const TileView &v, int row, int i, int m) {
+    if (!v.out) {
+        tile_load(p, v.D + tile_index(row >> 5, m, i), row & 31);
+        return;
+    }
+    int g, lane;
+    proj_lane(v.arena, row, i & 1, g, lane);
+    tile_load(p, v.D + proj_tile(v.arena, g, v.out[i >> 1]), lane);
 }
 
 // tile point -> strided slot (shared memory), one uint4 at a time, without

@@ -163,3 +163,66 @@ int emul_glv_split(uint64_t *out, const uint64_t *s, long count) {
     return 0;
 }
 }
+
+#include "proj_plan.cuh"
+extern "C" {
+// The projection plan of FFT size 2^log_m (proj_plan.cuh).  head: slots, tasks,
+// products, outputs, levels.  tasks: 16 ints each (op, sh, phi, neg, d0, d1, a,
+// b, b2, va, vb, vb2, w0, w1, phase, prog); scalars: 4 x u64 each; levels:
+// (first, count, phase).  Arrays may be null (sizes only).
+int emul_proj_plan(int log_m, int half, int *head, int *tasks, uint64_t *scalars, int *out, int *levels) {
+    static ProjPlan plans[2][10];
+    ProjPlan &p = plans[half][log_m];
+    if (p.tasks.empty()) p = host::build_proj_plan(log_m, half != 0);
+    head[0] = p.slots, head[1] = (int)p.tasks.size(), head[2] = p.muls, head[3] = (int)p.out.size();
+    head[4] = (int)p.levels.size();
+    if (!tasks) return 0;
+    for (size_t i = 0; i < p.tasks.size(); i++) {
+        const ProjTask &t = p.tasks[i];
+        const int v[16] = {t.op, t.sh, t.phi, t.neg, t.d0, t.d1, t.a, t.b, t.b2, t.va, t.vb, t.vb2, t.w0, t.w1, t.phase, t.prog};
+        for (int k = 0; k < 16; k++) tasks[16 * i + k] = v[k];
+    }
+    for (int i = 0; i < p.muls; i++)
+        for (int k = 0; k < 4; k++) scalars[4 * i + k] = p.scalars[i][k];
+    for (size_t i = 0; i < p.out.size(); i++) out[i] = p.out[i];
+    for (size_t i = 0; i < p.levels.size(); i++)
+        levels[3 * i] = p.levels[i].first, levels[3 * i + 1] = p.levels[i].count, levels[3 * i + 2] = p.levels[i].phase;
+    return 0;
+}
+
+// input slot, instance of hext position c
+void emul_proj_in(int c, int log_m, int *slot, int *inst) { *slot = proj_in_slot(c, log_m), *inst = proj_in_inst(c); }
+
+// launch order of nseg segments (rows each, FFT size 2^log_m each): (seg, task, group) per index
+long emul_proj_order(int nseg, const int *log_m, const int *rows, int *out, long cap) {
+    static ProjPlan plans[10];
+    static ProjRuns r;
+    const ProjPlan *pp[MAX_PROJ_SEGS];
+    int G[MAX_PROJ_SEGS];
+    for (int k = 0; k < nseg; k++) {
+        ProjPlan &p = plans[log_m[k]];
+        if (p.tasks.empty()) p = host::build_proj_plan(log_m[k], false);
+        pp[k] = &p;
+        G[k] = proj_arena(p.slots, (unsigned)rows[k]).G;
+    }
+    if (!host::build_proj_runs(r, pp, G, nseg)) return -1;
+    if ((long)r.total > cap) return -(long)r.total;
+    for (unsigned t = 0; t < r.total; t++) {
+        int *o = out + 3 * (size_t)t;
+        proj_decode(r, t, o[0], o[1], o[2]);
+    }
+    return (long)r.total;
+}
+
+// (P + Q, P - Q) by the shared formulas
+void emul_g1_addsub(uint64_t *sum, uint64_t *diff, const uint64_t *a, const uint64_t *b, long count) {
+    for (long i = 0; i < count; i++) {
+        G1P p, q, r[2];
+        g1_load(p, a + 18 * i);
+        g1_load(q, b + 18 * i);
+        g1_addsub_q(p, RegPoint{q}, [&](int w, int c, const Fp &f) { (c == 0 ? r[w].x : c == 1 ? r[w].y : r[w].z) = f; });
+        g1_store(sum + 18 * i, r[0]);
+        g1_store(diff + 18 * i, r[1]);
+    }
+}
+}
