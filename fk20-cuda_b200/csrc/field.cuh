@@ -10,14 +10,14 @@
 //
 // Montgomery product r = A*B/2^(32N): word-serial CIOS with the partial products of each
 // word b_i split between two accumulators, `e` (products a_j*b_i with j even:
-// lo at word j, hi at word j+1) and `o` (j odd).  Within one accumulator the
-// lo/hi words of different j never overlap, so each half is a single
-// mad.lo.cc/madc.hi.cc carry chain and the two chains are independent.  The
-// reduction multiple m*p is split the same way.  After the reduction the
-// word-0 sum e0+o0 is 0 mod 2^32; its carry (0 or 1) is fed into the next
-// iteration at word 0 of the odd chain, and both accumulators shift down one
-// word.  Bounds: with A < 2p (4p < 2^384) and B < 2^384 every partial value
-// stays below 2^416, so 13 words per accumulator suffice, and the result is
+// lo at word j, hi at word j+1) and `o` (j odd; o[k] is word k + 1).  Within one
+// accumulator the lo/hi words of different j never overlap, so each half is a
+// single mad.lo.cc/madc.hi.cc carry chain and the two chains are independent.
+// The reduction multiple m*p is split the same way.  After it word 0 is 0 and
+// everything moves down one word: the accumulators change roles, and the word
+// left between them, e[1], joins the next word 0, whose carry goes into the
+// next reduction's odd chain.  Bounds: with A < 2p (4p < 2^384) and B < 2^384
+// every partial value stays below 2^416, so 13 words suffice, and the result is
 // < 2p when A, B < 2p or when A < p (one conditional subtraction of p makes
 // it canonical).  A must not exceed ~2^382: a full-width A overflows.
 #pragma once
@@ -81,11 +81,10 @@ template <class F> FK_D void ptx_add(uint32_t *r, const uint32_t *a, const uint3
 template <class F> FK_D uint32_t ptx_sub(uint32_t *r, const uint32_t *a, const uint32_t *b);
 template <class F> FK_D uint32_t ptx_sub_mod(uint32_t *r, const uint32_t *t);
 template <class F> FK_D void ptx_row_even(uint32_t *e, const uint32_t *a, uint32_t b);
-template <class F> FK_D void ptx_row_odd(uint32_t *o, const uint32_t *a, uint32_t b, uint32_t c);
+template <class F> FK_D void ptx_row_odd(uint32_t *o, const uint32_t *a, uint32_t b);
 template <class F> FK_D void ptx_red_even(uint32_t *e, uint32_t m);
-template <class F> FK_D void ptx_red_odd(uint32_t *o, uint32_t m);
+template <class F> FK_D void ptx_red_odd(uint32_t *o, uint32_t m, uint32_t &e0, uint32_t x);
 template <class F> FK_D void ptx_final(uint32_t *t, const uint32_t *e, const uint32_t *o);
-template <class F> FK_D void ptx_final_c(uint32_t *t, const uint32_t *e, const uint32_t *o, uint32_t c);
 template <class F, int I> FK_D void ptx_sqrow_even(uint32_t *e, const uint32_t *v, uint32_t b);
 template <class F, int I> FK_D void ptx_sqrow_odd(uint32_t *o, const uint32_t *v, uint32_t b);
 #if defined(__CUDA_ARCH__)
@@ -143,22 +142,20 @@ FK_HD void ch_row_even(uint32_t *e, const uint32_t *a, uint32_t b) {
 #endif
 }
 
-// o[0] += c; o[1..N] += a[j]*b for odd j (lo word at j, hi word at j+1);
-// o[N] is written, not read
+// o[0..N-1] (words 1..N) += a[j]*b for odd j (lo word at o[j-1], hi word at
+// o[j]); o[N-1] is written, not read
 template <class F>
-FK_HD void ch_row_odd(uint32_t *o, const uint32_t *a, uint32_t b, uint32_t c) {
+FK_HD void ch_row_odd(uint32_t *o, const uint32_t *a, uint32_t b) {
 #if defined(__CUDA_ARCH__)
-    ptx_row_odd<F>(o, a, b, c);
+    ptx_row_odd<F>(o, a, b);
 #else
-    uint64_t s = (uint64_t)o[0] + c;
-    o[0] = (uint32_t)s;
-    s >>= 32;
-    for (int w = 1; w < F::N; w++) {
-        s += (uint64_t)o[w] + ((w & 1) ? mul_lo(a[w], b) : mul_hi(a[w - 1], b));
+    uint64_t s = 0;
+    for (int w = 0; w < F::N - 1; w++) {
+        s += (uint64_t)o[w] + ((w & 1) ? mul_hi(a[w], b) : mul_lo(a[w + 1], b));
         o[w] = (uint32_t)s;
         s >>= 32;
     }
-    o[F::N] = (uint32_t)(s + mul_hi(a[F::N - 1], b));
+    o[F::N - 1] = (uint32_t)(s + mul_hi(a[F::N - 1], b));
 #endif
 }
 
@@ -178,55 +175,42 @@ FK_HD void ch_red_even(uint32_t *e, uint32_t m) {
 #endif
 }
 
-// o[1..N] += m*mod[j] for odd j (o[0] unchanged)
+// e0 += x (word 0), its carry and m*mod[j] for odd j into o[0..N-1] (words 1..N)
 template <class F>
-FK_HD void ch_red_odd(uint32_t *o, uint32_t m) {
+FK_HD void ch_red_odd(uint32_t *o, uint32_t m, uint32_t &e0, uint32_t x) {
 #if defined(__CUDA_ARCH__)
-    ptx_red_odd<F>(o, m);
+    ptx_red_odd<F>(o, m, e0, x);
 #else
-    uint64_t c = 0;
-    for (int w = 1; w < F::N; w++) {
-        c += (uint64_t)o[w] + ((w & 1) ? mul_lo(m, F::mod(w)) : mul_hi(m, F::mod(w - 1)));
+    uint64_t c = (uint64_t)e0 + x;
+    e0 = (uint32_t)c;
+    c >>= 32;
+    for (int w = 0; w < F::N - 1; w++) {
+        c += (uint64_t)o[w] + ((w & 1) ? mul_hi(m, F::mod(w)) : mul_lo(m, F::mod(w + 1)));
         o[w] = (uint32_t)c;
         c >>= 32;
     }
-    o[F::N] += (uint32_t)c + mul_hi(m, F::mod(F::N - 1));
+    o[F::N - 1] += (uint32_t)c + mul_hi(m, F::mod(F::N - 1));
 #endif
 }
 
-// t[0..N-1] = (e + o) >> 32 over N+1 words
+// t[k] = e[k+1] + o[k], k < N
 template <class F>
 FK_HD void ch_final(uint32_t *t, const uint32_t *e, const uint32_t *o) {
 #if defined(__CUDA_ARCH__)
     ptx_final<F>(t, e, o);
 #else
-    uint64_t c = ((uint64_t)e[0] + o[0]) >> 32;
-    for (int k = 1; k <= F::N; k++) {
-        c += (uint64_t)e[k] + o[k];
-        t[k - 1] = (uint32_t)c;
+    uint64_t c = 0;
+    for (int k = 0; k < F::N; k++) {
+        c += (uint64_t)e[k + 1] + o[k];
+        t[k] = (uint32_t)c;
         c >>= 32;
     }
 #endif
 }
 
-// t[0..N-1] = (e + o + c) >> 32 over N+1 words, c (0 or 1) added at word 0
-template <class F>
-FK_HD void ch_final_c(uint32_t *t, const uint32_t *e, const uint32_t *o, uint32_t c) {
-#if defined(__CUDA_ARCH__)
-    ptx_final_c<F>(t, e, o, c);
-#else
-    uint64_t s = ((uint64_t)e[0] + o[0] + c) >> 32;
-    for (int k = 1; k <= F::N; k++) {
-        s += (uint64_t)e[k] + o[k];
-        t[k - 1] = (uint32_t)s;
-        s >>= 32;
-    }
-#endif
-}
-
-// squaring row I >= 1, one parity P of j (0: the e half, 1: the o half):
-// acc[j0..] += v[j] * b for j >= I, j = P mod 2 (lo word at j, hi word at
-// j + 1), the carry out of the e half into e[N]; acc[N] is written, not read
+// squaring row I >= 1, one parity P of j >= I: P = 0: e[j], e[j+1] += v[j] * b,
+// the carry out into e[N]; P = 1: o[j-1], o[j] += v[j] * b, o[N-1] written, not
+// read
 template <class F, int I, int P>
 FK_HD void ch_sqrow(uint32_t *acc, const uint32_t *v, uint32_t b) {
 #if defined(__CUDA_ARCH__)
@@ -235,32 +219,18 @@ FK_HD void ch_sqrow(uint32_t *acc, const uint32_t *v, uint32_t b) {
 #else
     constexpr int N = F::N;
     const int j0 = (I % 2 == P) ? I : I + 1;
-    if (j0 >= N) return;  // no product of this parity (acc[N] keeps its 0)
+    if (j0 >= N) return;  // no product of this parity
     uint64_t c = 0;
-    for (int w = j0; w < N; w++) {
-        c += (uint64_t)acc[w] + (((w - j0) & 1) ? mul_hi(v[w - 1], b) : mul_lo(v[w], b));
+    for (int j = j0; j < N; j += 2) {
+        const int w = j - P;
+        c += (uint64_t)acc[w] + mul_lo(v[j], b);
         acc[w] = (uint32_t)c;
         c >>= 32;
+        c += (P == 1 && j == N - 1 ? 0 : (uint64_t)acc[w + 1]) + mul_hi(v[j], b);
+        acc[w + 1] = (uint32_t)c;
+        c >>= 32;
     }
-    acc[N] = P == 0 ? (uint32_t)c : (uint32_t)(c + mul_hi(v[N - 1], b));
-#endif
-}
-
-// the carry out of e0 + o0 + c, c = 0 or 1
-FK_HD uint32_t ch_carry3(uint32_t e0, uint32_t o0, uint32_t c) {
-#if defined(__CUDA_ARCH__)
-    return ptx_carry3(e0, o0, c);
-#else
-    return (uint32_t)(((uint64_t)e0 + o0 + c) >> 32);
-#endif
-}
-
-// the carry out of e0 + o0
-FK_HD uint32_t ch_carry0(uint32_t e0, uint32_t o0) {
-#if defined(__CUDA_ARCH__)
-    return ptx_carry0(e0, o0);
-#else
-    return (uint32_t)(((uint64_t)e0 + o0) >> 32);
+    if (P == 0) acc[N] = (uint32_t)c;
 #endif
 }
 
@@ -304,12 +274,39 @@ FK_HD void f_reduce_once(uint32_t r[F::N], const uint32_t t[F::N]) {
 }
 
 // ---------------------------------------------------------------- Montgomery product
+// One reduction step and the shift by one word.  Word 0 is e[0] + x, x the word
+// left over from the step before; m makes it vanish.  The shift keeps each
+// accumulator's lo/hi pairs on even register positions: the odd words 1..N
+// become the even words 0..N-1, and e[2..N] the odd words (a lo/hi pair is one
+// 64-bit multiply-add only on an even register; shifting both accumulators in
+// place puts every second step's pairs on odd ones).  B200, 2^22 elements x 64
+// dependent products: Fp product 26.2 -> 30.2 G/s (98 % of half the IMAD peak),
+// square 31.3 -> 38.0 G/s; Fr 56.5 -> 56.9 G/s.
+template <class F>
+FK_HD void f_reduce_step(uint32_t *e, uint32_t *o, uint32_t &x, bool last) {
+    constexpr int N = F::N;
+    const uint32_t m = mul_lo(e[0] + x, F::M0);
+    ch_red_odd<F>(o, m, e[0], x);
+    ch_red_even<F>(e, m);
+    if (last) return;
+    uint32_t t[N + 1];
+#pragma unroll
+    for (int k = 0; k <= N; k++) t[k] = e[k];
+#pragma unroll
+    for (int k = 0; k < N; k++) e[k] = o[k];
+    e[N] = 0;
+#pragma unroll
+    for (int k = 0; k < N - 1; k++) o[k] = t[k + 2];
+    o[N - 1] = 0;
+    x = t[1];
+}
+
 template <class F>
 FK_HD void f_mul(Elem<F> &r, const Elem<F> &A, const Elem<F> &B) {
     constexpr int N = F::N;
     const uint32_t *a = A.w;
-    uint32_t e[N + 1], o[N + 1];
-    uint32_t c = 0;
+    uint32_t e[N + 1], o[N];
+    uint32_t x = 0;
 
     // word 0 of b: plain products, no chains needed
     {
@@ -318,40 +315,21 @@ FK_HD void f_mul(Elem<F> &r, const Elem<F> &A, const Elem<F> &B) {
         for (int j = 0; j < N; j += 2) {
             e[j] = mul_lo(a[j], bi);
             e[j + 1] = mul_hi(a[j], bi);
+            o[j] = mul_lo(a[j + 1], bi);
+            o[j + 1] = mul_hi(a[j + 1], bi);
         }
         e[N] = 0;
-        o[0] = 0;
-#pragma unroll
-        for (int j = 1; j < N; j += 2) {
-            o[j] = mul_lo(a[j], bi);
-            o[j + 1] = mul_hi(a[j], bi);
-        }
     }
 
 #pragma unroll
     for (int i = 0; i < N; i++) {
         if (i > 0) {
-            // even products into e[0..N]; the previous word-0 carry and the
-            // odd products into o[0..N]
             ch_row_even<F>(e, a, B.w[i]);
-            ch_row_odd<F>(o, a, B.w[i], c);
+            ch_row_odd<F>(o, a, B.w[i]);
         }
-        // reduction: add m*p, m chosen so that word 0 vanishes
-        const uint32_t m = mul_lo(e[0] + o[0], F::M0);
-        ch_red_even<F>(e, m);
-        ch_red_odd<F>(o, m);
-        if (i < N - 1) {
-            c = ch_carry0(e[0], o[0]);
-#pragma unroll
-            for (int k = 0; k < N; k++) {
-                e[k] = e[k + 1];
-                o[k] = o[k + 1];
-            }
-            e[N] = 0;
-            o[N] = 0;
-        }
+        f_reduce_step<F>(e, o, x, i == N - 1);
     }
-    // final: (e + o) >> 32, then one conditional subtraction
+    // the upper words, then one conditional subtraction
     uint32_t t[N];
     ch_final<F>(t, e, o);
     f_reduce_once<F>(r.w, t);
@@ -363,16 +341,14 @@ FK_HD void f_mul(Elem<F> &r, const Elem<F> &A, const Elem<F> &B) {
 // Fr): row i adds a_i * V_i, V_i = a_i 2^(32 i) + 2 sum_{j > i} a_j 2^(32 j),
 // whose words are a_i, a_{i+1} << 1 and then the words of 2A (the top bit of
 // a_i belongs to row i's own a_i, not to 2A's word i + 1).  Sum over i:
-// sum a_i^2 2^(64 i) + 2 sum_{i<j} a_i a_j 2^(32(i+j)) = A^2.  As a row no
-// longer starts at word 0, the word-0 carry c of each reduction step is
-// carried into the next step's word-0 sum (and the final shift) instead of
-// the odd half's first word.  Bounds: V_i <= 2A, so A < 2^(32N - 2) keeps
-// every partial value where f_mul's do (A canonical: A < m), except the top
-// word of the odd half, which holds hi(2 a_{N-1} a_i) + hi(m mod_{N-1}) and
-// stays below 2^32 only for a modulus whose top word is below 2^30 (Fp:
-// 0x1a0111ea; Fr's 0x73eda753 is not, so Fr squares are products).
+// sum a_i^2 2^(64 i) + 2 sum_{i<j} a_i a_j 2^(32(i+j)) = A^2.  Bounds: V_i <= 2A,
+// so A < 2^(32N - 2) keeps every partial value where f_mul's do (A canonical:
+// A < m), except the top word of the odd half, which holds hi(2 a_{N-1} a_i) +
+// hi(m mod_{N-1}) and stays below 2^32 only for a modulus whose top word is
+// below 2^30 (Fp: 0x1a0111ea; Fr's 0x73eda753 is not, so Fr squares are
+// products).
 template <class F, int I>
-FK_HD void f_sqr_rows(uint32_t *e, uint32_t *o, uint32_t &c, const uint32_t *a, const uint32_t *a2) {
+FK_HD void f_sqr_rows(uint32_t *e, uint32_t *o, uint32_t &x, const uint32_t *a, const uint32_t *a2) {
     constexpr int N = F::N;
     if constexpr (I > 0) {
         uint32_t v[N];
@@ -381,21 +357,8 @@ FK_HD void f_sqr_rows(uint32_t *e, uint32_t *o, uint32_t &c, const uint32_t *a, 
         ch_sqrow<F, I, 0>(e, v, a[I]);
         ch_sqrow<F, I, 1>(o, v, a[I]);
     }
-    // reduction: add m*p, m chosen so that word 0 (with the pending carry) vanishes
-    const uint32_t m = mul_lo(e[0] + o[0] + c, F::M0);
-    ch_red_even<F>(e, m);
-    ch_red_odd<F>(o, m);
-    if constexpr (I < N - 1) {
-        c = ch_carry3(e[0], o[0], c);
-#pragma unroll
-        for (int k = 0; k < N; k++) {
-            e[k] = e[k + 1];
-            o[k] = o[k + 1];
-        }
-        e[N] = 0;
-        o[N] = 0;
-        f_sqr_rows<F, I + 1>(e, o, c, a, a2);
-    }
+    f_reduce_step<F>(e, o, x, I == N - 1);
+    if constexpr (I < N - 1) f_sqr_rows<F, I + 1>(e, o, x, a, a2);
 }
 
 template <class F>
@@ -409,29 +372,24 @@ FK_HD void f_sqr(Elem<F> &r, const Elem<F> &A) {
         a2[0] = a[0] << 1;
 #pragma unroll
         for (int j = 1; j < N; j++) a2[j] = (a[j] << 1) | (a[j - 1] >> 31);
-        uint32_t e[N + 1], o[N + 1];
-        uint32_t c = 0;
+        uint32_t e[N + 1], o[N];
+        uint32_t x = 0;
         {
             // row 0: V_0 = (a_0, a_1 << 1, 2A's words 2..N-1), plain products
             const uint32_t b = a[0];
 #pragma unroll
             for (int j = 0; j < N; j += 2) {
-                const uint32_t v = j == 0 ? a[0] : a2[j];
-                e[j] = mul_lo(v, b);
-                e[j + 1] = mul_hi(v, b);
+                const uint32_t v0 = j == 0 ? a[0] : a2[j], v1 = j == 0 ? a[1] << 1 : a2[j + 1];
+                e[j] = mul_lo(v0, b);
+                e[j + 1] = mul_hi(v0, b);
+                o[j] = mul_lo(v1, b);
+                o[j + 1] = mul_hi(v1, b);
             }
             e[N] = 0;
-            o[0] = 0;
-#pragma unroll
-            for (int j = 1; j < N; j += 2) {
-                const uint32_t v = j == 1 ? a[1] << 1 : a2[j];
-                o[j] = mul_lo(v, b);
-                o[j + 1] = mul_hi(v, b);
-            }
         }
-        f_sqr_rows<F, 0>(e, o, c, a, a2);
+        f_sqr_rows<F, 0>(e, o, x, a, a2);
         uint32_t t[N];
-        ch_final_c<F>(t, e, o, c);
+        ch_final<F>(t, e, o);
         f_reduce_once<F>(r.w, t);
     }
 }

@@ -21,15 +21,9 @@ Run from this directory: python gen_chains.py > chains.inc"""
 FIELDS = (("FpDesc", 12), ("FrDesc", 8))
 
 
-def block(name, sig, lines, outs, ins, temps=()):
+def block(name, sig, lines, outs, ins):
     """One device function whose body is a single asm statement."""
-    body = []
-    if temps:
-        body.append('"{\\n\\t"')
-        body.append('".reg .u32 %s;\\n\\t"' % ", ".join(temps))
-    body += ['"%s;\\n\\t"' % l for l in lines]
-    if temps:
-        body.append('"}"')
+    body = ['"%s;\\n\\t"' % l for l in lines]
     txt = "template <> FK_D %s %s<%s>(%s) {\n" % (sig[0], name, sig[1], sig[2])
     txt += sig[3]
     txt += "    asm volatile(" + "\n        ".join(body) + "\n"
@@ -88,20 +82,22 @@ def gen(desc, n):
     out.append(block("ptx_row_even", ("void", desc, "uint32_t *e, const uint32_t *a, uint32_t b", "", ""),
                      lines, outs, ins))
 
-    # product row, odd half: o[0] += c, then o[1..n] += a[j] * b for odd j
-    # (lo word at j, hi word at j + 1); o[n] is overwritten (its old value is 0)
-    outs = ['"+r"(o[%d])' % i for i in range(n)] + ['"=r"(o[%d])' % n]
-    ins = ['"r"(a[%d])' % (2 * k + 1) for k in range(half)] + ['"r"(b)', '"r"(c)']
-    c_ = "%%%d" % (n + 1 + half + 1)
-    lines = ["add.cc.u32 %%0, %%0, %s" % c_]
+    # product row, odd half (o[k] is word k + 1): o[0..n-1] += a[j] * b for odd j
+    # (lo word at o[j-1], hi word at o[j]); no carry out of o[n-1], whose old
+    # value is 0
+    outs = ['"+r"(o[%d])' % i for i in range(n - 1)] + ['"=r"(o[%d])' % (n - 1)]
+    ins = ['"r"(a[%d])' % (2 * k + 1) for k in range(half)] + ['"r"(b)']
+    a_ = lambda k: "%%%d" % (n + k)
+    b_ = "%%%d" % (n + half)
+    lines = []
     for k in range(half):
-        lo, hi = 2 * k + 1, 2 * k + 2
-        lines.append("madc.lo.cc.u32 %%%d, %s, %s, %%%d" % (lo, a_(k), b_, lo))
+        lo, hi = 2 * k, 2 * k + 1
+        lines.append("%s.u32 %%%d, %s, %s, %%%d" % ("mad.lo.cc" if k == 0 else "madc.lo.cc", lo, a_(k), b_, lo))
         if k < half - 1:
             lines.append("madc.hi.cc.u32 %%%d, %s, %s, %%%d" % (hi, a_(k), b_, hi))
         else:
             lines.append("madc.hi.u32 %%%d, %s, %s, 0" % (hi, a_(k), b_))
-    out.append(block("ptx_row_odd", ("void", desc, "uint32_t *o, const uint32_t *a, uint32_t b, uint32_t c", "", ""),
+    out.append(block("ptx_row_odd", ("void", desc, "uint32_t *o, const uint32_t *a, uint32_t b", "", ""),
                      lines, outs, ins))
 
     # reduction, even half: e[0..n-1] += m * mod[j] for even j; e[n] += carry
@@ -117,22 +113,23 @@ def gen(desc, n):
     lines.append("addc.u32 %%%d, %%%d, 0" % (n, n))
     out.append(block("ptx_red_even", ("void", desc, "uint32_t *e, uint32_t m", "", ""), lines, outs, ins))
 
-    # reduction, odd half: o[1..n] += m * mod[j] for odd j (o[0] untouched)
-    outs = ['"+r"(o[%d])' % i for i in range(1, n + 1)]
-    ins = ['"r"(m)'] + ['"n"(%s::mod(%d))' % (desc, 2 * k + 1) for k in range(half)]
-    m_ = "%%%d" % n
-    q_ = lambda k: "%%%d" % (n + 1 + k)
-    O = lambda w: "%%%d" % (w - 1)  # o[w] is operand w - 1
-    lines = []
+    # reduction, odd half: e0 += x (word 0; the carry goes on to word 1), then
+    # o[0..n-1] += m * mod[j] for odd j (lo word at o[j-1], hi word at o[j])
+    outs = ['"+r"(o[%d])' % i for i in range(n)] + ['"+r"(e0)']
+    ins = ['"r"(m)', '"r"(x)'] + ['"n"(%s::mod(%d))' % (desc, 2 * k + 1) for k in range(half)]
+    m_, x_ = "%%%d" % (n + 1), "%%%d" % (n + 2)
+    q_ = lambda k: "%%%d" % (n + 3 + k)
+    lines = ["add.cc.u32 %%%d, %%%d, %s" % (n, n, x_)]
     for k in range(half):
-        lo, hi = 2 * k + 1, 2 * k + 2
-        lines.append("%s.u32 %s, %s, %s, %s" % ("mad.lo.cc" if k == 0 else "madc.lo.cc", O(lo), m_, q_(k), O(lo)))
-        lines.append("%s.u32 %s, %s, %s, %s" % ("madc.hi.cc" if k < half - 1 else "madc.hi", O(hi), m_, q_(k), O(hi)))
-    out.append(block("ptx_red_odd", ("void", desc, "uint32_t *o, uint32_t m", "", ""), lines, outs, ins))
+        lo, hi = 2 * k, 2 * k + 1
+        lines.append("madc.lo.cc.u32 %%%d, %s, %s, %%%d" % (lo, m_, q_(k), lo))
+        lines.append("%s.u32 %%%d, %s, %s, %%%d" % ("madc.hi.cc" if k < half - 1 else "madc.hi", hi, m_, q_(k), hi))
+    out.append(block("ptx_red_odd", ("void", desc, "uint32_t *o, uint32_t m, uint32_t &e0, uint32_t x", "", ""), lines, outs, ins))
 
     # squaring rows I = 1 .. n-1 (row 0 is plain products): e[j0..n-1] += v[j] * b
     # for even j >= I (lo word at j, hi word at j + 1), e[n] = the carry out;
-    # o[j0..n] += v[j] * b for odd j >= I, o[n] written (its old value is 0)
+    # odd j >= I: lo word at o[j-1], hi word at o[j], no carry out of o[n-1],
+    # whose old value is 0
     for I in range(1, n):
         for par, acc in ((0, "e"), (1, "o")):
             js = [j for j in range(I, n) if j % 2 == par]
@@ -141,13 +138,8 @@ def gen(desc, n):
             if not js:
                 out.append("template <> FK_D void %s<%s, %d>(uint32_t *, const uint32_t *, uint32_t) {}\n" % (name, desc, I))
                 continue
-            j0 = js[0]
-            top = n if par == 0 else n + 1  # words j0 .. top - 1 are read and written
-            words = list(range(j0, top))
-            outs = []
-            for w in words:
-                last_even = par == 0 and w == n
-                outs.append('"%s"(%s[%d])' % ("=r" if (w == n) else "+r", acc, w))
+            words = list(range(js[0] - par, n))
+            outs = ['"%s"(%s[%d])' % ("=r" if par == 1 and w == n - 1 else "+r", acc, w) for w in words]
             if par == 0:
                 outs.append('"=r"(%s[%d])' % (acc, n))
             op = {w: "%%%d" % k for k, w in enumerate(words + ([n] if par == 0 else []))}
@@ -157,9 +149,9 @@ def gen(desc, n):
             b_ = "%%%d" % (base + len(js))
             lines = []
             for k, j in enumerate(js):
-                lo, hi = j, j + 1
+                lo, hi = j - par, j - par + 1
                 lines.append("%s.u32 %s, %s, %s, %s" % ("mad.lo.cc" if k == 0 else "madc.lo.cc", op[lo], vj[j], b_, op[lo]))
-                if hi == n and par == 1:
+                if par == 1 and j == js[-1]:
                     lines.append("madc.hi.u32 %s, %s, %s, 0" % (op[hi], vj[j], b_))
                 else:
                     lines.append("madc.hi.cc.u32 %s, %s, %s, %s" % (op[hi], vj[j], b_, op[hi]))
@@ -167,28 +159,14 @@ def gen(desc, n):
                 lines.append("addc.u32 %s, 0, 0" % op[n])
             out.append(block(name, sig, lines, outs, ins))
 
-    # t = (e + o + c) >> 32 over n + 1 words, c the pending word-0 carry (0 or 1)
+    # t[k] = e[k+1] + o[k], k < n (the carry out of the top word is dropped)
     outs = ['"=r"(t[%d])' % i for i in range(n)]
-    ins = ['"r"(e[%d])' % i for i in range(n + 1)] + ['"r"(o[%d])' % i for i in range(n + 1)] + ['"r"(c)']
-    E = lambda i: "%%%d" % (n + i)
-    Oo = lambda i: "%%%d" % (2 * n + 1 + i)
-    c_ = "%%%d" % (3 * n + 2)
-    lines = ["add.cc.u32 x, %s, -1" % c_, "addc.cc.u32 x, %s, %s" % (E(0), Oo(0))]
-    lines += ["addc.cc.u32 %%%d, %s, %s" % (k - 1, E(k), Oo(k)) for k in range(1, n)]
-    lines += ["addc.u32 %%%d, %s, %s" % (n - 1, E(n), Oo(n))]
-    out.append(block("ptx_final_c", ("void", desc, "uint32_t *t, const uint32_t *e, const uint32_t *o, uint32_t c", "", ""),
-                     lines, outs, ins, temps=("x",)))
-
-    # t = (e + o) >> 32 over n + 1 words
-    outs = ['"=r"(t[%d])' % i for i in range(n)]
-    ins = ['"r"(e[%d])' % i for i in range(n + 1)] + ['"r"(o[%d])' % i for i in range(n + 1)]
-    E = lambda i: "%%%d" % (n + i)
-    Oo = lambda i: "%%%d" % (2 * n + 1 + i)
-    lines = ["add.cc.u32 x, %s, %s" % (E(0), Oo(0))]
-    lines += ["addc.cc.u32 %%%d, %s, %s" % (k - 1, E(k), Oo(k)) for k in range(1, n)]
-    lines += ["addc.u32 %%%d, %s, %s" % (n - 1, E(n), Oo(n))]
+    ins = ['"r"(e[%d])' % i for i in range(1, n + 1)] + ['"r"(o[%d])' % i for i in range(n)]
+    lines = ["add.cc.u32 %%0, %%%d, %%%d" % (n, 2 * n)]
+    lines += ["addc.cc.u32 %%%d, %%%d, %%%d" % (k, n + k, 2 * n + k) for k in range(1, n - 1)]
+    lines += ["addc.u32 %%%d, %%%d, %%%d" % (n - 1, 2 * n - 1, 3 * n - 1)]
     out.append(block("ptx_final", ("void", desc, "uint32_t *t, const uint32_t *e, const uint32_t *o", "", ""),
-                     lines, outs, ins, temps=("x",)))
+                     lines, outs, ins))
     return out
 
 
@@ -200,33 +178,6 @@ def main():
         print("\n// ---------------------------------------------------------------- %s (%d limbs)\n" % (desc, n))
         for f in gen(desc, n):
             print(f)
-    # word-0 carry of the Montgomery loop, shared by both fields
-    print("// the carry out of e0 + o0 (0 or 1)")
-    print("FK_D uint32_t ptx_carry0(uint32_t e0, uint32_t o0) {")
-    print("    uint32_t c;")
-    print('    asm volatile("{\\n\\t"')
-    print('        ".reg .u32 x;\\n\\t"')
-    print('        "add.cc.u32 x, %1, %2;\\n\\t"')
-    print('        "addc.u32 %0, 0, 0;\\n\\t"')
-    print('        "}"')
-    print('        : "=r"(c)')
-    print('        : "r"(e0), "r"(o0));')
-    print("    return c;")
-    print("}")
-    # carry out of e0 + o0 + c (c = 0 or 1): the carry flag is set to c first
-    print("// the carry out of e0 + o0 + c, c = 0 or 1")
-    print("FK_D uint32_t ptx_carry3(uint32_t e0, uint32_t o0, uint32_t c) {")
-    print("    uint32_t r;")
-    print('    asm volatile("{\\n\\t"')
-    print('        ".reg .u32 x;\\n\\t"')
-    print('        "add.cc.u32 x, %3, -1;\\n\\t"')
-    print('        "addc.cc.u32 x, %1, %2;\\n\\t"')
-    print('        "addc.u32 %0, 0, 0;\\n\\t"')
-    print('        "}"')
-    print('        : "=r"(r)')
-    print('        : "r"(e0), "r"(o0), "r"(c));')
-    print("    return r;")
-    print("}")
     print("// clang-format on")
 
 
