@@ -691,7 +691,7 @@ struct SegLayout {
     // a segment's arena, scalars inside, and its ready counters (full), or its scalar and point tiles
     void add(int k, int log_m, unsigned rows, bool full) {
         const int m = 1 << log_m, G = (int)((rows + 31) / 32);
-        arena[k] = full ? proj_arena(pipeline_slots(log_m), rows) : ProjArena{0, G, 0};
+        arena[k] = full ? proj_arena(pipeline_slots(log_m), rows) : ProjArena{0, G, 0, 0};
         s_stride[k] = full ? (size_t)arena[k].slots * TILE_Q * 32 : scal_group(log_m);
         s_off[k] = s_bytes;
         if (!full) s_bytes += scal_bytes(G, m);

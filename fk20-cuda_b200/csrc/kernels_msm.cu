@@ -163,48 +163,83 @@ FK_D int msm_add_scalar(G1Z &acc, const uint32_t s[9], const uint4 *__restrict__
     return carry;
 }
 
-// One warp per (segment, column c, group g of 32 rows); lanes are rows.
-// Warps are numbered segment by segment, g fastest, so the warps of a block
-// read the same table column.
+// sum of the lanes that differ in the lane bits off, 2 off, .. 16 (every lane
+// gets it)
+FK_D void g1_sum_lanes(G1P &p, int off) {
+#pragma unroll 1
+    for (; off < 32; off <<= 1) {
+        G1P q;
+#pragma unroll
+        for (int k = 0; k < 12; k++) {
+            q.x.w[k] = __shfl_xor_sync(0xffffffffu, p.x.w[k], off);
+            q.y.w[k] = __shfl_xor_sync(0xffffffffu, p.y.w[k], off);
+            q.z.w[k] = __shfl_xor_sync(0xffffffffu, p.z.w[k], off);
+        }
+        g1_add(p, p, q);
+    }
+}
+
+// sum of n warps' points (warps w0 .. w0 + n - 1 of the block), in warp w0;
+// part holds 36 x 32 words per warp.  Every thread of the block calls it.
+FK_D void g1_sum_warps(G1P &p, uint32_t *part, int w0, int n) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const StridedPoint mine{part + w * 36 * 32 + lane, 32};
+    if (w != w0) mine.put(p);
+    __syncthreads();
+    if (w == w0)
+        for (int k = 1; k < n; k++) {
+            const StridedPoint other{part + (w0 + k) * 36 * 32 + lane, 32};
+            g1_add_q(p, p, other, false);
+        }
+}
+
+// Unit (segment, column c, group g of rows): 2^rl rows on the low lane bits,
+// the 32 (base, GLV half) terms of a column shared by the 32 >> rl lane groups
+// and args.split warps of the unit; their sums are added by shuffles and
+// through shared memory.  Large batches have one warp per unit and a row per
+// lane.  Units are numbered segment by segment, g fastest, so the warps of a
+// block read the same table column.
 __global__ void __launch_bounds__(MSM_MAX_THREADS, FK_MSM_MINB) k_msm(const __grid_constant__ MsmArgs args) {
+    extern __shared__ uint32_t part[];
     const unsigned warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (warp >= args.warps) return;
+    bool on = warp < args.warps;  // uniform over a unit's warps
     int k = 0;
     while (k + 1 < args.nseg && warp >= args.seg[k + 1].warp_start) k++;
     const MsmSeg &a = args.seg[k];
     const int m = 1 << a.log_m;
     const int lane = threadIdx.x & 31;
-    const unsigned wl = warp - a.warp_start;
-    const int g = (int)(wl % (unsigned)a.G), c = (int)(wl / (unsigned)a.G);
-    if (!FK_CHECK(g_check_msm, k < args.nseg && c < m, FK20_CHECK_MSM_TILE)) return;
+    const unsigned wl = on ? warp - a.warp_start : 0;
+    const unsigned unit = wl / (unsigned)args.split;
+    const int sub = (int)(wl % (unsigned)args.split);
+    const int g = (int)(unit % (unsigned)a.G), c = (int)(unit / (unsigned)a.G);
+    on = on && FK_CHECK(g_check_msm, k < args.nseg && c < m && args.split * (32 >> a.rl) <= 32, FK20_CHECK_MSM_TILE);
+    if (!on && args.split == 1) return;
     if (args.test_check && warp == 0 && lane == 0) (void)FK_CHECK(g_check_msm, false, FK20_CHECK_MSM_PLANTED);
-    const int row = g * 32 + lane;
-    const bool live = row < a.rows;
+    const int row = a.row0 + g * 32 + (lane & ((1 << a.rl) - 1));
+    const bool live = on && row < a.rows;
     const int E = 1 << (a.cb - 1);
     // sum_i [s_i] X_i = phi(sum_i [s2_i] X_i) + sum_i [s1_i] X_i with
     // s_i = s1_i + s2_i lambda (the scalar tile holds s1 at uint4 0 and s2 at
-    // uint4 1): the s2 halves first, then phi on the accumulator
-    // ((X, Y, ZZ, ZZZ) -> (beta X, Y, ZZ, ZZZ)), then the s1 halves.
+    // uint4 1): terms 0..15 are the s2 halves, 16..31 the s1 halves; phi goes on
+    // the accumulator ((X, Y, ZZ, ZZZ) -> (beta X, Y, ZZ, ZZZ)) after the last
+    // s2 half.
+    const int per = 32 / ((32 >> a.rl) * args.split);
+    const int q0 = ((lane >> a.rl) * args.split + sub) * per;
     G1Z accz;
     g1z_set_inf(accz);
 #pragma unroll 1
-    for (int half = 1; half >= 0; half--) {
-#pragma unroll 1
-        for (int i = 0; i < L_COLS; i++) {
-            uint32_t s[9];
-            const uint4 v = a.S[g * a.s_stride + (((size_t)c * L_COLS + i) * SCAL_Q + half) * 32 + lane];
-            s[0] = v.x; s[1] = v.y; s[2] = v.z; s[3] = v.w;
+    for (int j = 0; j < per && on; j++) {
+        const int q = q0 + j, half = q < L_COLS, i = q & (L_COLS - 1);
+        uint32_t s[9];
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (live) v = a.S[(row >> 5) * a.s_stride + (((size_t)c * L_COLS + i) * SCAL_Q + half) * 32 + (row & 31)];
+        s[0] = v.x; s[1] = v.y; s[2] = v.z; s[3] = v.w;
 #pragma unroll
-            for (int k = 4; k < 9; k++) s[k] = 0;
-            if (!live) {
-#pragma unroll
-                for (int k = 0; k < 4; k++) s[k] = 0;
-            }
-            const uint4 *tb = a.table + ((size_t)(i * m + c) * a.W) * E * 6;
-            const int carry = msm_add_scalar(accz, s, tb, a.W, a.cb);
-            (void)FK_CHECK(g_check_msm, carry == 0, FK20_CHECK_MSM_CARRY);
-        }
-        if (half) {
+        for (int k = 4; k < 9; k++) s[k] = 0;
+        const uint4 *tb = a.table + ((size_t)(i * m + c) * a.W) * E * 6;
+        const int carry = msm_add_scalar(accz, s, tb, a.W, a.cb);
+        (void)FK_CHECK(g_check_msm, carry == 0, FK20_CHECK_MSM_CARRY);
+        if (q == L_COLS - 1 || (half && j == per - 1)) {
             Fp beta;
 #pragma unroll
             for (int k = 0; k < 12; k++) beta.w[k] = beta_mont(k);
@@ -213,14 +248,19 @@ __global__ void __launch_bounds__(MSM_MAX_THREADS, FK_MSM_MINB) k_msm(const __gr
     }
     G1P acc;
     g1z_to_proj(acc, accz);
+    g1_sum_lanes(acc, 1 << a.rl);
+    if (args.split > 1) g1_sum_warps(acc, part, (threadIdx.x >> 5) - sub, args.split);
+    if (!on || sub != 0) return;
     if (args.times_m) {
         for (int t = 0; t < a.log_m; t++) g1_dbl(acc, acc);
     }
+    // every lane stores: lanes beyond the rows get copies of the rows' points
+    const int to = a.row0 + g * 32 + lane;
     if (a.arena.slots == 0) {
-        tile_store(a.D + tile_index(g, m, c), lane, acc);
-    } else if (!a.arena.paired || row < 16) {
+        tile_store(a.D + tile_index(to >> 5, m, c), lane, acc);
+    } else {
         int ga, la;
-        proj_lane(a.arena, row, proj_in_inst(c), ga, la);
+        if (!proj_lane(a.arena, to, proj_in_inst(c), ga, la)) return;
         tile_store(a.D + proj_tile(a.arena, ga, proj_in_slot(c, a.log_m)), la, acc);
     }
 }
@@ -228,23 +268,24 @@ __global__ void __launch_bounds__(MSM_MAX_THREADS, FK_MSM_MINB) k_msm(const __gr
 // ---------------------------------------------------------------- KZG commitments
 // commitment[row] = sum_i poly[row][i] * s_i over fixed-base tables of the
 // setup points s_i (commit_to_poly, FK20Py/kzg_proofs.py:159-163).  Pass 1:
-// warp (g, p) sums bases [p n / P, (p+1) n / P) for the 32 rows of group g
-// into a partial-sum tile, P = commit_parts(rows, n) warps per group, chosen
-// so that pass 1 is one wave of resident warps (whole warps of fixed chunks
-// left a second, mostly idle wave); pass 2: one thread per row adds its P
-// partials.
+// warp (g, p) sums bases [p n / P, (p+1) n / P) for the rows of group g into a
+// partial-sum tile, P = commit_parts(rows, n) warps per group, chosen so that
+// pass 1 is one wave of resident warps; with 16 rows or fewer the bases of a
+// warp are shared by 32 >> rl lane groups.  Pass 2: one block per row adds its
+// P partials, as a tree.
 __global__ void __launch_bounds__(128) k_commit_partial(uint4 *__restrict__ part, const uint64_t *__restrict__ poly,
                                                         const uint4 *__restrict__ table, int rows, int n, int W,
-                                                        int cb, int P) {
+                                                        int cb, int P, int rl) {
     const int G = (rows + 31) / 32;
     const unsigned warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (warp >= (unsigned)G * P) return;
     const int lane = threadIdx.x & 31;
     const int g = (int)(warp % (unsigned)G), c = (int)(warp / (unsigned)G);
-    const int row = g * 32 + lane;
+    const int row = g * 32 + (lane & ((1 << rl) - 1));
     const bool live = row < rows;
     const int E = 1 << (cb - 1);
-    const int i0 = (int)((long long)c * n / P), i1 = (int)((long long)(c + 1) * n / P);
+    const long long ways = (long long)P * (32 >> rl), way = (long long)c * (32 >> rl) + (lane >> rl);
+    const int i0 = (int)(way * n / ways), i1 = (int)((way + 1) * n / ways);
     G1Z accz;
     g1z_set_inf(accz);
     for (int i = i0; i < i1; i++) {
@@ -257,22 +298,30 @@ __global__ void __launch_bounds__(128) k_commit_partial(uint4 *__restrict__ part
         }
         (void)msm_add_scalar(accz, s, table + (size_t)i * W * E * 6, W, cb);
     }
+    __syncwarp();
     G1P acc;
     g1z_to_proj(acc, accz);
-    tile_store(part + tile_index(g, P, c), lane, acc);
+    g1_sum_lanes(acc, 1 << rl);
+    if ((lane >> rl) == 0) tile_store(part + tile_index(g, P, c), row & 31, acc);
 }
 
-__global__ void k_commit_reduce(uint64_t *__restrict__ out, const uint4 *__restrict__ part, int rows, int P) {
-    for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < rows; row += gridDim.x * blockDim.x) {
-        const int g = row >> 5, lane = row & 31;
-        G1P acc, q;
-        tile_load(acc, part + tile_index(g, P, 0), lane);
-        for (int c = 1; c < P; c++) {
-            tile_load(q, part + tile_index(g, P, c), lane);
-            g1_add(acc, acc, q);
-        }
-        g1p_to_ref(out + 18 * (size_t)row, acc);
+constexpr int REDUCE_THREADS = 128;
+__global__ void __launch_bounds__(REDUCE_THREADS) k_commit_reduce(uint64_t *__restrict__ out, const uint4 *__restrict__ part,
+                                                                  int P) {
+    __shared__ uint32_t sm[(REDUCE_THREADS / 32) * 36 * 32];
+    const int row = blockIdx.x, g = row >> 5, lane = row & 31;
+    G1P acc, q;
+    g1_set_inf(acc);
+    for (int c = threadIdx.x; c < P; c += REDUCE_THREADS) {
+        tile_load(q, part + tile_index(g, P, c), lane);
+        g1_add(acc, acc, q);
     }
+    __syncwarp();
+    g1_sum_lanes(acc, 1);
+    constexpr int WARPS = REDUCE_THREADS / 32;
+    const int warps = (P + 31) / 32;
+    g1_sum_warps(acc, sm, 0, warps < WARPS ? warps : WARPS);
+    if (threadIdx.x == 0) g1p_to_ref(out + 18 * (size_t)row, acc);
 }
 
 // pass-1 warps per group of 32 rows: one wave of the warps the device holds
@@ -289,22 +338,61 @@ int commit_parts(int rows, int n) {
         }
         resident = sms * bps * 4;
     }
-    const int G = (rows + 31) / 32;
-    return std::max(1, std::min(n, resident / G));
+    const int G = (rows + 31) / 32, lanes = 32 >> msm_row_lanes(rows);
+    return std::max(1, std::min((n + lanes - 1) / lanes, resident / G));
 }
 
 void launch_commit(uint64_t *out, uint4 *part, const uint64_t *poly, const uint4 *table, int rows, int n, int W,
                    int cb, cudaStream_t st) {
     const int P = commit_parts(rows, n);
     const unsigned warps = (unsigned)((rows + 31) / 32) * (unsigned)P;
-    k_commit_partial<<<blocks_for(warps, 4), 128, 0, st>>>(part, poly, table, rows, n, W, cb, P);
-    k_commit_reduce<<<blocks_for((size_t)rows, 128), 128, 0, st>>>(out, part, rows, P);
+    k_commit_partial<<<blocks_for(warps, 4), 128, 0, st>>>(part, poly, table, rows, n, W, cb, P, msm_row_lanes(rows));
+    k_commit_reduce<<<(unsigned)rows, REDUCE_THREADS, 0, st>>>(out, part, P);
 }
 
-void launch_msm(const MsmArgs &a, int threads, cudaStream_t st) {
+// How a launch is cut.  A segment's last rows % 32 rows form a segment of their
+// own whose lanes are packed (msm_row_lanes); and while whole units leave the
+// chip's last wave of warps a large share of the time, four warps (two in
+// 64-thread blocks) share a unit.  Resident: three 128-thread blocks per SM.
+// A batch of one or two rows has 16 or 32 lane groups already, and more warps
+// would only add sums.  B200, window 10, MSM alone, before (a row per lane, a
+// warp per unit) and after: 1 row of 4096 4.41 -> 0.21 ms, 19 of 2048 4.64 ->
+// 1.63, 160 of 4096 15.1 -> 13.5; at 512 rows of 4096 (4.6 waves) splitting
+// costs 1 %, 40.7 -> 41.1, hence the line at 4 waves.  48 commitments of 4096:
+// 10.5 -> 3.0 ms, most of it the partial sums, which one thread per row added.
+void launch_msm(const MsmArgs &in, int threads, cudaStream_t st) {
     if (threads != 64 && threads != 128 && threads != 256) threads = 128;
     if (threads > MSM_MAX_THREADS) threads = MSM_MAX_THREADS;
-    k_msm<<<blocks_for(a.warps, (unsigned)threads / 32), threads, 0, st>>>(a);
+    MsmArgs a = in;
+    a.nseg = 0;
+    unsigned units = 0;
+    for (int k = 0; k < in.nseg; k++) {
+        const int full = in.seg[k].rows & ~31, rest = in.seg[k].rows & 31;
+        for (int part = 0; part < 2; part++) {
+            if (part ? !rest : !full) continue;
+            MsmSeg s = in.seg[k];
+            s.row0 = part ? full : 0;
+            s.rl = part ? msm_row_lanes(rest) : 5;
+            s.G = part ? 1 : full / 32;
+            if (!part) s.rows = full;
+            s.warp_start = units;
+            units += (unsigned)s.G << s.log_m;
+            a.seg[a.nseg++] = s;
+        }
+    }
+    const unsigned resident = 148 * 12;
+    int rl_max = 0;
+    for (int k = 0; k < a.nseg; k++) rl_max = std::max(rl_max, a.seg[k].rl);
+    a.split = 1;
+    if (rl_max > 1 && units < 4 * resident) a.split = threads == 64 ? 2 : 4;
+    for (int k = 0; k < a.nseg; k++) {
+        // at most 32 terms: lane groups and warps together
+        a.seg[k].rl = std::max(a.seg[k].rl, a.split == 4 ? 2 : a.split == 2 ? 1 : 0);
+        a.seg[k].warp_start *= (unsigned)a.split;
+    }
+    a.warps = units * (unsigned)a.split;
+    const size_t smem = a.split > 1 ? (size_t)threads * 36 * sizeof(uint32_t) : 0;
+    k_msm<<<blocks_for(a.warps, (unsigned)threads / 32), threads, smem, st>>>(a);
 }
 
 }  // namespace fk

@@ -110,8 +110,9 @@ __global__ void __launch_bounds__(FFT_THREADS, 1) k_proj(const __grid_constant__
         unsigned *rg = S.ready + (size_t)g * (A.slots + 1);
         // an output reads the other instance's slot: b for instance 0, b2 for
         // instance 1 (both, in the same group, when instances share a group)
-        const int inst = A.paired ? lane >> 4 : g >= (A.G >> 1);
-        const int gx = A.paired ? g : inst ? g - (A.G >> 1) : g + (A.G >> 1);
+        const bool pair = g >= 2 * A.F;
+        const int inst = pair ? lane >> 4 : g >= A.F;
+        const int gx = pair ? g : inst ? g - A.F : g + A.F;
         const int sx = inst ? t.b2 : t.b;
         int ok = 1;
         if (lane < 4) {  // lane 0: a, 1: b, 2: b2, 3: the group's products
@@ -119,10 +120,10 @@ __global__ void __launch_bounds__(FFT_THREADS, 1) k_proj(const __grid_constant__
             unsigned need = 0;
             const bool out = t.op == PROJ_OUT;
             if (lane == 0) r = rg + t.a, need = t.va;
-            if (lane == 1 && t.b != PROJ_NONE && !(out && !A.paired && inst)) {
+            if (lane == 1 && t.b != PROJ_NONE && !(out && !pair && inst)) {
                 r = (out ? S.ready + (size_t)gx * (A.slots + 1) : rg) + t.b, need = t.vb;
             }
-            if (lane == 2 && t.b2 != PROJ_NONE && !(out && !A.paired && !inst)) {
+            if (lane == 2 && t.b2 != PROJ_NONE && !(out && !pair && !inst)) {
                 r = (out ? S.ready + (size_t)gx * (A.slots + 1) : rg) + t.b2, need = t.vb2;
             }
             if (lane == 3 && t.phase == 2) r = rg + A.slots, need = (unsigned)S.nprod;
@@ -151,7 +152,7 @@ __global__ void __launch_bounds__(FFT_THREADS, 1) k_proj(const __grid_constant__
             store_cg(d0, lane, acc);
         } else {
             const uint4 *pb = t.op == PROJ_OUT ? S.D + proj_tile(A, gx, sx) : S.D + proj_tile(A, g, t.b);
-            const int lb = t.op == PROJ_OUT && A.paired ? lane ^ 16 : lane;
+            const int lb = t.op == PROJ_OUT && pair ? lane ^ 16 : lane;
             // the operand with the coefficient goes to the scratch point: b, or a for an output
             const bool out = t.op == PROJ_OUT;
             slot_cg(slot[1], out ? pa : pb, out ? lane : lb);
@@ -195,21 +196,21 @@ void launch_proj(const ProjArgs &p, int blocks, cudaStream_t st) { k_proj<<<bloc
 
 // reference hext_fft rows [rows][m] -> arena inputs
 __global__ void k_ref_to_arena(uint4 *__restrict__ D, ProjArena A, const uint64_t *__restrict__ src, int rows, int log_m) {
-    const int m = 1 << log_m, lanes_rows = A.paired ? 16 : 16 * A.G;
-    const size_t total = (size_t)lanes_rows * m;
+    const int m = 1 << log_m;
+    const size_t total = (size_t)(32 * A.F + 16 * A.paired) * m;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
         const int row = (int)(e >> log_m), c = (int)(e & (size_t)(m - 1));
         G1P p;
         if (row < rows) g1p_from_ref(p, src + 18 * e);
         else g1_set_inf(p);
         int g, lane;
-        proj_lane(A, row, proj_in_inst(c), g, lane);
+        (void)proj_lane(A, row, proj_in_inst(c), g, lane);
         tile_store(D + proj_tile(A, g, proj_in_slot(c, log_m)), lane, p);
     }
 }
 
 void launch_ref_to_arena(uint4 *D, const ProjArena &A, const uint64_t *src, int rows, int log_m, cudaStream_t st) {
-    const size_t lanes = (size_t)(A.paired ? 16 : 16 * A.G) << log_m;
+    const size_t lanes = (size_t)(32 * A.F + 16 * A.paired) << log_m;
     k_ref_to_arena<<<grid_stride_blocks(lanes), 256, 0, st>>>(D, A, src, rows, log_m);
 }
 

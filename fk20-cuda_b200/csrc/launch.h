@@ -24,10 +24,12 @@ struct MsmSeg {
     unsigned warp_start;  // first warp (of the launch) that works on this segment
     ProjArena arena;      // slots > 0: D is an arena (proj_task.cuh), else point tiles [G][m]
     size_t s_stride;      // uint4 from one row group's scalars to the next
+    int row0, rl;         // set by launch_msm: the first row, log2 of the rows a warp takes
 };
 struct MsmArgs {
-    MsmSeg seg[MAX_SEGS];
+    MsmSeg seg[2 * MAX_SEGS];  // a caller fills at most MAX_SEGS
     int nseg, times_m;
+    int split;  // set by launch_msm: warps per (column, row group)
     int test_check;  // checked build: record FK20_CHECK_MSM_PLANTED (tests of the checks)
     unsigned warps;  // total warps = sum of G * m
 };
@@ -99,6 +101,13 @@ void launch_tc_fft(uint4 *S, size_t stride, const uint64_t *poly, const size_t *
 void launch_fr_fft_ref(uint64_t *out, const uint64_t *in, int log_m, unsigned count, int inverse, cudaStream_t st);
 void launch_toeplitz_ref(uint64_t *tc, const uint64_t *poly, int n, int log_m, unsigned rows, cudaStream_t st);
 void launch_ref_to_scalars(uint4 *S, const uint64_t *tcf, int rows, int log_m, cudaStream_t st);
+
+// log2 of the lanes that rows <= 32 rows take
+inline int msm_row_lanes(int rows) {
+    int rl = 0;
+    while (rl < 5 && (1 << rl) < rows) rl++;
+    return rl;
+}
 
 // kernels_msm.cu
 void launch_msm(const MsmArgs &a, int threads, cudaStream_t st);  // threads: 64, 128 or 256

@@ -53,7 +53,7 @@ FK_D void view_load(G1P &p, const TileView &v, int row, int i, int m) {
         return;
     }
     int g, lane;
-    proj_lane(v.arena, row, i & 1, g, lane);
+    (void)proj_lane(v.arena, row, i & 1, g, lane);
     tile_load(p, v.D + proj_tile(v.arena, g, v.out[i >> 1]), lane);
 }
 

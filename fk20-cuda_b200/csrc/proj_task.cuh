@@ -28,19 +28,24 @@ static_assert(sizeof(ProjTask) == 24, "three 8-byte loads");
 // ---------------------------------------------------------------- arena and launch
 // A segment's points live in an arena of G groups of `slots` point tiles
 // (layout.cuh: 9 x 32 uint4 each).  Lanes of a group are (row, instance)
-// pairs: with at most 16 rows one group holds both instances (lane 16 inst +
-// row, `paired`); else groups [0, G/2) are instance 0 of 32 rows each and
-// groups [G/2, G) instance 1.
+// pairs: groups [0, F) are instance 0 of 32 rows each and groups [F, 2 F)
+// instance 1; the last rows of a segment, when 16 or fewer, share one more
+// group (`paired`): lane 16 inst + row.
 struct ProjArena {
-    int slots, G, paired;
+    int slots, G, F, paired;
 };
 FK_HD ProjArena proj_arena(int slots, unsigned rows) {
-    const int paired = rows <= 16;
-    return ProjArena{slots, paired ? 1 : 2 * (int)((rows + 31) / 32), paired};
+    const int rest = (int)(rows & 31u), paired = rest > 0 && rest <= 16;
+    const int F = (int)(rows >> 5) + (rest > 16);
+    return ProjArena{slots, 2 * F + paired, F, paired};
 }
-FK_HD void proj_lane(const ProjArena &a, int row, int inst, int &g, int &lane) {
-    g = a.paired ? 0 : inst * (a.G >> 1) + (row >> 5);
-    lane = a.paired ? 16 * inst + row : row & 31;
+// false: a lane beyond the rows that the paired group holds
+FK_HD bool proj_lane(const ProjArena &a, int row, int inst, int &g, int &lane) {
+    const bool pair = row >= 32 * a.F;
+    const int r = pair ? row - 32 * a.F : row & 31;
+    g = pair ? 2 * a.F : inst * a.F + (row >> 5);
+    lane = pair ? 16 * inst + r : r;
+    return !pair || (a.paired && r < 16);
 }
 FK_HD size_t proj_tile(const ProjArena &a, int g, int slot) { return ((size_t)g * a.slots + slot) * 9 * 32; }
 

@@ -142,7 +142,7 @@ def test_launch_order(emul, rows):
     """Every (segment, task, group) once, and never before a task it depends on."""
     log_m = [9, 8, 7][:len(rows)] if len(rows) > 1 else [7]
     plans = [load_plan(emul, l, 0) for l in log_m]
-    G = [1 if r <= 16 else 2 * ((r + 31) // 32) for r in rows]
+    G = [2 * (r // 32) + (r % 32 > 0) + (r % 32 > 16) for r in rows]
     cap = sum(len(p[1]) * g for p, g in zip(plans, G))
     order = np.zeros((cap, 3), np.int32)
     ci = lambda v: (ctypes.c_int * len(v))(*v)
