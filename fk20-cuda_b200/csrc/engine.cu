@@ -133,8 +133,19 @@ int current_device_ready() {
 
 namespace {
 
-// ---- projection plans (proj_plan.cuh): built once per process and length, then
-// uploaded once per device; kept for the life of the process (0.3 MB at m = 512)
+// Allocations and uploads that a captured call makes the first time it meets a
+// size run outside the capture.
+struct OutsideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// ---- plans of additions and products (proj_plan.cuh): built once per process
+// and size when first used, then uploaded once per device; kept for the life of
+// the process (0.4 MB at m = 512)
+enum PlanKind { PLAN_PROJ = 0, PLAN_PROJ_HALF = 1, PLAN_DFT = 2, PLAN_IDFT = 3 };
+constexpr int PLAN_KINDS = 4;
 struct HostPlan {
     ProjPlan plan;
     std::vector<uint32_t> progs;  // [muls][PROG_WORDS]
@@ -143,16 +154,16 @@ struct HostPlan {
 };
 struct DevPlan {
     ProjTask *tasks = nullptr;
-    uint32_t *progs = nullptr;
-    uint16_t *out = nullptr;
+    uint32_t *progs = nullptr, *out = nullptr;
 };
 
-const HostPlan &host_plan(int log_m, bool half) {
-    static HostPlan plans[2][3];
-    static std::once_flag once[2][3];
-    HostPlan &h = plans[half][log_m - 7];
-    std::call_once(once[half][log_m - 7], [&] {
-        h.plan = host::build_proj_plan(log_m, half);
+const HostPlan &host_plan(PlanKind kind, int log_m) {
+    static HostPlan plans[PLAN_KINDS][MAX_LOG_M + 1];
+    static std::once_flag once[PLAN_KINDS][MAX_LOG_M + 1];
+    HostPlan &h = plans[kind][log_m];
+    std::call_once(once[kind][log_m], [&] {
+        h.plan = kind == PLAN_PROJ || kind == PLAN_PROJ_HALF ? host::build_proj_plan(log_m, kind == PLAN_PROJ_HALF)
+                                                            : host::build_dft_plan(log_m, kind == PLAN_IDFT);
         h.progs.resize((size_t)h.plan.muls * PROG_WORDS);
         for (int k = 0; k < h.plan.muls; k++) {
             uint32_t *p = &h.progs[(size_t)k * PROG_WORDS];
@@ -167,24 +178,29 @@ const HostPlan &host_plan(int log_m, bool half) {
 }
 
 std::mutex g_plan_mu;
-DevPlan g_dev_plan[64][2][3];
+DevPlan g_dev_plan[64][PLAN_KINDS][MAX_LOG_M + 1];
 
 // the plan on the current device `dev`
-int device_plan(int dev, int log_m, bool half, DevPlan *out) {
+int device_plan(int dev, PlanKind kind, int log_m, DevPlan *out) {
     if (dev < 0 || dev >= 64) return FK20_ENODEV;
-    const HostPlan &h = host_plan(log_m, half);
+    const HostPlan &h = host_plan(kind, log_m);
     std::lock_guard<std::mutex> lk(g_plan_mu);
-    DevPlan &d = g_dev_plan[dev][half][log_m - 7];
+    DevPlan &d = g_dev_plan[dev][kind][log_m];
     if (!d.out) {
+        OutsideCapture outside;
         DevPlan n;
+        cudaStream_t st = nullptr;
         const size_t tb = h.plan.tasks.size() * sizeof(ProjTask), pb = h.progs.size() * sizeof(uint32_t),
-                     ob = h.plan.out.size() * sizeof(uint16_t);
-        cudaError_t e = cudaMalloc((void **)&n.tasks, tb);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&n.progs, pb);
+                     ob = h.plan.out.size() * sizeof(uint32_t);
+        cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaMalloc((void **)&n.tasks, tb);
+        if (e == cudaSuccess) e = cudaMalloc((void **)&n.progs, pb + sizeof(uint32_t));
         if (e == cudaSuccess) e = cudaMalloc((void **)&n.out, ob);
-        if (e == cudaSuccess) e = cudaMemcpy(n.tasks, h.plan.tasks.data(), tb, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(n.progs, h.progs.data(), pb, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(n.out, h.plan.out.data(), ob, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(n.tasks, h.plan.tasks.data(), tb, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess && pb) e = cudaMemcpyAsync(n.progs, h.progs.data(), pb, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(n.out, h.plan.out.data(), ob, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (st) cudaStreamDestroy(st);
         if (e != cudaSuccess) {
             cudaGetLastError();
             cudaFree(n.tasks);
@@ -268,6 +284,7 @@ struct DevBuf {
     int reserve(size_t need) {
         if (need <= bytes) return 0;
         if (injected_alloc_failure()) return FK20_ENOMEM;
+        OutsideCapture outside;
         void *q = nullptr;
         if (cudaMalloc(&q, need) != cudaSuccess) {
             cudaGetLastError();
@@ -553,17 +570,22 @@ Work msm_products(int W, int log_m, bool times_m) {
     return w;
 }
 
-// the map hext_fft -> h_fft of one row: counted algorithmically as the FFTs it
-// stands for (inverse DIF stages 0..L-2, last inverse butterfly + zeroing +
-// first forward one, forward DIT stages 1..L-1); executed, two instances of
-// the plan's products and additions
-Work proj_products(int log_m, bool half) {
+// One row of a plan.  Algorithmically the radix-2 transforms it stands for
+// (projection: inverse DIF stages 0..L-2, last inverse butterfly + zeroing +
+// first forward one, forward DIT stages 1..L-1); executed, the plan's products
+// and additions (for a projection, of two instances).
+Work plan_products(PlanKind kind, int log_m) {
     Work w;
-    for (int s = 0; s < log_m - 1; s++) w += stage_products(1, log_m, s, 0) + stage_products(1, log_m, s + 1, 1);
-    w += Work(ADD_P) * (double)(1 << (log_m - 1));
-    const HostPlan &h = host_plan(log_m, half);
-    w.exe = 2 * (h.programs * (37.0 * MP + 16.0 * MS_X) + (h.alg_dbl - h.programs) * (2 * MP + 5 * MS_X) +
-                 (h.alg_add - 3 * h.programs) * (8 * MP + 3 * MS_X) + h.plan.lin_products * MP);
+    const bool proj = kind == PLAN_PROJ || kind == PLAN_PROJ_HALF;
+    if (proj) {
+        for (int s = 0; s < log_m - 1; s++) w += stage_products(1, log_m, s, 0) + stage_products(1, log_m, s + 1, 1);
+        w += Work(ADD_P) * (double)(1 << (log_m - 1));
+    } else {
+        for (int s = 0; s < log_m; s++) w += stage_products(1, log_m, s, kind == PLAN_IDFT ? 0 : 1);
+    }
+    const HostPlan &h = host_plan(kind, log_m);
+    w.exe = (proj ? 2 : 1) * (h.programs * (37.0 * MP + 16.0 * MS_X) + (h.alg_dbl - h.programs) * (2 * MP + 5 * MS_X) +
+                              (h.alg_add - 3 * h.programs) * (8 * MP + 3 * MS_X) + h.plan.lin_products * MP);
     return w;
 }
 
@@ -616,7 +638,7 @@ int build_tables(fk20_ctx *ctx, int log_m, const uint64_t *xext, cudaStream_t st
     T->ready = false;
     T->gen++;
     DevPlan plan;  // the pipeline's plan goes to the device with the tables
-    CKR(device_plan(ctx->device, log_m, false, &plan));
+    CKR(device_plan(ctx->device, PLAN_PROJ, log_m, &plan));
     if (xext != (const uint64_t *)T->xext.p) {  // keep the bases for rebuilds at another window
         CKR(T->xext.reserve((size_t)L_COLS * m * sizeof(g1p_t)));
         CK(cudaMemcpyAsync(T->xext.p, xext, (size_t)L_COLS * m * sizeof(g1p_t), cudaMemcpyDeviceToDevice, st));
@@ -680,7 +702,7 @@ constexpr double PROOF_OUT_MP = 575.0;
 // before the MSM has read them.
 int pipeline_slots(int log_m) {
     const int need = (int)((scal_group(log_m) + TILE_Q * 32 - 1) / (TILE_Q * 32));
-    return std::max(host_plan(log_m, false).plan.slots, (1 << (log_m - 1)) + need);
+    return std::max(host_plan(PLAN_PROJ, log_m).plan.slots, (1 << (log_m - 1)) + need);
 }
 
 struct SegLayout {
@@ -733,25 +755,25 @@ int reserve_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, bool
     return 0;
 }
 
-// The projection of the arenas D + d_off[k] (inputs stored) on st: one
+// The plan `kind` on the arenas D + d_off[k] (inputs stored) on st: one
 // persistent launch, or (staged) one launch per run of independent tasks.
 // `first` clears the error word too; a later pass of the same call keeps it.
-int run_projection(fk20_ctx *ctx, Workspace &ws, const SegLayout &lay, const int *log_m, const unsigned *rows, int nseg,
-                   bool half, bool first, int bps, cudaStream_t st) {
+int run_plan(fk20_ctx *ctx, Workspace &ws, const SegLayout &lay, const int *log_m, const unsigned *rows, int nseg,
+                   PlanKind kind, bool first, int bps, cudaStream_t st) {
     ProjArgs p{};
     const ProjPlan *plans[MAX_PROJ_SEGS];
     int G[MAX_PROJ_SEGS];
     Work prod;
     for (int k = 0; k < nseg; k++) {
-        const HostPlan &h = host_plan(log_m[k], half);
+        const HostPlan &h = host_plan(kind, log_m[k]);
         DevPlan d;
-        CKR(device_plan(ctx->device, log_m[k], half, &d));
+        CKR(device_plan(ctx->device, kind, log_m[k], &d));
         plans[k] = &h.plan;
         G[k] = lay.arena[k].G;
         p.seg[k] = ProjSeg{(uint4 *)ws.D.p + lay.d_off[k] / sizeof(uint4),
                            (unsigned *)((char *)ws.sync.p + SYNC_HDR + lay.r_off[k]), d.tasks, d.progs, lay.arena[k],
                            (int)h.plan.tasks.size(), h.plan.muls, h.plan.muls};
-        prod += proj_products(log_m[k], half) * (double)rows[k];
+        prod += plan_products(kind, log_m[k]) * (double)rows[k];
     }
     if (!host::build_proj_runs(p.runs, plans, G, nseg)) return FK20_EINVAL;
     p.nseg = nseg;
@@ -838,13 +860,13 @@ int run_pass(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, const fr_t *
         int log_m[MAX_PROJ_SEGS];
         unsigned rows[MAX_PROJ_SEGS];
         for (int k = 0; k < nseg; k++) log_m[k] = sg[k].log_m, rows[k] = sg[k].rows;
-        CKR(run_projection(ctx, ws, lay, log_m, rows, nseg, false, first, fft_bps, st));
+        CKR(run_plan(ctx, ws, lay, log_m, rows, nseg, PLAN_PROJ, first, fft_bps, st));
     }
     for (int k = 0; k < nseg; k++) {
-        TileView v{D + lay.d_off[k] / U, nullptr, lay.arena[k]};
+        TileView v{D + lay.d_off[k] / U, nullptr, lay.arena[k], 1};
         if (full) {
             DevPlan d;
-            CKR(device_plan(ctx->device, sg[k].log_m, false, &d));
+            CKR(device_plan(ctx->device, PLAN_PROJ, sg[k].log_m, &d));
             v.out = d.out;
         }
         if (proofs) {  // compressed, data-availability order (kernels_out.cu)
@@ -993,36 +1015,40 @@ int setup2xext(fk20_ctx *ctx, g1p_t *xext_fft, const g1p_t *setup, unsigned n, c
         launch_g1_stage(D, 1, log_m, s, 1, st);
         CKL();
     }
-    launch_tile_to_ref((uint64_t *)xext_fft, TileView{D, nullptr, {}}, nullptr, L_COLS, log_m, 0, st);
+    launch_tile_to_ref((uint64_t *)xext_fft, TileView{D, nullptr, {}, 0}, nullptr, L_COLS, log_m, 0, st);
     CKL();
     return 0;
 }
 
-// natural-order G1 transforms of `count` rows of m points
-int g1_transform(fk20_ctx *ctx, g1p_t *out, const g1p_t *in, int log_m, unsigned count, int inverse, cudaStream_t st) {
-    const int m = 1 << log_m;
-    const int G = (int)((count + 31) / 32);
-    CKR(ctx->D2.reserve(tile_bytes(G, m)));
-    uint4 *D = (uint4 *)ctx->D2.p;
-    if (!inverse) {  // bit-reversed load, DIT forward -> natural order
-        launch_ref_to_tile(D, (const uint64_t *)in, (int)count, G, log_m, 1, 0, st);
+// A plan on `rows` rows of m = 2^log_m points (reference layout, natural order
+// in and out; out may be in), at most PASS_ROWS rows at a time
+int run_points(fk20_ctx *ctx, PlanKind kind, g1p_t *out, const g1p_t *in, int log_m, unsigned rows, cudaStream_t st) {
+    const size_t m = (size_t)1 << log_m;
+    const int two = kind == PLAN_PROJ_HALF;
+    Workspace &ws = ctx->ws;
+    CKR(ws.init());
+    if (*ws.err_host) return launch_error(*ws.err_host);
+    DevPlan d;
+    CKR(device_plan(ctx->device, kind, log_m, &d));
+    const int slots = host_plan(kind, log_m).plan.slots;
+    const auto arena = [&](unsigned n) {
+        const int G = (int)((n + 31) / 32);
+        return two ? proj_arena(slots, n) : ProjArena{slots, G, G, 0};
+    };
+    const ProjArena most = arena(std::min(rows, PASS_ROWS));
+    CKR(ws.D.reserve(arena_bytes(most)));
+    CKR(ws.sync.reserve(SYNC_HDR + ready_bytes(most)));
+    for (unsigned r0 = 0; r0 < rows; r0 += PASS_ROWS) {
+        const unsigned n = std::min(rows - r0, PASS_ROWS);
+        SegLayout lay;
+        lay.arena[0] = arena(n);
+        lay.d_off[0] = lay.r_off[0] = 0;
+        lay.r_bytes = ready_bytes(lay.arena[0]);
+        launch_ref_to_arena((uint4 *)ws.D.p, lay.arena[0], (const uint64_t *)(in + r0 * m), (int)n, log_m, two, st);
         CKL();
-        for (int s = 0; s < log_m; s++) {
-            launch_g1_stage(D, G, log_m, s, 1, st);
-            CKL();
-        }
-        launch_tile_to_ref((uint64_t *)out, TileView{D, nullptr, {}}, nullptr, (int)count, log_m, 0, st);
-        CKL();
-    } else {  // natural load, DIF inverse -> bit-reversed, times 1/m, reorder on store
-        launch_ref_to_tile(D, (const uint64_t *)in, (int)count, G, log_m, 0, 0, st);
-        CKL();
-        for (int s = 0; s < log_m; s++) {
-            launch_g1_stage(D, G, log_m, s, 0, st);
-            CKL();
-        }
-        launch_g1_scale(D, G, log_m, 512 + log_m, st);
-        CKL();
-        launch_tile_to_ref((uint64_t *)out, TileView{D, nullptr, {}}, nullptr, (int)count, log_m, 1, st);
+        CKR(run_plan(ctx, ws, lay, &log_m, &n, 1, kind, r0 == 0, 0, st));
+        const TileView v{(const uint4 *)ws.D.p, d.out, lay.arena[0], two};
+        launch_tile_to_ref((uint64_t *)(out + r0 * m), v, nullptr, (int)n, log_m, 0, st);
         CKL();
     }
     return 0;
@@ -1253,7 +1279,7 @@ int fk20_ctx_msm(fk20_ctx *ctx, g1p_t *hext_fft, const fr_t *tc_fft, unsigned ro
     launch_ref_to_scalars((uint4 *)ctx->ws.S.p, (const uint64_t *)tc_fft, (int)rows, log_m, st);
     CKL();
     CKR(msm_launch(ctx, T, (uint4 *)ctx->ws.D.p, (const uint4 *)ctx->ws.S.p, G, (int)rows, 1, st));
-    CKR(output_launch(ctx->prof, (uint64_t *)hext_fft, TileView{(const uint4 *)ctx->ws.D.p, nullptr, {}}, nullptr, (int)rows,
+    CKR(output_launch(ctx->prof, (uint64_t *)hext_fft, TileView{(const uint4 *)ctx->ws.D.p, nullptr, {}, 0}, nullptr, (int)rows,
                       log_m, 0, st));
     return 0;
 }
@@ -1665,7 +1691,7 @@ int g1p_fft_n(g1p_t *output, const g1p_t *input, unsigned log_m, unsigned count,
     fk20_ctx *ctx;
     CKR(default_ctx(&ctx));
     std::lock_guard<std::mutex> lk(ctx->mu);
-    return g1_transform(ctx, output, input, (int)log_m, count, inverse, S_(stream));
+    return run_points(ctx, inverse ? PLAN_IDFT : PLAN_DFT, output, input, (int)log_m, count, S_(stream));
 }
 int g1p_fft(g1p_t *output, const g1p_t *input, unsigned count, void *stream) {
     return g1p_fft_n(output, input, 9, count, 0, stream);
@@ -1696,31 +1722,7 @@ int fk20_hext_fft2h_fft(g1p_t *h_fft, const g1p_t *hext_fft, unsigned rows, void
     fk20_ctx *ctx;
     CKR(default_ctx(&ctx));
     std::lock_guard<std::mutex> lk(ctx->mu);
-    cudaStream_t st = S_(stream);
-    const int log_m = 9, m = 512;
-    Workspace &ws = ctx->ws;
-    CKR(ws.init());
-    if (*ws.err_host) return launch_error(*ws.err_host);
-    DevPlan d;
-    CKR(device_plan(ctx->device, log_m, true, &d));
-    const int slots = host_plan(log_m, true).plan.slots;
-    const ProjArena most = proj_arena(slots, std::min(rows, PASS_ROWS));
-    CKR(ws.D.reserve(arena_bytes(most)));
-    CKR(ws.sync.reserve(SYNC_HDR + ready_bytes(most)));
-    for (unsigned r0 = 0; r0 < rows; r0 += PASS_ROWS) {
-        const unsigned n = std::min(rows - r0, PASS_ROWS);
-        SegLayout lay;
-        lay.arena[0] = proj_arena(slots, n);
-        lay.d_off[0] = lay.r_off[0] = 0;
-        lay.r_bytes = ready_bytes(lay.arena[0]);
-        launch_ref_to_arena((uint4 *)ws.D.p, lay.arena[0], (const uint64_t *)(hext_fft + (size_t)r0 * m), (int)n, log_m, st);
-        CKL();
-        CKR(run_projection(ctx, ws, lay, &log_m, &n, 1, true, r0 == 0, 0, st));
-        const TileView v{(const uint4 *)ws.D.p, d.out, lay.arena[0]};
-        launch_tile_to_ref((uint64_t *)(h_fft + (size_t)r0 * m), v, nullptr, (int)n, log_m, 0, st);
-        CKL();
-    }
-    return 0;
+    return run_points(ctx, PLAN_PROJ_HALF, h_fft, hext_fft, 9, rows, S_(stream));
 }
 
 int fk20_setup2xext_fft(g1p_t *xext_fft, const g1p_t *setup, void *stream) {
@@ -2314,7 +2316,7 @@ int cohort_launch(fk20_server *s, const std::vector<int> &act) {
         c.stage = p.blk.s_hi[k];
         if (c.stage < 2 * c.log_m - 1) continue;
         const int m = 1 << c.log_m;
-        launch_tile_to_ref((uint64_t *)b.dout.p, TileView{(const uint4 *)b.D.p, nullptr, {}}, nullptr, c.rows, c.log_m, 0, st);
+        launch_tile_to_ref((uint64_t *)b.dout.p, TileView{(const uint4 *)b.D.p, nullptr, {}, 0}, nullptr, c.rows, c.log_m, 0, st);
         CKL();
         CK(cudaMemcpyAsync(b.hout, b.dout.p, (size_t)c.rows * m * sizeof(g1p_t), cudaMemcpyDeviceToHost, st));
         CK(cudaEventRecord(b.out_done, st));

@@ -194,8 +194,10 @@ int proj_blocks_per_sm() {
 
 void launch_proj(const ProjArgs &p, int blocks, cudaStream_t st) { k_proj<<<blocks, FFT_THREADS, 0, st>>>(p); }
 
-// reference hext_fft rows [rows][m] -> arena inputs
-__global__ void k_ref_to_arena(uint4 *__restrict__ D, ProjArena A, const uint64_t *__restrict__ src, int rows, int log_m) {
+// reference rows [rows][m] -> arena inputs: of the two instances of a
+// projection, or of a transform (position c in slot c)
+__global__ void k_ref_to_arena(uint4 *__restrict__ D, ProjArena A, const uint64_t *__restrict__ src, int rows, int log_m,
+                               int two) {
     const int m = 1 << log_m;
     const size_t total = (size_t)(32 * A.F + 16 * A.paired) * m;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
@@ -204,14 +206,14 @@ __global__ void k_ref_to_arena(uint4 *__restrict__ D, ProjArena A, const uint64_
         if (row < rows) g1p_from_ref(p, src + 18 * e);
         else g1_set_inf(p);
         int g, lane;
-        (void)proj_lane(A, row, proj_in_inst(c), g, lane);
-        tile_store(D + proj_tile(A, g, proj_in_slot(c, log_m)), lane, p);
+        (void)proj_lane(A, row, two ? proj_in_inst(c) : 0, g, lane);
+        tile_store(D + proj_tile(A, g, two ? proj_in_slot(c, log_m) : c), lane, p);
     }
 }
 
-void launch_ref_to_arena(uint4 *D, const ProjArena &A, const uint64_t *src, int rows, int log_m, cudaStream_t st) {
+void launch_ref_to_arena(uint4 *D, const ProjArena &A, const uint64_t *src, int rows, int log_m, int two, cudaStream_t st) {
     const size_t lanes = (size_t)(32 * A.F + 16 * A.paired) << log_m;
-    k_ref_to_arena<<<grid_stride_blocks(lanes), 256, 0, st>>>(D, A, src, rows, log_m);
+    k_ref_to_arena<<<grid_stride_blocks(lanes), 256, 0, st>>>(D, A, src, rows, log_m, two);
 }
 
 }  // namespace fk

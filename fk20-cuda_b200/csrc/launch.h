@@ -78,14 +78,17 @@ struct ProjArgs {
 };
 int proj_blocks_per_sm();
 void launch_proj(const ProjArgs &p, int blocks, cudaStream_t st);
-void launch_ref_to_arena(uint4 *D, const ProjArena &A, const uint64_t *src, int rows, int log_m, cudaStream_t st);
+void launch_ref_to_arena(uint4 *D, const ProjArena &A, const uint64_t *src, int rows, int log_m, int two,
+                         cudaStream_t st);
 
 // Points read by the output kernels: natural tiles [G][m], or (out != null) an
-// arena whose slot out[k] holds position 2k + instance
+// arena.  Entry slot | neg << 16 | phi << 17 of out: position i is out[i], or
+// with two instances out[i / 2] of instance i mod 2, times (-1)^neg phi^phi.
 struct TileView {
     const uint4 *D;
-    const uint16_t *out;
+    const uint32_t *out;
     ProjArena arena;
+    int two;
 };
 
 // per-module constant upload (one per translation unit)

@@ -53,8 +53,11 @@ FK_D void view_load(G1P &p, const TileView &v, int row, int i, int m) {
         return;
     }
     int g, lane;
-    (void)proj_lane(v.arena, row, i & 1, g, lane);
-    tile_load(p, v.D + proj_tile(v.arena, g, v.out[i >> 1]), lane);
+    (void)proj_lane(v.arena, row, v.two ? i & 1 : 0, g, lane);
+    const uint32_t e = v.out[v.two ? i >> 1 : i];
+    tile_load(p, v.D + proj_tile(v.arena, g, (int)(e & 0xffffu)), lane);
+    if (e >> 17) fp_mul_beta(p.x, p.x, (int)(e >> 17));
+    if ((e >> 16) & 1u) f_neg(p.y, p.y);
 }
 
 // tile point -> strided slot (shared memory), one uint4 at a time, without

@@ -85,12 +85,12 @@ extern "C" int g1p_fft_noalloc(g1p_t *output, const g1p_t *input, unsigned log_m
     if (!inverse) {  // bit-reversed load, forward DIT stages -> natural order
         launch_ref_to_tile(D, (const uint64_t *)input, (int)count, G, L, 1, 0, st);
         for (int s = 0; s < L; s++) launch_g1_stage(D, G, L, s, 1, st);
-        launch_tile_to_ref((uint64_t *)output, TileView{D, nullptr, {}}, nullptr, (int)count, L, 0, st);
+        launch_tile_to_ref((uint64_t *)output, TileView{D, nullptr, {}, 0}, nullptr, (int)count, L, 0, st);
     } else {  // natural load, inverse DIF stages -> bit-reversed, times 1/m
         launch_ref_to_tile(D, (const uint64_t *)input, (int)count, G, L, 0, 0, st);
         for (int s = 0; s < L; s++) launch_g1_stage(D, G, L, s, 0, st);
         launch_g1_scale(D, G, L, 512 + L, st);
-        launch_tile_to_ref((uint64_t *)output, TileView{D, nullptr, {}}, nullptr, (int)count, L, 1, st);
+        launch_tile_to_ref((uint64_t *)output, TileView{D, nullptr, {}, 0}, nullptr, (int)count, L, 1, st);
     }
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : (int)e;

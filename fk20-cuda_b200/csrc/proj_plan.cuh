@@ -47,11 +47,10 @@ struct ProjLevel {
 };
 
 struct ProjPlan {
-    int log_m = 0, slots = 0, muls = 0;
-    bool half = false;  // the diagonal term by products with 1/2 (else by log_m - 1 doublings)
+    int slots = 0, muls = 0;
     std::vector<ProjTask> tasks;
     std::vector<ProjLevel> levels;
-    std::vector<uint16_t> out;                                // slot of output k
+    std::vector<uint32_t> out;                                // output k: slot | neg << 16 | phi << 17
     std::vector<std::array<uint64_t, 4>> scalars;             // the products' constants (standard form)
     double lin_products = 0;                                  // Fp products of the additions and doublings
 };
@@ -80,6 +79,11 @@ inline Fr fr_pow(const Fr &a, unsigned e) {
         if (e > 1) q = q * q;
     }
     return r;
+}
+inline int log2_of(int v) {
+    int l = 0;
+    while ((1 << l) < v) l++;
+    return l;
 }
 inline Fr fr_lambda() {  // z^2 - 1
     Fr t, r;
@@ -201,6 +205,18 @@ public:
             id = it->second;
         }
         return ProjRef{id, a.neg, a.phi};
+    }
+
+    ProjRef mul(int v, const Fr &c) {
+        Node n{PROJ_MUL, ProjRef{v, 0, 0}, {}};
+        n.c = (int)consts.size();
+        consts.push_back(c);
+        nodes.push_back(n);
+        return ProjRef{(int)nodes.size() - 1, 0, 0};
+    }
+    ProjRef mul(const ProjRef &a, const Fr &c) {
+        const ProjRef r = mul(a.v, c);
+        return ProjRef{r.v, a.neg, a.phi};
     }
 
     // the negacyclic product of length n: evaluation of x (n refs) appended to
@@ -393,104 +409,13 @@ private:
     }
 };
 
-// The plan of FFT size 2^log_m.  The inputs are hext_fft / 2^log_m (the bases of
-// the pipeline's tables carry the inverse FFT's factor) or, `half`, hext_fft itself.
-inline ProjPlan build_proj_plan(int log_m, bool half) {
-    const int m = 1 << log_m, H = m / 2;
-    ProjBuilder g;
-    std::vector<ProjRef> x(H);
-    for (int t = 0; t < H; t++) x[t] = ProjRef{g.input(), 0, 0};
-    // h_t = p(2t + 1), times m when the inputs are divided by m
-    std::vector<Fr> h(H);
-    const Fr w = fr_root(log_m), one = fr_from_u64(1);
-    for (int t = 0; t < H; t++) {
-        h[t] = fr_from_u64(2) * fr_inv(one - fr_pow(w, (unsigned)(2 * t + 1)));
-        if (half) h[t] = h[t] * fr_inv(fr_from_u64((uint64_t)m));
-    }
-    const Fr ihalf = fr_inv(fr_from_u64(2));
-    std::vector<ProjRef> ev;
-    std::vector<Fr> beta;
-    for (int n = H / 2; n >= 1; n /= 2) {  // X^(2n) - 1 = (X^n + 1)(X^n - 1)
-        std::vector<ProjRef> xn(n), xc(n);
-        std::vector<Fr> hn(n), hc(n);
-        for (int t = 0; t < n; t++) {
-            xc[t] = g.add(x[t], x[t + n]);
-            xn[t] = g.sub(x[t], x[t + n]);
-            hc[t] = ihalf * (h[t] + h[t + n]);
-            hn[t] = ihalf * (h[t] - h[t + n]);
-        }
-        g.negacyclic(n, xn, hn, ev, beta);
-        x = xc;
-        h = hc;
-    }
-    ev.push_back(x[0]);
-    beta.push_back(h[0]);
-    const int npre = (int)g.nodes.size();
-
-    // products: [beta coef^2] of the node itself, so that the transposed map starts at the node
-    std::map<int, Fr> prod;
-    const Fr lam = fr_lambda();
-    for (size_t s = 0; s < ev.size(); s++) {
-        const Fr c = beta[s] * fr_pow(lam, (unsigned)(2 * ev[s].phi % 3));
-        auto it = prod.find(ev[s].v);
-        if (it == prod.end()) prod[ev[s].v] = c;
-        else it->second = it->second + c;
-    }
-    std::vector<std::vector<ProjRef>> adj(npre);
-    std::vector<int> diag(H);
-    if (half)  // the diagonal term's x / 2: products too
-        for (int t = 0; t < H; t++) {
-            ProjBuilder::Node n{PROJ_MUL, ProjRef{t, 0, 0}, {}};
-            n.c = (int)g.consts.size();
-            g.consts.push_back(ihalf);
-            g.nodes.push_back(n);
-            diag[t] = (int)g.nodes.size() - 1;
-        }
-    else
-        for (int t = 0; t < H; t++) diag[t] = g.shl(ProjRef{t, 0, 0}, log_m - 1).v;
-    for (auto &p : prod) {
-        if (f_is_zero(p.second)) continue;
-        ProjBuilder::Node n{PROJ_MUL, ProjRef{p.first, 0, 0}, {}};
-        n.c = (int)g.consts.size();
-        g.consts.push_back(p.second);
-        g.nodes.push_back(n);
-        adj[p.first].push_back(ProjRef{(int)g.nodes.size() - 1, 0, 0});
-    }
-    // the transposed additions, in reverse order
-    const auto total = [&](std::vector<ProjRef> v) {
-        while (v.size() > 1) {
-            std::vector<ProjRef> nx;
-            for (size_t i = 0; i + 1 < v.size(); i += 2) nx.push_back(g.add(v[i], v[i + 1]));
-            if (v.size() & 1) nx.push_back(v.back());
-            v = nx;
-        }
-        return v.empty() ? ProjRef{} : v[0];
-    };
-    for (int v = npre - 1; v >= H; v--) {
-        const ProjRef s = total(adj[v]);
-        if (s.v < 0) continue;
-        const ProjBuilder::Node n = g.nodes[v];
-        if (n.op == PROJ_LIN) {
-            adj[n.a.v].push_back(s);
-            adj[n.b.v].push_back(ProjBuilder::times(s, n.b.neg, n.b.phi));
-        } else {  // SHL
-            adj[n.a.v].push_back(g.shl(s, n.sh));
-        }
-    }
-    std::vector<int> outs(H);
-    for (int k = 0; k < H; k++) {
-        const ProjRef c = total(adj[k]);
-        ProjBuilder::Node n{PROJ_OUT, c, {}};
-        n.cross0 = diag[(H - k) & (H - 1)];   // instance 0 reads x[2k] from instance 1
-        n.cross1 = diag[H - 1 - k];           // instance 1 reads x[2k + 1] from instance 0
-        g.nodes.push_back(n);
-        outs[k] = (int)g.nodes.size() - 1;
-    }
-
+// Tasks, levels and slots of the graph's nodes that the outputs need; nodes 0 ..
+// inputs - 1 are the inputs, in slots of the same number.
+inline ProjPlan finish_plan(const ProjBuilder &g, int inputs, const std::vector<ProjRef> &outs) {
     // ---- live nodes, pairs (a + b, a - b), doublings folded into their only user
     const int N = (int)g.nodes.size();
     std::vector<char> live(N, 0);
-    for (int k : outs) live[k] = 1;
+    for (const ProjRef &k : outs) live[k.v] = 1;
     for (int v = N - 1; v >= 0; v--) {
         if (!live[v]) continue;
         const auto &n = g.nodes[v];
@@ -584,8 +509,6 @@ inline ProjPlan build_proj_plan(int log_m, bool half) {
     // when it runs.  Tasks of the last phase wait until every product of their
     // group is done, so all readers of the first two phases are above them.
     ProjPlan P;
-    P.log_m = log_m;
-    P.half = half;
     std::vector<int> slot(N, -1), ver(N, 0), pos(NT, 0);
     std::vector<std::vector<int>> readers(N);
     for (int k = 0; k < NT; k++) pos[order[k]] = k;
@@ -603,8 +526,9 @@ inline ProjPlan build_proj_plan(int log_m, bool half) {
     std::vector<std::pair<uint16_t, uint8_t>> wrote(NT);  // slot and version of each task's d0
     std::vector<int> left(N);  // readers not yet placed
     for (int v = 0; v < N; v++) left[v] = (int)readers[v].size();
-    for (int t = 0; t < H; t++) slot[t] = t;
-    int next = H;
+    for (const ProjRef &k : outs) left[k.v]++;  // outputs are never written over
+    for (int t = 0; t < inputs; t++) slot[t] = t;
+    int next = inputs;
     int last_level = -1, last_phase = -1;
     for (int i : order) {
         const Task &t = tasks[i];
@@ -671,8 +595,207 @@ inline ProjPlan build_proj_plan(int log_m, bool half) {
     }
     P.slots = next;
     P.muls = (int)P.scalars.size();
-    for (int k = 0; k < H; k++) P.out.push_back((uint16_t)slot[outs[k]]);
+    for (const ProjRef &k : outs) P.out.push_back((uint32_t)slot[k.v] | (uint32_t)k.neg << 16 | (uint32_t)k.phi << 17);
     return P;
+}
+
+// the sum of v, as a tree
+inline ProjRef total(ProjBuilder &g, std::vector<ProjRef> v) {
+    while (v.size() > 1) {
+        std::vector<ProjRef> nx;
+        for (size_t i = 0; i + 1 < v.size(); i += 2) nx.push_back(g.add(v[i], v[i + 1]));
+        if (v.size() & 1) nx.push_back(v.back());
+        v = nx;
+    }
+    return v.empty() ? ProjRef{} : v[0];
+}
+
+// The projection of FFT size 2^log_m.  The inputs are hext_fft / 2^log_m (the bases of
+// the pipeline's tables carry the inverse FFT's factor) or, `half`, hext_fft itself.
+inline ProjPlan build_proj_plan(int log_m, bool half) {
+    const int m = 1 << log_m, H = m / 2;
+    ProjBuilder g;
+    std::vector<ProjRef> x(H);
+    for (int t = 0; t < H; t++) x[t] = ProjRef{g.input(), 0, 0};
+    // h_t = p(2t + 1), times m when the inputs are divided by m
+    std::vector<Fr> h(H);
+    const Fr w = fr_root(log_m), one = fr_from_u64(1);
+    for (int t = 0; t < H; t++) {
+        h[t] = fr_from_u64(2) * fr_inv(one - fr_pow(w, (unsigned)(2 * t + 1)));
+        if (half) h[t] = h[t] * fr_inv(fr_from_u64((uint64_t)m));
+    }
+    const Fr ihalf = fr_inv(fr_from_u64(2));
+    std::vector<ProjRef> ev;
+    std::vector<Fr> beta;
+    for (int n = H / 2; n >= 1; n /= 2) {  // X^(2n) - 1 = (X^n + 1)(X^n - 1)
+        std::vector<ProjRef> xn(n), xc(n);
+        std::vector<Fr> hn(n), hc(n);
+        for (int t = 0; t < n; t++) {
+            xc[t] = g.add(x[t], x[t + n]);
+            xn[t] = g.sub(x[t], x[t + n]);
+            hc[t] = ihalf * (h[t] + h[t + n]);
+            hn[t] = ihalf * (h[t] - h[t + n]);
+        }
+        g.negacyclic(n, xn, hn, ev, beta);
+        x = xc;
+        h = hc;
+    }
+    ev.push_back(x[0]);
+    beta.push_back(h[0]);
+    const int npre = (int)g.nodes.size();
+
+    // products: [beta coef^2] of the node itself, so that the transposed map starts at the node
+    std::map<int, Fr> prod;
+    const Fr lam = fr_lambda();
+    for (size_t s = 0; s < ev.size(); s++) {
+        const Fr c = beta[s] * fr_pow(lam, (unsigned)(2 * ev[s].phi % 3));
+        auto it = prod.find(ev[s].v);
+        if (it == prod.end()) prod[ev[s].v] = c;
+        else it->second = it->second + c;
+    }
+    std::vector<std::vector<ProjRef>> adj(npre);
+    std::vector<int> diag(H);
+    if (half)  // the diagonal term's x / 2: products too
+        for (int t = 0; t < H; t++)
+            diag[t] = g.mul(t, ihalf).v;
+    else
+        for (int t = 0; t < H; t++) diag[t] = g.shl(ProjRef{t, 0, 0}, log_m - 1).v;
+    for (auto &p : prod) {
+        if (f_is_zero(p.second)) continue;
+        adj[p.first].push_back(g.mul(p.first, p.second));
+    }
+    // the transposed additions, in reverse order
+    for (int v = npre - 1; v >= H; v--) {
+        const ProjRef s = total(g, adj[v]);
+        if (s.v < 0) continue;
+        const ProjBuilder::Node n = g.nodes[v];
+        if (n.op == PROJ_LIN) {
+            adj[n.a.v].push_back(s);
+            adj[n.b.v].push_back(ProjBuilder::times(s, n.b.neg, n.b.phi));
+        } else {  // SHL
+            adj[n.a.v].push_back(g.shl(s, n.sh));
+        }
+    }
+    std::vector<ProjRef> outs(H);
+    for (int k = 0; k < H; k++) {
+        const ProjRef c = total(g, adj[k]);
+        ProjBuilder::Node n{PROJ_OUT, c, {}};
+        n.cross0 = diag[(H - k) & (H - 1)];   // instance 0 reads x[2k] from instance 1
+        n.cross1 = diag[H - 1 - k];           // instance 1 reads x[2k + 1] from instance 0
+        g.nodes.push_back(n);
+        outs[k] = ProjRef{(int)g.nodes.size() - 1, 0, 0};
+    }
+    return finish_plan(g, H, outs);
+}
+
+
+// ---------------------------------------------------------------- whole transforms
+// The negacyclic Hankel map of length n with functional h on x: its graph is
+// built apart, copied in, and run backwards to the n outputs.
+inline std::vector<ProjRef> hankel(ProjBuilder &g, const std::vector<ProjRef> &x, const std::vector<Fr> &h) {
+    const int n = (int)x.size();
+    ProjBuilder e;
+    std::vector<ProjRef> in(n), out;
+    std::vector<Fr> beta;
+    for (int t = 0; t < n; t++) in[t] = ProjRef{e.input(), 0, 0};
+    e.negacyclic(n, in, h, out, beta);
+    const auto coef = [](ProjRef r, ProjRef by) { return ProjBuilder::times(r, by.neg, by.phi); };
+    std::vector<ProjRef> at(e.nodes.size());
+    for (size_t v = 0; v < e.nodes.size(); v++) {
+        const auto &nd = e.nodes[v];
+        if (nd.op < 0) at[v] = x[v];
+        else if (nd.op == PROJ_LIN) at[v] = g.add(at[nd.a.v], coef(at[nd.b.v], nd.b));
+        else at[v] = g.shl(at[nd.a.v], nd.sh);
+    }
+    std::vector<std::vector<ProjRef>> adj(e.nodes.size());
+    const Fr lam = fr_lambda();
+    for (size_t s = 0; s < out.size(); s++) {
+        if (f_is_zero(beta[s])) continue;
+        const ProjRef v = at[out[s].v];  // the node's place in g, with its own coefficient
+        Fr c = beta[s] * fr_pow(lam, (unsigned)((2 * out[s].phi + v.phi) % 3));
+        if (v.neg) c = fr_from_u64(0) - c;
+        adj[out[s].v].push_back(g.mul(v.v, c));
+    }
+    for (int v = (int)e.nodes.size() - 1; v >= n; v--) {
+        const ProjRef s = total(g, adj[v]);
+        if (s.v < 0) continue;
+        const auto &nd = e.nodes[v];
+        if (nd.op == PROJ_LIN) {
+            adj[nd.a.v].push_back(s);
+            adj[nd.b.v].push_back(coef(s, nd.b));
+        } else {
+            adj[nd.a.v].push_back(g.shl(s, nd.sh));
+        }
+    }
+    std::vector<ProjRef> y(n);
+    for (int t = 0; t < n; t++) y[t] = total(g, adj[t]);
+    return y;
+}
+
+// sum_{j < d/2} u_j w_d^(sign j k) times `scale` at the odd k < d, in order
+// (d = 2 u.size()).  Even j give the same sums of half the length.  Odd j and
+// odd k are +-5^b mod d, and 5^(d/8) = 1 + d/2 turns the sign: with the sums
+// and differences over +-, two negacyclic Hankel maps of length d/8.
+inline std::vector<ProjRef> odd_sums(ProjBuilder &g, const std::vector<ProjRef> &u, const Fr &w, const Fr &scale,
+                                     bool scaled) {
+    const int half = (int)u.size(), d = 2 * half;
+    if (d == 2) return {scaled ? g.mul(u[0], scale) : u[0]};
+    std::vector<ProjRef> ue;
+    for (int j = 0; j < half; j += 2) ue.push_back(u[j]);
+    const std::vector<ProjRef> E = odd_sums(g, ue, w * w, scale, scaled);
+    std::vector<ProjRef> O(half / 2);  // odd k < d/2
+    if (d == 4) {
+        O[0] = g.mul(u[1], w * scale);
+    } else {
+        const int n = d / 8;
+        std::vector<ProjRef> v[2], p(n), q(n);
+        std::vector<Fr> hp(n), hm(n);
+        std::vector<int> res(n);
+        const Fr ih = fr_inv(fr_from_u64(2)) * scale, iw = fr_inv(w);
+        const auto pick = [&](int r) { return r < half ? u[r] : ProjBuilder::times(u[r - half], 1, 0); };
+        for (int b = 0, r = 1; b < n; b++, r = r * 5 % d) {
+            res[b] = r;
+            const ProjRef x = pick(r), y = pick(d - r);
+            p[b] = g.add(x, y), q[b] = g.sub(x, y);
+            const Fr c0 = fr_pow(w, (unsigned)r), c1 = fr_pow(iw, (unsigned)r);
+            hp[b] = ih * (c0 + c1), hm[b] = ih * (c0 - c1);
+        }
+        const std::vector<ProjRef> A = hankel(g, p, hp), B = hankel(g, q, hm);
+        for (int b = 0; b < n; b++) {
+            const ProjRef y[2] = {g.add(A[b], B[b]), g.sub(A[b], B[b])};
+            const int k[2] = {res[b], d - res[b]};
+            for (int a = 0; a < 2; a++) {  // k + d/2 has the opposite sign
+                if (k[a] < half) O[k[a] / 2] = y[a];
+                else O[(k[a] - half) / 2] = ProjBuilder::times(y[a], 1, 0);
+            }
+        }
+    }
+    std::vector<ProjRef> out(half);
+    for (int i = 0; i < half / 2; i++) out[i] = g.add(E[i], O[i]), out[i + half / 2] = g.sub(E[i], O[i]);
+    return out;
+}
+
+// The transform of 2^log_m points, or its inverse with the factor 1/m: input j
+// in slot j, output k in out[k].  1,388 products at m = 512 (the inverse 1,398,
+// its factor on every product and on the few values that meet none), one deep;
+// radix 2 takes 1,793 (2,305), nine (ten) deep.  B200: 32 inverse transforms of
+// 512 points 12.8 -> 4.9 ms.
+inline ProjPlan build_dft_plan(int log_m, bool inverse) {
+    const int m = 1 << log_m;
+    ProjBuilder g;
+    std::vector<ProjRef> x(m), out(m);
+    for (int t = 0; t < m; t++) x[t] = ProjRef{g.input(), 0, 0};
+    const Fr scale = inverse ? fr_inv(fr_from_u64((uint64_t)m)) : fr_from_u64(1);
+    for (int d = m, step = 1; d > 1; d /= 2, step *= 2) {  // outputs k = step * odd
+        const Fr w = inverse ? fr_inv(fr_root(log2_of(d))) : fr_root(log2_of(d));
+        std::vector<ProjRef> s, t;
+        for (int j = 0; j < d / 2; j++) s.push_back(g.add(x[j], x[j + d / 2])), t.push_back(g.sub(x[j], x[j + d / 2]));
+        const std::vector<ProjRef> y = odd_sums(g, t, w, scale, inverse);
+        for (int i = 0; i < d / 2; i++) out[step * (2 * i + 1)] = y[i];
+        x = s;
+    }
+    out[0] = inverse ? g.mul(x[0], scale) : x[0];
+    return finish_plan(g, m, out);
 }
 
 // The launch order over segments of plans p[k] with G[k] groups: phase by

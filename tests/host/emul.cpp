@@ -166,14 +166,15 @@ int emul_glv_split(uint64_t *out, const uint64_t *s, long count) {
 
 #include "proj_plan.cuh"
 extern "C" {
-// The projection plan of FFT size 2^log_m (proj_plan.cuh).  head: slots, tasks,
+// The plan of FFT size 2^log_m (proj_plan.cuh): kind 0 projection, 1 projection of
+// unscaled inputs, 2 transform, 3 inverse transform.  head: slots, tasks,
 // products, outputs, levels.  tasks: 16 ints each (op, sh, phi, neg, d0, d1, a,
 // b, b2, va, vb, vb2, w0, w1, phase, prog); scalars: 4 x u64 each; levels:
 // (first, count, phase).  Arrays may be null (sizes only).
-int emul_proj_plan(int log_m, int half, int *head, int *tasks, uint64_t *scalars, int *out, int *levels) {
-    static ProjPlan plans[2][10];
-    ProjPlan &p = plans[half][log_m];
-    if (p.tasks.empty()) p = host::build_proj_plan(log_m, half != 0);
+int emul_proj_plan(int log_m, int kind, int *head, int *tasks, uint64_t *scalars, int *out, int *levels) {
+    static ProjPlan plans[4][10];
+    ProjPlan &p = plans[kind][log_m];
+    if (p.tasks.empty()) p = kind < 2 ? host::build_proj_plan(log_m, kind == 1) : host::build_dft_plan(log_m, kind == 3);
     head[0] = p.slots, head[1] = (int)p.tasks.size(), head[2] = p.muls, head[3] = (int)p.out.size();
     head[4] = (int)p.levels.size();
     if (!tasks) return 0;
@@ -184,7 +185,7 @@ int emul_proj_plan(int log_m, int half, int *head, int *tasks, uint64_t *scalars
     }
     for (int i = 0; i < p.muls; i++)
         for (int k = 0; k < 4; k++) scalars[4 * i + k] = p.scalars[i][k];
-    for (size_t i = 0; i < p.out.size(); i++) out[i] = p.out[i];
+    for (size_t i = 0; i < p.out.size(); i++) out[i] = (int)p.out[i];
     for (size_t i = 0; i < p.levels.size(); i++)
         levels[3 * i] = p.levels[i].first, levels[3 * i + 1] = p.levels[i].count, levels[3 * i + 2] = p.levels[i].phase;
     return 0;

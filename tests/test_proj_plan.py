@@ -1,6 +1,6 @@
-"""The projection plans (csrc/proj_plan.cuh): hext_fft -> h_fft as additions and
-one layer of fixed-scalar products, replayed on Fr values against the two
-transforms they replace; the dependencies and slot reuse the kernel relies on;
+"""The plans of additions and one layer of fixed-scalar products
+(csrc/proj_plan.cuh), hext_fft -> h_fft and whole transforms, replayed on Fr
+values against the transforms they replace; the dependencies and slot reuse the kernel relies on;
 the launch order; the shared P + Q / P - Q formulas."""
 import ctypes
 import os
@@ -42,14 +42,18 @@ def load_plan(emul, log_m, half):
     return slots, tasks.tolist(), [O.limbs_to_int(v) for v in sc], out.tolist(), lev.tolist()
 
 
-@pytest.mark.parametrize("log_m,half", [(7, 0), (8, 0), (9, 0), (9, 1)])
-def test_plan_replayed_on_scalars(emul, log_m, half):
+PLANS = [(7, 0), (8, 0), (9, 0), (9, 1)] + [(l, k) for l in range(1, 10) for k in (2, 3)]
+
+
+@pytest.mark.parametrize("log_m,kind", PLANS)
+def test_plan_replayed_on_scalars(emul, log_m, kind):
     """In task order every read finds the version it asks for; the outputs are
-    FFT(upper half zeroed(IFFT)) of the inputs; and a slot is written over only
+    FFT(upper half zeroed(IFFT)) of the inputs (kinds 0 and 1, two instances a
+    row) or their transform (2) or inverse transform (3); and a slot is written over only
     by a task that depends on every reader of the old value (or, after the
     products, when all readers ran before or as products)."""
     m, H = 1 << log_m, 1 << (log_m - 1)
-    slots, tasks, scalars, out, levels = load_plan(emul, log_m, half)
+    slots, tasks, scalars, out, levels = load_plan(emul, log_m, kind)
     rng = np.random.default_rng(log_m)
     x = [int(v) for v in rng.integers(0, 2**62, m)]
     w = O.root_of_unity(m)
@@ -58,10 +62,13 @@ def test_plan_replayed_on_scalars(emul, log_m, half):
     s_, i_ = ctypes.c_int(), ctypes.c_int()
     seen = set()
     for c in range(m):
+        if kind > 1:
+            val[0][c] = x[c]
+            continue
         emul.emul_proj_in(c, log_m, ctypes.byref(s_), ctypes.byref(i_))
         assert 0 <= s_.value < H and (s_.value, i_.value) not in seen
         seen.add((s_.value, i_.value))
-        val[i_.value][s_.value] = x[c] if half else x[c] * inv_m % R
+        val[i_.value][s_.value] = x[c] if kind else x[c] * inv_m % R
     ver = [0] * slots
     wrote = {}
     readers = [[] for _ in range(slots)]
@@ -69,6 +76,11 @@ def test_plan_replayed_on_scalars(emul, log_m, half):
     cross = set()
     phi = [1, LAMBDA, LAMBDA * LAMBDA % R]
     phase_before = 0
+    last = [0] * slots  # final version of each slot
+    for t in tasks:
+        for d, wv in ((t[4], t[12]), (t[5], t[13])):
+            if d != NONE:
+                last[d] = max(last[d], wv)
     for k, (op, sh, ph, neg, d0, d1, a, b, b2, va, vb, vb2, w0, w1, phase, prog) in enumerate(tasks):
         assert phase >= phase_before and (op == MUL) == (phase == 1)
         phase_before = phase
@@ -102,6 +114,7 @@ def test_plan_replayed_on_scalars(emul, log_m, half):
             else:
                 res.append(((A * phi[ph] * (-1 if neg else 1) + val[1 - inst][b2 if inst else b]) % R,))
         for n, (d, wv) in enumerate([(d0, w0)] + ([(d1, w1)] if d1 != NONE else [])):
+            assert not any(e & 0xFFFF == d and ver[d] == last[d] for e in out)  # outputs stay
             for r in readers[d]:
                 assert r == k or r in anc or (phase == 2 and tasks[r][14] < 2), (k, d, r)
             assert d not in cross and wv == ver[d] + 1 and wv < 256
@@ -116,12 +129,19 @@ def test_plan_replayed_on_scalars(emul, log_m, half):
     for _ in range(m - 1):
         pw.append(pw[-1] * w % R)
         pi.append(pi[-1] * wi % R)
-    h = [sum(x[c] * pi[j * c % m] for c in range(m)) * inv_m % R for j in range(H)]
+    h = [sum(x[c] * pi[j * c % m] for c in range(m)) * inv_m % R for j in range(H)] if kind < 2 else []
     for k in range(0, m, 1 if m < 512 else 5):
-        assert val[k & 1][out[k >> 1]] == sum(h[j] * pw[j * k % m] for j in range(H)) % R, k
+        if kind < 2:
+            got, exp = val[k & 1][out[k >> 1]], sum(h[j] * pw[j * k % m] for j in range(H)) % R
+        else:
+            e = out[k]
+            got = val[0][e & 0xFFFF] * phi[e >> 17] * (-1 if (e >> 16) & 1 else 1) % R
+            tw, f = (pw, 1) if kind == 2 else (pi, inv_m)
+            exp = sum(x[j] * tw[j * k % m] for j in range(m)) * f % R
+        assert got == exp, k
 
 
-@pytest.mark.parametrize("log_m,half", [(7, 0), (8, 0), (9, 0), (9, 1)])
+@pytest.mark.parametrize("log_m,half", PLANS)
 def test_plan_programs_avoid_exceptional_additions(emul, log_m, half):
     """As for the twiddle programs: no partial sum of a product's program meets
     the added point, its negative or infinity."""
