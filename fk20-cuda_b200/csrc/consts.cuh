@@ -15,7 +15,7 @@ constexpr int L_COLS = 16;       // l: toeplitz columns per row (fk20_multi_cuda
 
 // fixed-scalar programs: read with warp-uniform addresses (one broadcast per load)
 static __device__ uint32_t c_prog[NPROG][PROG_WORDS];
-static __device__ uint32_t g_fr_tw[512][8];   // w_512^t * 2^256 mod r (Montgomery form)
+static __device__ __align__(16) uint32_t g_fr_tw[512][8];   // w_512^t * 2^256 mod r (Montgomery form)
 static __device__ uint32_t g_fr_inv2[16][8];  // 2^-s * 2^256 mod r
 
 struct HostConsts {

@@ -1,0 +1,24 @@
+"""Every size of the Fr transform, with counts that leave a block's last
+transforms unused, in place as well."""
+import numpy as np
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("log_m", range(1, 10))
+@pytest.mark.parametrize("inverse", [0, 1])
+def test_fr_fft_every_size(engine, log_m, inverse):
+    m = 1 << log_m
+    count = 1024 // m + 3
+    x = O.seeded_fr(40 + log_m, count * m).reshape(count, m, 4)
+    x[0, :] = O.int_to_limbs(O.R - 1, 4)
+    d = engine.to_device(x)
+    out = engine.empty(x.shape)
+    exp = O.fr_fft(x, inverse=bool(inverse))
+    engine.call("fr_fft_n", engine._ptr(out), engine._ptr(d), log_m, count, inverse, engine._stream())
+    assert np.array_equal(engine.to_host(out), exp)
+    engine.call("fr_fft_n", engine._ptr(d), engine._ptr(d), log_m, count, inverse, engine._stream())
+    assert np.array_equal(engine.to_host(d), exp)
