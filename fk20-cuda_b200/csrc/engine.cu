@@ -1769,21 +1769,19 @@ int fk20_ctx_check_proof_multi(fk20_ctx *ctx, uint8_t *ok, const g1p_t *commitme
     const int G = (int)((count + 31) / 32);
     const size_t poly_b = (size_t)count * COMMIT_CHUNK * sizeof(fr_t), xl_b = (size_t)count * sizeof(fr_t),
                  pt_b = (size_t)count * sizeof(g1p_t);
-    CKR(ctx->verify.reserve(poly_b + xl_b + 3 * pt_b));
+    CKR(ctx->verify.reserve(poly_b + xl_b + 2 * pt_b));
     CKR(ctx->commit.part.reserve(tile_bytes(G, commit_parts((int)count, (int)COMMIT_CHUNK))));
     char *base = (char *)ctx->verify.p;
     uint64_t *poly = (uint64_t *)base, *xl = (uint64_t *)(base + poly_b);
-    uint64_t *I = (uint64_t *)(base + poly_b + xl_b), *T = I + 18 * (size_t)count, *A = T + 18 * (size_t)count;
+    uint64_t *I = (uint64_t *)(base + poly_b + xl_b), *A = I + 18 * (size_t)count;
     const cudaStream_t st = S_(stream);
     // I(X) over the coset and x^l; [I(s)]G1 with the commitment tables
     launch_interp(poly, xl, (const uint64_t *)x, (const uint64_t *)ys, log_l, count, st);
     launch_commit(I, (uint4 *)ctx->commit.part.p, poly, (const uint4 *)ctx->commit.table.p, (int)count,
                   (int)COMMIT_CHUNK, ctx->commit.W, ctx->commit.cb, st);
     // e(C - [I(s)] + [x^l] proof, G2) == e(proof, [s^l]G2)
-    launch_g1_op(4, T, (const uint64_t *)proof, xl, count, st);
-    launch_g1_op(3, A, (const uint64_t *)commitment, I, count, st);
-    launch_g1_op(0, I, A, T, count, st);
-    launch_pairing(1, nullptr, ok, I, (const uint64_t *)setup_g2, (const uint64_t *)proof,
+    launch_verify_points(A, (const uint64_t *)commitment, I, (const uint64_t *)proof, xl, count, st);
+    launch_pairing(1, nullptr, ok, A, (const uint64_t *)setup_g2, (const uint64_t *)proof,
                    (const uint64_t *)(setup_g2 + l), count, st, 3);
     CKL();
     return 0;

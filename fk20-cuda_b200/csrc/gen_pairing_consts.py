@@ -18,6 +18,10 @@ Run from this directory: python gen_pairing_consts.py > pairing_consts.inc"""
 P = 0x1A0111EA397FE69A4B1BA7B6434BACD764774B84F38512BF6730D2A0F6B0F6241EABFFFEB153FFFFB9FEFFFFFFFFAAAB
 R = 0x73EDA753299D7D483339D80809A1D80553BDA402FFFE5BFEFFFFFFFF00000001
 Z = -0xD201000000010000
+G2 = (0x024AA2B2F08F0A91260805272DC51051C6E47AD4FA403B02B4510B647AE3D1770BAC0326A805BBEFD48056C8C121BDB8,
+      0x13E02B6052719F607DACD3A088274F65596BD0D09920B61AB5DA61BBDC7F5049334CF11213945D57E5AC7D055D042B7E,
+      0x0CE5D527727D6E118CC9CDC6DA2E351AADFD9BAA8CBDD3A76D429A695160D12C923AC9CC3BACA289E193548608B82801,
+      0x0606C4A02EA734CC32ACD2B02BC28B99CB3E287E85A763AF267492AB572E99AB3F370D275CEC1DA1AAA9075FF05F79BE)
 assert (P ** 12 - 1) % R == 0 and (P ** 4 - P ** 2 + 1) % R == 0
 assert 3 * (P ** 4 - P ** 2 + 1) // R == (Z - 1) ** 2 * (Z + P) * (Z ** 2 + P ** 2 - 1) + 3
 
@@ -62,6 +66,10 @@ assert pow(w32, 16, R) == R - 1
 print("__device__ const uint32_t c_w32_inv[32][8] = {")
 for k in range(32):
     print(f"    {{{fr_limbs(pow(w32, (32 - k) % 32, R))}}},")
+print("};")
+print("__device__ const uint32_t c_g2_gen[4][12] = {  // the G2 generator's x and y")
+for v in G2:
+    print(f"    {{{limbs(v)}}},")
 print("};")
 print("__device__ const uint32_t c_inv_pow2[6][8] = {")
 for j in range(6):

@@ -28,13 +28,21 @@
 //     inverses of the cyclotomic subgroup).  A fixed exponent coprime to r
 //     keeps a check's answer the same: f^(3(p^12-1)/r) == 1 exactly when
 //     f^((p^12-1)/r) == 1.
-// One thread per pairing or check; field elements live in local memory and
-// the Fp2 / Fp6 / Fp12 products are out-of-line routines, which keeps the
-// code small.
+// Two kernels.  One warp per pairing or check (k_pairing): its Fp values are
+// slots in shared memory and the steps above are programs of rounds
+// (pairing_prog.inc, traced and scheduled by gen_pairing_prog.py); a round
+// gives every lane one Fp product or one sum, so a Miller step with both lines
+// is 8 products deep instead of 226, and a cyclotomic square 1 instead of 18.
+// One thread per check (k_pairing_threads), its values in local memory and the
+// Fp2 / Fp6 / Fp12 products out of line, is thousands of products
+// deep but needs fewer instructions, so it takes over where checks fill the
+// chip (launch_pairing).
 #define FK_FP_MUL_OUTLINE 1
+#include "glv.cuh"
 #include "launch.h"
 #include "layout.cuh"
 #include "tower.cuh"
+#include "pairing_prog.inc"
 
 namespace fk {
 
@@ -269,11 +277,264 @@ static __device__ __noinline__ void g2_add(Fp2 *xr, Fp2 *yr, bool *ir, Fp2 x1, F
     *ir = false;
 }
 
+// ---------------------------------------------------------------- the 32-lane machine
+constexpr int PV_WARPS = 2;  // checks per block
+
+FK_D void pv_load(Fp &f, const uint32_t *sm, int slot) {
+    const uint4 *q = reinterpret_cast<const uint4 *>(sm + 12 * slot);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const uint4 v = q[k];
+        f.w[4 * k] = v.x; f.w[4 * k + 1] = v.y; f.w[4 * k + 2] = v.z; f.w[4 * k + 3] = v.w;
+    }
+}
+FK_D void pv_store(uint32_t *sm, int slot, const Fp &f) {
+    uint4 *q = reinterpret_cast<uint4 *>(sm + 12 * slot);
+#pragma unroll
+    for (int k = 0; k < 3; k++) q[k] = make_uint4(f.w[4 * k], f.w[4 * k + 1], f.w[4 * k + 2], f.w[4 * k + 3]);
+}
+// x or p - x (p for x = 0: a product or a sum takes it)
+FK_D void pv_load_signed(Fp &f, const uint32_t *sm, int slot, bool neg) {
+    pv_load(f, sm, slot);
+    uint32_t m[12], t[12];
+#pragma unroll
+    for (int k = 0; k < 12; k++) m[k] = FpDesc::mod(k);
+    (void)ch_sub<FpDesc>(t, m, f.w);
+#pragma unroll
+    for (int k = 0; k < 12; k++) f.w[k] = neg ? t[k] : f.w[k];
+}
+// acc < 2^7 p as 12 column sums below 2^39, reduced
+FK_D void pv_reduce(Fp &r, const uint64_t acc[12]) {
+    uint32_t t[13];
+    uint64_t c = 0;
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+        c += acc[k];
+        t[k] = (uint32_t)c;
+        c >>= 32;
+    }
+    t[12] = (uint32_t)c;
+    // q = floor(top / (top of p + 1)): at most one below acc div p
+    const uint64_t h = ((uint64_t)t[12] << 32) | t[11];
+    const uint32_t q = (uint32_t)(h / (FpDesc::mod(11) + 1u));
+    int64_t b = 0;
+    uint32_t u[12];
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+        b += (int64_t)t[k] - (int64_t)((uint64_t)q * FpDesc::mod(k));
+        u[k] = (uint32_t)b;
+        b >>= 32;
+    }
+    f_reduce_once<FpDesc>(r.w, u);
+}
+static __device__ __noinline__ void pv_run(uint32_t *sm, int at, int rounds, int lane) {
+#pragma unroll 1
+    for (int i = 0; i < rounds; i++) {
+        const int head = c_pv_head[at + i];
+        const uint4 w = c_pv_code[at + i][lane];
+        Fp r;
+        if (head < 8) {
+            Fp a, b, t;
+            pv_load_signed(a, sm, (w.x >> 8) & 255, w.y & 0x100u);
+            pv_load_signed(b, sm, w.x >> 24, w.y & 0x400u);
+            if (head) {
+                pv_load_signed(t, sm, (w.x >> 16) & 255, w.y & 0x200u);
+                f_add(a, a, t);
+                pv_load_signed(t, sm, w.y & 255, w.y & 0x800u);
+                f_add(b, b, t);
+            }
+            fp_mul(r, a, b);
+        } else {
+            uint64_t acc[12];
+#pragma unroll
+            for (int k = 0; k < 12; k++) acc[k] = 0;
+            const int n = head - 8;
+#pragma unroll 1
+            for (int k = 1; k <= n; k++) {
+                const uint32_t word = k < 2 ? w.x : k < 4 ? w.y : k < 6 ? w.z : w.w;
+                const uint32_t e = (k & 1) ? word >> 16 : word & 0xffffu;
+                const int cf = (int)(int8_t)(e >> 8);
+                const uint32_t mag = (uint32_t)(cf < 0 ? -cf : cf);
+                Fp x;
+                pv_load_signed(x, sm, e & 255, cf < 0);
+#pragma unroll
+                for (int j = 0; j < 12; j++) acc[j] += (uint64_t)x.w[j] * mag;
+            }
+            pv_reduce(r, acc);
+        }
+        __syncwarp();
+        pv_store(sm, w.x & 255, r);
+        __syncwarp();
+    }
+}
+#define PV_RUN(name) pv_run(sm, PV_##name##_AT, PV_##name##_ROUNDS, lane)
+
+// an Fp12 value to other slots, conjugated over Fp6 if conj
+FK_D void pv_copy12(uint32_t *sm, int dst, int src, bool conj, int lane) {
+    Fp f;
+    if (lane < 12) {
+        pv_load(f, sm, src + lane);
+        if (conj && ((lane >> 1) & 1)) f_neg(f, f);
+    }
+    __syncwarp();
+    if (lane < 12) pv_store(sm, dst + lane, f);
+    __syncwarp();
+}
+// dst = src^p (conj) or src^(p^2)
+FK_D void pv_frob(uint32_t *sm, int dst, int src, bool conj, int lane) {
+    Fp2 x, g;
+    if (lane < 6) {
+        pv_load(x.c0, sm, src + 2 * lane);
+        pv_load(x.c1, sm, src + 2 * lane + 1);
+        if (conj) f_neg(x.c1, x.c1);
+        frob_coef(g, conj ? c_frob1[lane] : c_frob2[lane]);
+        x = f2m(x, g);
+    }
+    __syncwarp();
+    if (lane < 6) {
+        pv_store(sm, dst + 2 * lane, x.c0);
+        pv_store(sm, dst + 2 * lane + 1, x.c1);
+    }
+    __syncwarp();
+}
+// ACC = ACC^z in the cyclotomic subgroup (z = -|z|); B is overwritten
+static __device__ __noinline__ void pv_exp_z(uint32_t *sm, int lane) {
+    pv_copy12(sm, PV_B, PV_ACC, false, lane);
+#pragma unroll 1
+    for (int i = 62; i >= 0; i--) {
+        PV_RUN(CYC);
+        if ((Z_ABS >> i) & 1ull) PV_RUN(MUL);
+    }
+    pv_copy12(sm, PV_ACC, PV_ACC, true, lane);
+}
+
 // ---------------------------------------------------------------- kernels
 // op 0: out[i] = e(a[i], b[i]) (12 fp_t: the 6 Fp2 coefficients of w);
 // op 1: ok[i] = e(a[i], b[i]) == e(c[i], d[i]).
 // bcast bit 0: b is one point for every i; bit 1: d likewise.
-__global__ void __launch_bounds__(64) k_pairing(int op, uint64_t *out, uint8_t *ok, const uint64_t *a,
+__global__ void __launch_bounds__(32 * PV_WARPS) k_pairing(int op, uint64_t *out, uint8_t *ok, const uint64_t *a,
+                                                          const uint64_t *b, const uint64_t *c, const uint64_t *d,
+                                                          size_t count, int bcast) {
+    __shared__ __align__(16) uint32_t file[PV_WARPS][PV_SLOTS * 12];
+    const int lane = threadIdx.x & 31;
+    uint32_t *sm = file[threadIdx.x >> 5];
+    const size_t i = blockIdx.x * (size_t)PV_WARPS + (threadIdx.x >> 5);
+    if (i >= count) return;
+    Fp one, zero;
+    f_set_one(one);
+    f_set_zero(zero);
+    if (lane == 0) {
+        pv_store(sm, PV_ZERO, zero);
+        pv_store(sm, PV_ONE, one);
+    }
+    if (lane < 12) pv_store(sm, PV_ACC + lane, lane ? zero : one);
+    // lanes 0, 1: the G1 points; 2, 3: the G2 points
+    const int j = lane & 1;
+    bool finite = false;
+    if (lane < 2 && (j == 0 || op == 1)) {
+        Fp x, y;
+        finite = g1_affine(x, y, (j ? c : a) + 18 * i);
+        if (finite) {
+            if (j) f_neg(y, y);  // e(c, d)^-1 = e(-c, d)
+            pv_store(sm, PV_PT + 2 * j, x);
+            pv_store(sm, PV_PT + 2 * j + 1, y);
+        }
+    }
+    Fp2 xq, yq;
+    if ((lane == 2 || lane == 3) && (j == 0 || op == 1)) {
+        const bool same = bcast & (j ? 2 : 1);
+        finite = g2_affine(xq, yq, (j ? d : b) + (same ? 0 : 36 * i));
+    }
+    // A pair with a point at infinity (or op 0's second) contributes 1: P = (0, 0)
+    // leaves of each line its Fp2 term, which the final exponentiation removes;
+    // any finite Q whose multiples keep that term nonzero will do: the generator.
+    const unsigned fin = __ballot_sync(0xffffffffu, finite);
+    const bool pair = ((fin >> j) & (fin >> (2 + j))) & 1u;
+    if (lane < 2 && !pair) {
+        pv_store(sm, PV_PT + 2 * j, zero);
+        pv_store(sm, PV_PT + 2 * j + 1, zero);
+    }
+    if (lane == 2 || lane == 3) {
+        if (!pair) {
+#pragma unroll
+            for (int k = 0; k < 12; k++) {
+                xq.c0.w[k] = c_g2_gen[0][k];
+                xq.c1.w[k] = c_g2_gen[1][k];
+                yq.c0.w[k] = c_g2_gen[2][k];
+                yq.c1.w[k] = c_g2_gen[3][k];
+            }
+        }
+        for (int t = 0; t < 2; t++) {  // Q, and T = Q
+            const int at = t ? PV_T + 6 * j : PV_Q + 4 * j;
+            pv_store(sm, at, xq.c0);
+            pv_store(sm, at + 1, xq.c1);
+            pv_store(sm, at + 2, yq.c0);
+            pv_store(sm, at + 3, yq.c1);
+        }
+        pv_store(sm, PV_T + 6 * j + 4, one);
+        pv_store(sm, PV_T + 6 * j + 5, zero);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int k = 62; k >= 0; k--) {
+        PV_RUN(DBL);
+        if ((Z_ABS >> k) & 1ull) PV_RUN(ADD);
+    }
+    // easy part: m = f^((p^6 - 1)(p^2 + 1))
+    PV_RUN(INV1);
+    if (lane == 0) {
+        Fp n;
+        pv_load(n, sm, PV_X + 8);
+        f_inv(n, n);
+        pv_store(sm, PV_X + 8, n);
+    }
+    __syncwarp();
+    PV_RUN(INV2);
+    pv_copy12(sm, PV_ACC, PV_ACC, true, lane);
+    PV_RUN(MUL);
+    pv_frob(sm, PV_B, PV_ACC, false, lane);
+    PV_RUN(MUL);
+    pv_copy12(sm, PV_M, PV_ACC, false, lane);
+    // hard part: (z - 1)^2 (z + p) (z^2 + p^2 - 1) + 3
+    pv_exp_z(sm, lane);
+    pv_copy12(sm, PV_B, PV_M, true, lane);
+    PV_RUN(MUL);  // m^(z - 1)
+    pv_copy12(sm, PV_S1, PV_ACC, false, lane);
+    pv_exp_z(sm, lane);
+    pv_copy12(sm, PV_B, PV_S1, true, lane);
+    PV_RUN(MUL);  // m^((z - 1)^2)
+    pv_copy12(sm, PV_S1, PV_ACC, false, lane);
+    pv_exp_z(sm, lane);
+    pv_frob(sm, PV_B, PV_S1, true, lane);
+    PV_RUN(MUL);
+    pv_copy12(sm, PV_S2, PV_ACC, false, lane);  // b = .. ^(z + p)
+    pv_exp_z(sm, lane);
+    pv_exp_z(sm, lane);
+    pv_frob(sm, PV_B, PV_S2, false, lane);
+    PV_RUN(MUL);
+    pv_copy12(sm, PV_B, PV_S2, true, lane);
+    PV_RUN(MUL);  // b^(z^2 + p^2 - 1)
+    pv_copy12(sm, PV_S1, PV_ACC, false, lane);
+    pv_copy12(sm, PV_ACC, PV_M, false, lane);
+    pv_copy12(sm, PV_B, PV_M, false, lane);
+    PV_RUN(CYC);
+    PV_RUN(MUL);
+    pv_copy12(sm, PV_B, PV_S1, false, lane);
+    PV_RUN(MUL);  // times m^3
+    Fp e;
+    if (lane < 12) pv_load(e, sm, PV_ACC + lane);
+    if (op == 1) {
+        const bool is = lane >= 12 || f_eq(e, lane ? zero : one);
+        const bool all = __all_sync(0xffffffffu, is);
+        if (lane == 0) ok[i] = all ? 1 : 0;
+    } else if (lane < 12) {
+        fp_to_words(out + 72 * i + 6 * lane, e);
+    }
+}
+
+// The same, one thread per check: under half of the warp kernel's instructions a
+// check, nine times as deep.
+__global__ void __launch_bounds__(64) k_pairing_threads(int op, uint64_t *out, uint8_t *ok, const uint64_t *a,
                                                 const uint64_t *b, const uint64_t *c, const uint64_t *d,
                                                 size_t count, int bcast) {
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -308,49 +569,117 @@ __global__ void __launch_bounds__(64) k_pairing(int op, uint64_t *out, uint8_t *
 // interpolation polynomial I(X) = sum_j c_j X^j, c_j = (1/l) sum_k ys[k] w^-jk
 // / x^j, written as poly[32 i + j] (zero above l), and xl[i] = x^l.  Fr in
 // Montgomery form inside; fr_t standard form (any representative) in,
-// canonical out.
+// canonical out.  One warp per check, lane j its coefficient j.
 __global__ void __launch_bounds__(64) k_interp(uint64_t *poly, uint64_t *xl, const uint64_t *x, const uint64_t *ys,
                                                int log_l, size_t count) {
-    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    const size_t i = blockIdx.x * (size_t)2 + (threadIdx.x >> 5);
     if (i >= count) return;
-    const int l = 1 << log_l, step = 32 >> log_l;
-    Fr y[32], xm, xinv, t, acc, w, s;
-#pragma unroll 1
-    for (int k = 0; k < l; k++) {
-        fr_from_ref(t, ys + 4 * ((size_t)l * i + k));
-        f_to_mont(y[k], t);
+    const int lane = threadIdx.x & 31, l = 1 << log_l, step = 32 >> log_l;
+    Fr y, xm, p, t, acc, w;
+    f_set_zero(y);
+    if (lane < l) {
+        fr_from_ref(t, ys + 4 * ((size_t)l * i + lane));
+        f_to_mont(y, t);
     }
     fr_from_ref(t, x + 4 * i);
     f_to_mont(xm, t);
-    f_inv(xinv, xm);
-#pragma unroll
-    for (int q = 0; q < 8; q++) s.w[q] = c_inv_pow2[log_l][q];  // s = (1/l) x^-j, from j = 0
+    f_set_zero(acc);
 #pragma unroll 1
-    for (int j = 0; j < 32; j++) {
-        uint64_t *dst = poly + 4 * (32 * i + j);
-        if (j >= l) {
-            dst[0] = dst[1] = dst[2] = dst[3] = 0;
-            continue;
-        }
-        f_set_zero(acc);
-#pragma unroll 1
-        for (int k = 0; k < l; k++) {
-            const int e = (j * k * step) & 31;
+    for (int k = 0; k < l; k++) {
+        Fr v;
 #pragma unroll
-            for (int q = 0; q < 8; q++) w.w[q] = c_w32_inv[e][q];
-            f_mul(t, y[k], w);
-            f_add(acc, acc, t);
-        }
-        f_mul(acc, acc, s);
-        f_from_mont(t, acc);
-        fr_to_ref(dst, t);
-        f_mul(s, s, xinv);
+        for (int q = 0; q < 8; q++) v.w[q] = __shfl_sync(0xffffffffu, y.w[q], k);
+        const int e = (lane * k * step) & 31;
+#pragma unroll
+        for (int q = 0; q < 8; q++) w.w[q] = c_w32_inv[e][q];
+        f_mul(t, v, w);
+        f_add(acc, acc, t);
     }
-    t = xm;
+    // lane j: x^j, then (1/l) x^-j (the lanes' inverses run together)
+    f_set_one(p);
 #pragma unroll 1
-    for (int q = 0; q < log_l; q++) f_mul(t, t, t);
-    f_from_mont(acc, t);
-    fr_to_ref(xl + 4 * i, acc);
+    for (int q = 4; q >= 0; q--) {
+        f_mul(p, p, p);
+        if ((lane >> q) & 1) f_mul(p, p, xm);
+    }
+    f_inv(p, p);
+#pragma unroll
+    for (int q = 0; q < 8; q++) t.w[q] = c_inv_pow2[log_l][q];
+    f_mul(p, p, t);
+    f_mul(acc, acc, p);
+    f_from_mont(t, acc);
+    if (lane >= l) f_set_zero(t);
+    fr_to_ref(poly + 4 * (32 * i + lane), t);
+    if (lane == 0) {
+        t = xm;
+#pragma unroll 1
+        for (int q = 0; q < log_l; q++) f_mul(t, t, t);
+        f_from_mont(acc, t);
+        fr_to_ref(xl + 4 * i, acc);
+    }
+}
+
+// out[i] = C[i] - I[i] + [k_i] P_i for check_proof_multi: k = k1 + k2 lambda
+// (glv.cuh), [k1] P and [k2] phi(P) on neighbouring lanes with signed 4-bit
+// windows and complete formulas (32 x 4 doublings and 33 additions deep).  For
+// a P with a part outside the order-r subgroup the two halves differ from
+// [k] P by a point of the cofactor's order, which the pairing does not see.
+// The element-wise product's 256 doublings and ~128 additions are 2.5 times as
+// deep.  With the warp kernels of this file, 300 checks 40.6 -> 5.2 ms.
+__global__ void __launch_bounds__(64) k_verify_points(uint64_t *out, const uint64_t *C, const uint64_t *I,
+                                                      const uint64_t *P, const uint64_t *k, size_t count) {
+    const size_t i = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 1;
+    const int half = threadIdx.x & 1;
+    const bool on = i < count;
+    G1P acc, p, q;
+    g1_set_inf(acc);
+    g1_set_inf(p);
+    int8_t dig[33];
+    if (on) {
+        Fr s;
+        uint32_t s1[4], s2[4];
+        fr_from_ref(s, k + 4 * i);
+        glv_split(s1, s2, s.w);
+        int carry = 0;
+#pragma unroll
+        for (int w = 0; w < 32; w++) {
+            int v = (int)(((half ? s2[w >> 3] : s1[w >> 3]) >> (4 * (w & 7))) & 15u) + carry;
+            carry = v > 8;
+            dig[w] = (int8_t)(v - 16 * carry);
+        }
+        dig[32] = (int8_t)carry;
+        g1p_from_ref(p, P + 18 * i);
+        if (half) g1_phi(p, p);
+        G1P tab[8];
+        tab[0] = p;
+        for (int e = 1; e < 8; e++) g1_add(tab[e], tab[e - 1], p);
+#pragma unroll 1
+        for (int w = 32; w >= 0; w--) {
+            if (w < 32)
+                for (int b = 0; b < 4; b++) g1_dbl(acc, acc);
+            const int v = dig[w];
+            if (v) {
+                q = tab[(v < 0 ? -v : v) - 1];
+                if (v < 0) f_neg(q.y, q.y);
+                g1_add(acc, acc, q);
+            }
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int w = 0; w < 12; w++) {
+        q.x.w[w] = __shfl_xor_sync(0xffffffffu, acc.x.w[w], 1);
+        q.y.w[w] = __shfl_xor_sync(0xffffffffu, acc.y.w[w], 1);
+        q.z.w[w] = __shfl_xor_sync(0xffffffffu, acc.z.w[w], 1);
+    }
+    if (!on || half) return;
+    g1_add(acc, acc, q);
+    g1p_from_ref(q, C + 18 * i);
+    g1_add(acc, acc, q);
+    g1p_from_ref(q, I + 18 * i);
+    g1_neg(q, q);
+    g1_add(acc, acc, q);
+    g1p_to_ref(out + 18 * i, acc);
 }
 
 // G2 element-wise: 0 add, 1 dbl, 2 neg, 3 sub, 4 mul by fr_t scalar, 5 normalize,
@@ -406,13 +735,24 @@ __global__ void __launch_bounds__(64) k_g2_op(int op, uint64_t *out, const uint6
     g2_store(out + 36 * i, xr, yr, ir);
 }
 
+// Checks one warp each up to here, one thread each beyond.  B200: the warp kernel
+// 2.8 ms to 300 checks, then 409 k checks/s (23.8 ms at 9,472); the thread kernel
+// 26 ms to 10^4 checks, 37.6 ms at 37,888 (1.0 M/s).
+constexpr size_t PAIRING_WARP_MAX = 10240;
 void launch_pairing(int op, uint64_t *out, uint8_t *ok, const uint64_t *a, const uint64_t *b, const uint64_t *c,
                     const uint64_t *d, size_t count, cudaStream_t st, int bcast) {
-    k_pairing<<<blocks_for(count, 64), 64, 0, st>>>(op, out, ok, a, b, c, d, count, bcast);
+    if (count <= PAIRING_WARP_MAX)
+        k_pairing<<<blocks_for(count, PV_WARPS), 32 * PV_WARPS, 0, st>>>(op, out, ok, a, b, c, d, count, bcast);
+    else
+        k_pairing_threads<<<blocks_for(count, 64), 64, 0, st>>>(op, out, ok, a, b, c, d, count, bcast);
 }
 void launch_interp(uint64_t *poly, uint64_t *xl, const uint64_t *x, const uint64_t *ys, int log_l, size_t count,
                    cudaStream_t st) {
-    k_interp<<<blocks_for(count, 64), 64, 0, st>>>(poly, xl, x, ys, log_l, count);
+    k_interp<<<blocks_for(count, 2), 64, 0, st>>>(poly, xl, x, ys, log_l, count);
+}
+void launch_verify_points(uint64_t *out, const uint64_t *C, const uint64_t *I, const uint64_t *P, const uint64_t *k,
+                          size_t count, cudaStream_t st) {
+    k_verify_points<<<blocks_for(2 * count, 64), 64, 0, st>>>(out, C, I, P, k, count);
 }
 void launch_g2_op(int op, uint64_t *out, const uint64_t *a, const void *b, size_t count, cudaStream_t st) {
     k_g2_op<<<blocks_for(count, 64), 64, 0, st>>>(op, out, a, b, count);

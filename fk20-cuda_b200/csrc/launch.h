@@ -149,6 +149,8 @@ void launch_pairing(int op, uint64_t *out, uint8_t *ok, const uint64_t *a, const
                     const uint64_t *d, size_t count, cudaStream_t st, int bcast = 0);
 void launch_interp(uint64_t *poly, uint64_t *xl, const uint64_t *x, const uint64_t *ys, int log_l, size_t count,
                    cudaStream_t st);
+void launch_verify_points(uint64_t *out, const uint64_t *C, const uint64_t *I, const uint64_t *P, const uint64_t *k,
+                          size_t count, cudaStream_t st);
 void launch_g2_op(int op, uint64_t *out, const uint64_t *a, const void *b, size_t count, cudaStream_t st);
 
 // kernels_tables.cu

@@ -1,0 +1,43 @@
+"""Pairing checks on both sides of the line between the two kernels (a warp per
+check up to 10,240, a thread per check beyond): true and false equations and
+points at infinity on either side, by known scalars."""
+import numpy as np
+import pytest
+
+import oracle as O
+import pairing_py as PP
+
+pytestmark = pytest.mark.gpu
+
+
+def g2_rows(pts):
+    out = np.zeros((len(pts), 36), np.uint64)
+    for i, q in enumerate(pts):
+        if q is None:
+            out[i, 12] = 1
+            continue
+        for k, v in enumerate((q[0][0], q[0][1], q[1][0], q[1][1], 1, 0)):
+            out[i, 6 * k:6 * k + 6] = O.int_to_limbs(v, 6)
+    return out
+
+
+@pytest.mark.parametrize("count", [1, 2, 3, 37, 10240, 10241])
+def test_checks_by_known_scalars(engine, count):
+    import torch
+    ks = [O.limbs_to_int(v) for v in O.seeded_fr(77, 8)]
+    # (a, b, c, d): e([a]G1, [b]G2) == e([c]G1, [d]G2) exactly when ab = cd
+    rows = [(ks[0], ks[1], ks[0] * ks[1] % O.R, 1), (ks[2], ks[3], (ks[2] * ks[3] + 1) % O.R, 1), (0, ks[1], 0, ks[2]),
+            (0, ks[1], 5, ks[2]), (ks[4], 0, ks[5], 0), (ks[4], 0, 0, ks[6]), (ks[4], ks[5], ks[5], ks[4]),
+            (ks[4], ks[5], ks[4], ks[6])]
+    want = [int(a * b % O.R == c * d % O.R) for a, b, c, d in rows]
+    assert want == [1, 0, 1, 0, 1, 1, 1, 0]
+    g1 = O.g1_generator().reshape(1, 18)
+    g2 = PP.g2_generator()
+    mul1 = lambda v: O.g1_op("mul", np.repeat(g1, len(v), 0), O.ints_to_array(v, 4))
+    A, C = mul1([r[0] for r in rows]), mul1([r[2] for r in rows])
+    Bq, D = (g2_rows([PP.g2mul(r[k], g2) if r[k] else None for r in rows]) for k in (1, 3))
+    idx = np.arange(count) % len(rows)
+    dev = [engine.to_device(np.ascontiguousarray(v[idx])) for v in (A, Bq, C, D)]
+    ok = torch.full((count,), 7, dtype=torch.uint8, device="cuda")
+    engine.call("fk20_pairing_check_n", engine._ptr(ok), *[engine._ptr(v) for v in dev], count, engine._stream())
+    assert ok.cpu().numpy().tolist() == [want[i] for i in idx]
