@@ -755,6 +755,19 @@ int reserve_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, bool
     return 0;
 }
 
+// Blocks per SM for `products` product tasks.  Two warps a scheduler share the
+// multiply pipe without slowing each other down; three take 1.44 times as
+// long a task, together 4 % less.  So the third is worth it for many tasks, or
+// where it saves much of a wave (a last wave at three takes its share of the
+// 1.44, at least 1): 865 products (one blob of 4096) 2.9 ms at four blocks
+// against 4.2 at six, 1,398 (32 inverse transforms) 4.9 against 4.4, 2,796 7.2
+// against 6.4, 3,363 (40 rows) 7.3 against 7.5, 11,210 21.0 against 20.6.
+int proj_grid(double products, int sms, int most) {
+    const double four = std::ceil(products / (8.0 * sms)), n = products / (12.0 * sms);
+    const double six = n <= 1 ? 1.44 : 1.44 * std::floor(n) + std::max(1.0, 1.44 * (n - std::floor(n)));
+    return std::min(most, n > 4 || six < 0.9 * four ? 6 : 4);
+}
+
 // The plan `kind` on the arenas D + d_off[k] (inputs stored) on st: one
 // persistent launch, or (staged) one launch per run of independent tasks.
 // `first` clears the error word too; a later pass of the same call keeps it.
@@ -782,9 +795,10 @@ int run_plan(fk20_ctx *ctx, Workspace &ws, const SegLayout &lay, const int *log_
     p.spin_limit = ctx->wait_limit;
     p.unpublished = ctx->unpublished;
     // persistent grid: the context's setting, or the caller's share of the SMs (server packs)
-    int per_sm = ctx->proj_occupancy;
     const int want = bps > 0 ? bps : ctx->fft_blocks_per_sm;
-    if (want > 0 && want < per_sm) per_sm = want;
+    double products = 0;
+    for (int k = 0; k < nseg; k++) products += (double)plans[k]->muls * G[k];
+    const int per_sm = want > 0 ? std::min(want, ctx->proj_occupancy) : proj_grid(products, ctx->sms, ctx->proj_occupancy);
     const auto blocks = [&](unsigned tasks) {
         return (int)std::min<unsigned>((unsigned)(ctx->sms * per_sm), (tasks + FFT_WARPS - 1) / FFT_WARPS);
     };
@@ -2047,7 +2061,7 @@ int enqueue_pack(fk20_server *s, Slot &sl, bool latency) {
         // time); a throughput-mode pack takes 1/slots of the SMs, so packs of
         // different slots run side by side and hide each other's dependency
         // waits.
-        int share = ctx->proj_occupancy;
+        int share = 0;  // by the number of products
         if (s->cfg.fft_blocks_per_sm)
             share = std::min((int)s->cfg.fft_blocks_per_sm, ctx->proj_occupancy);
         else if (!latency)

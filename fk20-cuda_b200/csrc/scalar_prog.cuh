@@ -30,7 +30,8 @@ namespace fk {
 constexpr int PROG_POSITIONS = 136;
 constexpr int PROG_WORDS = 1 + PROG_POSITIONS / 4;
 constexpr int PROG_SLOTS = 4;                         // P, 3P, 5P, 7P
-constexpr int PROG_SLOT_WORDS = 36 * PROG_SLOTS + 12;  // (x', y', beta x') of each point, then u
+constexpr int PROG_POINT_WORDS = 36 * PROG_SLOTS;          // (x', y', beta x') of each point
+constexpr int PROG_SLOT_WORDS = PROG_POINT_WORDS + 12;     // then u
 
 // The executor's scratch: for each thread PROG_SLOT_WORDS 32-bit words at
 // base[0], base[stride], ...  While P, 3P, 5P, 7P are formed, point i is
@@ -86,8 +87,8 @@ struct SlotQ {
 // 3. Back to E: Jacobian (X, Y, Z u), i.e. homogeneous (X Z', Y, Z'^3) with
 //    Z' = Z u.  P = infinity (u = 0) makes every value above meaningless;
 //    the lane's flag then selects infinity.
-template <class ProgPtr>
-FK_HD void g1_mul_prog(G1P &acc, const ProgSlots &slot, ProgPtr prog) {
+template <class ProgPtr, class U>
+FK_HD void g1_mul_prog(G1P &acc, const ProgSlots &slot, ProgPtr prog, const U &keep) {
     const uint32_t hdr = prog[0];
     if (hdr & 0x100u) { g1_set_inf(acc); return; }
     const bool negate = (hdr & 0x400u) != 0;
@@ -122,7 +123,7 @@ FK_HD void g1_mul_prog(G1P &acc, const ProgSlots &slot, ProgPtr prog) {
             slot_put(slot.word(36 * i + 12), st, b.y);
             slot_put(slot.word(36 * i + 24), st, t);
         }
-        slot_put(slot.word(144), st, b.z);  // u: the Z of 7P
+        keep.put(b.z);  // u: the Z of 7P
     }
     {
         // onto the Z of 7P: 5P by e3, 3P by e2 e3, P by e1 e2 e3
@@ -181,7 +182,7 @@ FK_HD void g1_mul_prog(G1P &acc, const ProgSlots &slot, ProgPtr prog) {
     if (negate) f_neg(j.y, j.y);
     {
         Fp u, t;
-        slot_get(u, slot.word(144), st);
+        keep.get(u);
         fp_mul(j.z, j.z, u);  // Z' = Z u
         fp_mul(acc.x, j.x, j.z);
         fp_sqr(t, j.z);
@@ -189,6 +190,18 @@ FK_HD void g1_mul_prog(G1P &acc, const ProgSlots &slot, ProgPtr prog) {
         acc.y = j.y;
     }
     if (inf) g1_set_inf(acc);
+}
+
+// u behind the four points
+struct SlotU {
+    uint32_t *p;
+    int stride;
+    FK_HD void put(const Fp &f) const { slot_put(p, stride, f); }
+    FK_HD void get(Fp &f) const { slot_get(f, p, stride); }
+};
+template <class ProgPtr>
+FK_HD void g1_mul_prog(G1P &acc, const ProgSlots &slot, ProgPtr prog) {
+    g1_mul_prog(acc, slot, prog, SlotU{slot.word(PROG_POINT_WORDS), slot.stride});
 }
 
 // register-only convenience form (setup-time and element-wise kernels): a
