@@ -254,10 +254,12 @@ __global__ void __launch_bounds__(MSM_MAX_THREADS, FK_MSM_MINB) k_msm(const __gr
     if (args.times_m) {
         for (int t = 0; t < a.log_m; t++) g1_dbl(acc, acc);
     }
-    // every lane stores: lanes beyond the rows get copies of the rows' points
+    // lanes beyond the rows of the segment get copies of its rows' points
+    if (!a.fill && (lane >> a.rl) != 0) return;
     const int to = a.row0 + g * 32 + lane;
+    if ((a.row0 & 31) + lane > 31) return;
     if (a.arena.slots == 0) {
-        tile_store(a.D + tile_index(to >> 5, m, c), lane, acc);
+        tile_store(a.D + tile_index(to >> 5, m, c), to & 31, acc);
     } else {
         int ga, la;
         if (!proj_lane(a.arena, to, proj_in_inst(c), ga, la)) return;
@@ -350,14 +352,14 @@ void launch_commit(uint64_t *out, uint4 *part, const uint64_t *poly, const uint4
     k_commit_reduce<<<(unsigned)rows, REDUCE_THREADS, 0, st>>>(out, part, P);
 }
 
-// How a launch is cut.  A segment's last rows % 32 rows form a segment of their
-// own whose lanes are packed (msm_row_lanes); and while whole units leave the
+// How a launch is cut.  A segment's last rows % 32 rows form one or two segments
+// of their own whose lanes are packed (msm_row_lanes); and while whole units leave the
 // chip's last wave of warps a large share of the time, four warps (two in
 // 64-thread blocks) share a unit.  Resident: three 128-thread blocks per SM.
 // A batch of one or two rows has 16 or 32 lane groups already, and more warps
 // would only add sums.  B200, window 10, MSM alone, before (a row per lane, a
 // warp per unit) and after: 1 row of 4096 4.41 -> 0.21 ms, 19 of 2048 4.64 ->
-// 1.63, 160 of 4096 15.1 -> 13.5; at 512 rows of 4096 (4.6 waves) splitting
+// 1.33, 160 of 4096 15.1 -> 13.5; at 512 rows of 4096 (4.6 waves) splitting
 // costs 1 %, 40.7 -> 41.1, hence the line at 4 waves.  48 commitments of 4096:
 // 10.5 -> 3.0 ms, most of it the partial sums, which one thread per row added.
 void launch_msm(const MsmArgs &in, int threads, cudaStream_t st) {
@@ -367,14 +369,19 @@ void launch_msm(const MsmArgs &in, int threads, cudaStream_t st) {
     a.nseg = 0;
     unsigned units = 0;
     for (int k = 0; k < in.nseg; k++) {
-        const int full = in.seg[k].rows & ~31, rest = in.seg[k].rows & 31;
-        for (int part = 0; part < 2; part++) {
-            if (part ? !rest : !full) continue;
+        // whole groups; then 16 rows when the rest is 17 to 24 (at most half of
+        // the packed lanes of the last part idle); then the rest
+        const int rows = in.seg[k].rows, full = rows & ~31, rest = rows & 31;
+        const int cut[4] = {0, full, full + (rest > 16 && rest <= 24 ? 16 : 0), rows};
+        for (int part = 0; part < 3; part++) {
+            const int n = cut[part + 1] - cut[part];
+            if (n <= 0) continue;
             MsmSeg s = in.seg[k];
-            s.row0 = part ? full : 0;
-            s.rl = part ? msm_row_lanes(rest) : 5;
-            s.G = part ? 1 : full / 32;
-            if (!part) s.rows = full;
+            s.row0 = cut[part];
+            s.rows = cut[part + 1];
+            s.rl = part ? msm_row_lanes(n) : 5;
+            s.G = part ? 1 : n / 32;
+            s.fill = cut[part + 1] == rows;
             s.warp_start = units;
             units += (unsigned)s.G << s.log_m;
             a.seg[a.nseg++] = s;

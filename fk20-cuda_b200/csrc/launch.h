@@ -24,10 +24,10 @@ struct MsmSeg {
     unsigned warp_start;  // first warp (of the launch) that works on this segment
     ProjArena arena;      // slots > 0: D is an arena (proj_task.cuh), else point tiles [G][m]
     size_t s_stride;      // uint4 from one row group's scalars to the next
-    int row0, rl;         // set by launch_msm: the first row, log2 of the rows a warp takes
+    int row0, rl, fill;   // set by launch_msm: the first row, log2 of the rows a warp takes, last part of its rows
 };
 struct MsmArgs {
-    MsmSeg seg[2 * MAX_SEGS];  // a caller fills at most MAX_SEGS
+    MsmSeg seg[3 * MAX_SEGS];  // a caller fills at most MAX_SEGS
     int nseg, times_m;
     int split;  // set by launch_msm: warps per (column, row group)
     int test_check;  // checked build: record FK20_CHECK_MSM_PLANTED (tests of the checks)
