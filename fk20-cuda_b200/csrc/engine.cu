@@ -1592,10 +1592,9 @@ int fk20_ctx_commit(fk20_ctx *ctx, g1p_t *commitment, const fr_t *polynomial, un
     std::lock_guard<std::mutex> lk(ctx->mu);
     DeviceGuard dg(ctx->device);
     if (!ctx->commit.n || (int)n > ctx->commit.n) return FK20_ENOSETUP;
-    const int G = (int)((rows + 31) / 32);
-    const int parts = commit_parts((int)rows, (int)n);
-    CKR(ctx->commit.part.reserve(tile_bytes(G, parts)));
-    const double terms = (double)rows * n * ctx->commit.W, sums = (double)rows * parts * ADD_P;
+    const CommitCut cut = commit_cut((int)rows, (int)n, ctx->commit.W);
+    CKR(ctx->commit.part.reserve(tile_bytes(1, cut.tiles())));
+    const double terms = (double)rows * n * ctx->commit.W, sums = (double)rows * (cut.full ? cut.P : cut.Pr) * ADD_P;
     ctx->prof.begin(FK20_K_MSM, terms * MADD_A + sums, terms * MADD_X + sums, S_(stream));
     launch_commit((uint64_t *)commitment, (uint4 *)ctx->commit.part.p, (const uint64_t *)polynomial,
                   (const uint4 *)ctx->commit.table.p, (int)rows, (int)n, ctx->commit.W, ctx->commit.cb, S_(stream));
@@ -1780,11 +1779,10 @@ int fk20_ctx_check_proof_multi(fk20_ctx *ctx, uint8_t *ok, const g1p_t *commitme
     if (ctx->commit.n < (int)COMMIT_CHUNK) return FK20_ENOSETUP;
     int log_l = 0;
     while ((1u << log_l) < l) log_l++;
-    const int G = (int)((count + 31) / 32);
     const size_t poly_b = (size_t)count * COMMIT_CHUNK * sizeof(fr_t), xl_b = (size_t)count * sizeof(fr_t),
                  pt_b = (size_t)count * sizeof(g1p_t);
     CKR(ctx->verify.reserve(poly_b + xl_b + 2 * pt_b));
-    CKR(ctx->commit.part.reserve(tile_bytes(G, commit_parts((int)count, (int)COMMIT_CHUNK))));
+    CKR(ctx->commit.part.reserve(tile_bytes(1, commit_cut((int)count, (int)COMMIT_CHUNK, ctx->commit.W).tiles())));
     char *base = (char *)ctx->verify.p;
     uint64_t *poly = (uint64_t *)base, *xl = (uint64_t *)(base + poly_b);
     uint64_t *I = (uint64_t *)(base + poly_b + xl_b), *A = I + 18 * (size_t)count;

@@ -119,10 +119,15 @@ void launch_msm(const MsmArgs &a, int threads, cudaStream_t st);  // threads: 64
 int check_take_msm();
 int check_take_fft();
 int check_take_proj();
-// KZG commitments: polynomial lengths are multiples of COMMIT_CHUNK; pass 1
-// has commit_parts(rows, n) warps per 32 rows, and part holds as many tiles
+// KZG commitments: polynomial lengths are multiples of COMMIT_CHUNK.  Pass 1 has
+// P warps for each of `full` groups of 32 rows and Pr for the rest (2^rl of its
+// lanes are rows), one partial-sum tile each.
 constexpr int COMMIT_CHUNK = 32;
-int commit_parts(int rows, int n);
+struct CommitCut {
+    int full, P, Pr, rl;
+    FK_HD int tiles() const { return full * P + Pr; }
+};
+CommitCut commit_cut(int rows, int n, int W);
 void launch_commit(uint64_t *out, uint4 *part, const uint64_t *poly, const uint4 *table, int rows, int n, int W,
                    int cb, cudaStream_t st);
 
