@@ -20,6 +20,7 @@ ACC, B, M, S1, S2 = 4, 16, 28, 40, 52
 T, PT, Q = 64, 76, 80  # two points: X, Y, Z (6 each); xP, yP (2 each); xQ, yQ (4 each)
 X = 88                 # the inverse's intermediates: t0, t1, t2, n, 1/norm
 TMP = 97
+VA, VQ, VT = 4, 10, 16  # the G1 machine: two sums, two addends, 2 x 8 multiples (inside the pairing's slots)
 Z_ABS = 0xD201000000010000
 
 
@@ -270,6 +271,45 @@ def prog_inv2():
     return tr, out
 
 
+def g1at(tr, s): return tr.slot(s), tr.slot(s + 1), tr.slot(s + 2)
+
+
+def prog_vdbl():
+    """A_j = 2 A_j on G1 (complete, Renes-Costello-Batina algorithm 9), j = 0, 1"""
+    tr, out = Trace(), {}
+    m = tr.mul
+
+    def hold(v): return LC(tr, {tr.lin(v): 1})
+    for j in range(2):
+        x, y, z = g1at(tr, VA + 3 * j)
+        yy, yz, zz, xy = m(y, y), m(y, z), m(z, z), m(x, y)
+        t2, z3, u, t0 = hold(12 * zz), hold(8 * yy), hold(yy + 12 * zz), hold(yy - 36 * zz)
+        out[VA + 3 * j] = 2 * m(t0, xy)
+        out[VA + 3 * j + 1] = m(t0, u) + m(t2, z3)
+        out[VA + 3 * j + 2] = m(yz, z3)
+    return tr, out
+
+
+def prog_vadd():
+    """A_j = A_j + Q_j on G1 (complete, algorithm 7), j = 0, 1"""
+    tr, out = Trace(), {}
+    m = tr.mul
+
+    def hold(v): return LC(tr, {tr.lin(v): 1})
+    for j in range(2):
+        x1, y1, z1 = g1at(tr, VA + 3 * j)
+        x2, y2, z2 = g1at(tr, VQ + 3 * j)
+        t0, t1, t2 = m(x1, x2), m(y1, y2), m(z1, z2)
+        t3 = hold(m(x1 + y1, x2 + y2) - t0 - t1)
+        t4 = hold(m(y1 + z1, y2 + z2) - t1 - t2)
+        s = hold(12 * (m(x1 + z1, x2 + z2) - t0 - t2))
+        w, u, v = hold(3 * t0), hold(t1 - 12 * t2), hold(t1 + 12 * t2)
+        out[VA + 3 * j] = m(t3, u) - m(t4, s)
+        out[VA + 3 * j + 1] = m(s, w) + m(u, v)
+        out[VA + 3 * j + 2] = m(v, t4) + m(w, t3)
+    return tr, out
+
+
 def schedule(tr, out):
     """rounds [(kind, [(dst slot, node)])] and the slots used"""
     nodes = tr.nodes
@@ -387,7 +427,7 @@ def place_at(place, k):
 
 
 PROGRAMS = (("DBL", prog_dbl), ("ADD", prog_add), ("MUL", prog_mul), ("CYC", prog_cyc), ("INV1", prog_inv1),
-            ("INV2", prog_inv2))
+            ("INV2", prog_inv2), ("VDBL", prog_vdbl), ("VADD", prog_vadd))
 
 
 def build():
@@ -428,7 +468,7 @@ def main():
     print("// pairing_prog.inc -- written by gen_pairing_prog.py (run it to regenerate; do not edit).")
     print("// clang-format off")
     print("constexpr int PV_SLOTS = %d;" % slots)
-    names = ("ZERO", ZERO), ("ONE", ONE), ("DUMP", DUMP), ("ACC", ACC), ("B", B), ("M", M), ("S1", S1), ("S2", S2), ("T", T), ("PT", PT), ("Q", Q), ("X", X)
+    names = ("ZERO", ZERO), ("ONE", ONE), ("DUMP", DUMP), ("ACC", ACC), ("B", B), ("M", M), ("S1", S1), ("S2", S2), ("T", T), ("PT", PT), ("Q", Q), ("X", X), ("VA", VA), ("VQ", VQ), ("VT", VT)
     for n, v in names:
         print("constexpr int PV_%s = %d;" % (n, v))
     at, heads, data = 0, [], []

@@ -619,6 +619,116 @@ __global__ void __launch_bounds__(64) k_interp(uint64_t *poly, uint64_t *xl, con
     }
 }
 
+// signed 4-bit windows of the GLV half `half` (0: k mod lambda, 1: k div lambda)
+// of a canonical scalar, least significant first
+FK_D void glv_digits(int8_t dig[33], const Fr &s, int half) {
+    uint32_t s1[4], s2[4];
+    glv_split(s1, s2, s.w);
+    int carry = 0;
+#pragma unroll
+    for (int w = 0; w < 32; w++) {
+        const int v = (int)(((half ? s2[w >> 3] : s1[w >> 3]) >> (4 * (w & 7))) & 15u) + carry;
+        carry = v > 8;
+        dig[w] = (int8_t)(v - 16 * carry);
+    }
+    dig[32] = (int8_t)carry;
+}
+
+// k_verify_points' result with a warp per check: both halves' doublings and
+// additions are rounds of the 32-lane machine, 2 products and 2 or 3 sums deep
+// instead of 8 and 12 products.
+__global__ void __launch_bounds__(32 * PV_WARPS) k_verify_points_warp(uint64_t *out, const uint64_t *C, const uint64_t *I,
+                                                                     const uint64_t *P, const uint64_t *k,
+                                                                     size_t count) {
+    __shared__ __align__(16) uint32_t file[PV_WARPS][PV_SLOTS * 12];
+    __shared__ int8_t digits[PV_WARPS][2][33];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    uint32_t *sm = file[wp];
+    const size_t i = blockIdx.x * (size_t)PV_WARPS + wp;
+    if (i >= count) return;
+    const auto put = [&](int slot, const G1P &p) {
+        pv_store(sm, slot, p.x);
+        pv_store(sm, slot + 1, p.y);
+        pv_store(sm, slot + 2, p.z);
+    };
+    // A_j = from[j] (j = 0, 1), three lanes each
+    const auto copy = [&](int dst, int src0, int src1, bool neg0, bool neg1) {
+        Fp f;
+        const int j = lane / 3, c = lane % 3;
+        if (lane < 6) {
+            const int src = j ? src1 : src0;
+            if (src < 0) {  // infinity
+                f_set_zero(f);
+                if (c == 1) f_set_one(f);
+            } else {
+                pv_load(f, sm, src + c);
+                if (c == 1 && (j ? neg1 : neg0)) f_neg(f, f);
+            }
+        }
+        __syncwarp();
+        if (lane < 6) pv_store(sm, dst + lane, f);
+        __syncwarp();
+    };
+    if (lane == 0) {
+        Fp f;
+        f_set_zero(f);
+        pv_store(sm, PV_ZERO, f);
+    }
+    if (lane < 2) {  // P and phi(P): multiples 1 .. 8 of half j at PV_VT + 24 j
+        Fr s;
+        G1P p;
+        fr_from_ref(s, k + 4 * i);
+        glv_digits(digits[wp][lane], s, lane);
+        g1p_from_ref(p, P + 18 * i);
+        if (lane) g1_phi(p, p);
+        put(PV_VT + 24 * lane, p);
+    }
+    __syncwarp();
+    copy(PV_VA, PV_VT, PV_VT + 24, false, false);
+    copy(PV_VQ, PV_VT, PV_VT + 24, false, false);
+#pragma unroll 1
+    for (int e = 1; e < 8; e++) {
+        PV_RUN(VADD);
+        Fp f;
+        if (lane < 6) {
+            pv_load(f, sm, PV_VA + lane);
+            pv_store(sm, PV_VT + 24 * (lane / 3) + 3 * e + lane % 3, f);
+        }
+        __syncwarp();
+    }
+    copy(PV_VA, -1, -1, false, false);
+#pragma unroll 1
+    for (int w = 32; w >= 0; w--) {
+        if (w < 32)
+#pragma unroll 1
+            for (int b = 0; b < 4; b++) PV_RUN(VDBL);
+        const int v0 = digits[wp][0][w], v1 = digits[wp][1][w];
+        if (!v0 && !v1) continue;
+        copy(PV_VQ, v0 ? PV_VT + 3 * ((v0 < 0 ? -v0 : v0) - 1) : -1, v1 ? PV_VT + 24 + 3 * ((v1 < 0 ? -v1 : v1) - 1) : -1,
+             v0 < 0, v1 < 0);
+        PV_RUN(VADD);
+    }
+    // the two halves, then C and -I, each pair in one addition
+    if (lane < 2) {
+        G1P p;
+        g1p_from_ref(p, (lane ? I : C) + 18 * i);
+        if (lane) f_neg(p.y, p.y);
+        put(PV_VT + 3 * lane, p);
+    }
+    __syncwarp();
+    copy(PV_VQ, PV_VT, PV_VT + 3, false, false);
+    PV_RUN(VADD);  // A_0 + C, A_1 - I
+    copy(PV_VQ, PV_VA + 3, -1, false, false);
+    PV_RUN(VADD);
+    if (lane == 0) {
+        G1P p;
+        pv_load(p.x, sm, PV_VA);
+        pv_load(p.y, sm, PV_VA + 1);
+        pv_load(p.z, sm, PV_VA + 2);
+        g1p_to_ref(out + 18 * i, p);
+    }
+}
+
 // out[i] = C[i] - I[i] + [k_i] P_i for check_proof_multi: k = k1 + k2 lambda
 // (glv.cuh), [k1] P and [k2] phi(P) on neighbouring lanes with signed 4-bit
 // windows and complete formulas (32 x 4 doublings and 33 additions deep).  For
@@ -637,17 +747,8 @@ __global__ void __launch_bounds__(64) k_verify_points(uint64_t *out, const uint6
     int8_t dig[33];
     if (on) {
         Fr s;
-        uint32_t s1[4], s2[4];
         fr_from_ref(s, k + 4 * i);
-        glv_split(s1, s2, s.w);
-        int carry = 0;
-#pragma unroll
-        for (int w = 0; w < 32; w++) {
-            int v = (int)(((half ? s2[w >> 3] : s1[w >> 3]) >> (4 * (w & 7))) & 15u) + carry;
-            carry = v > 8;
-            dig[w] = (int8_t)(v - 16 * carry);
-        }
-        dig[32] = (int8_t)carry;
+        glv_digits(dig, s, half);
         g1p_from_ref(p, P + 18 * i);
         if (half) g1_phi(p, p);
         G1P tab[8];
@@ -750,9 +851,14 @@ void launch_interp(uint64_t *poly, uint64_t *xl, const uint64_t *x, const uint64
                    cudaStream_t st) {
     k_interp<<<blocks_for(count, 2), 64, 0, st>>>(poly, xl, x, ys, log_l, count);
 }
+// Points one warp each up to here, two lanes each beyond.
+constexpr size_t VERIFY_WARP_MAX = 2048;
 void launch_verify_points(uint64_t *out, const uint64_t *C, const uint64_t *I, const uint64_t *P, const uint64_t *k,
                           size_t count, cudaStream_t st) {
-    k_verify_points<<<blocks_for(2 * count, 64), 64, 0, st>>>(out, C, I, P, k, count);
+    if (count <= VERIFY_WARP_MAX)
+        k_verify_points_warp<<<blocks_for(count, PV_WARPS), 32 * PV_WARPS, 0, st>>>(out, C, I, P, k, count);
+    else
+        k_verify_points<<<blocks_for(2 * count, 64), 64, 0, st>>>(out, C, I, P, k, count);
 }
 void launch_g2_op(int op, uint64_t *out, const uint64_t *a, const void *b, size_t count, cudaStream_t st) {
     k_g2_op<<<blocks_for(count, 64), 64, 0, st>>>(op, out, a, b, count);

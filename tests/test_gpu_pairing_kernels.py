@@ -41,3 +41,45 @@ def test_checks_by_known_scalars(engine, count):
     ok = torch.full((count,), 7, dtype=torch.uint8, device="cuda")
     engine.call("fk20_pairing_check_n", engine._ptr(ok), *[engine._ptr(v) for v in dev], count, engine._stream())
     assert ok.cpu().numpy().tolist() == [want[i] for i in idx]
+
+
+@pytest.mark.parametrize("count", [5, 2048, 2049])
+def test_check_proof_multi_on_both_point_kernels(engine, count):
+    """check_proof_multi with its points a warp each and two lanes each, checks of
+    every verdict with a zero coset shift, an infinite proof and an infinite
+    commitment among them (scalars known: C = [c], proof = [q], I from ys)."""
+    import torch
+    l, R = 4, O.R
+    t = 1234567
+    rng = np.random.default_rng(12)
+    word = lambda: int.from_bytes(rng.bytes(32), "little") % R
+    w = O.root_of_unity(l)
+    rows = []
+    for kind in range(6):
+        x, r = (0 if kind == 3 else word()), [word() for _ in range(l)]
+        rt = sum(v * pow(t, k, R) for k, v in enumerate(r)) % R
+        d = (pow(t, l, R) - pow(x, l, R)) % R
+        c = 0 if kind == 4 else rt if kind == 2 else word()  # kind 2: quotient 0
+        q = (c - rt) * pow(d, -1, R) % R
+        if kind == 3:  # every value of a coset at 0 is r_0
+            r = [r[0]] + [0] * (l - 1)
+            rt, q = r[0], (c - r[0]) * pow(d, -1, R) % R
+        ys = [sum(v * pow(x * pow(w, k, R) % R, e, R) for e, v in enumerate(r)) % R for k in range(l)]
+        rows.append((c, q, x, ys, 1))
+        rows.append((c, q, x, [(ys[0] + 1) % R] + ys[1:], 0))
+    idx = np.arange(count) % len(rows)
+    g1 = O.g1_generator().reshape(1, 18)
+    mul1 = lambda v: O.g1_op("mul", np.repeat(g1, len(v), 0), O.ints_to_array(v, 4))
+    c = engine.Context(0, 8)
+    c.load_commit(32, engine.to_device(mul1([pow(t, k, R) for k in range(32)])), 8)
+    dev = lambda a: engine.to_device(np.ascontiguousarray(a[idx]))
+    C, Q = dev(mul1([r[0] for r in rows])), dev(mul1([r[1] for r in rows]))
+    X = dev(O.ints_to_array([r[2] for r in rows], 4))
+    Y = dev(np.stack([O.ints_to_array(r[3], 4) for r in rows]))
+    s2 = engine.to_device(g2_rows([PP.g2mul(pow(t, k, R), PP.g2_generator()) for k in range(l + 1)]))
+    ok = torch.full((count,), 7, dtype=torch.uint8, device="cuda")
+    c.check_proof_multi(ok, C, Q, X, Y, l, s2, count)
+    got = ok.cpu().numpy().tolist()
+    c.close()
+    # at x = 0 the interpolation keeps coefficient 0 only, as before: ys[0] alone moves the mean
+    assert got == [rows[i][4] for i in idx]

@@ -134,3 +134,38 @@ def test_generator_keeps_the_constant_term_of_every_line():
             lam = PP.f2mul(PP.f2sub(q[1], t[1]), PP.f2inv(PP.f2sub(q[0], t[0])))
             assert PP.f2sub(PP.f2mul(lam, t[0]), t[1]) != (0, 0)
             t = PP.g2add(t, q)
+
+
+def g1_jac(st, at):
+    x, y, z = st[at:at + 3]
+    if z == 0:
+        return None
+    zi = pow(z, -1, P)
+    return x * zi % P, y * zi % P
+
+
+def test_g1_sums(progs):
+    """Both sums of a doubling and an addition round sequence, with equal points,
+    opposite points and infinity among the operands (homogeneous coordinates)."""
+    rng = random.Random(6)
+    gen = (0x17F1D3A73197D7942695638C4FA9AC0FC3688C4F9774B905A14E3A3F171BAC586C55E83FF97A1AEFFB3AF00ADB22C6BB,
+           0x08B3F481E3AAA0F1A09E30ED741D8AE4FCF5E095D5D00AF600DB18CB2C04B3EDD03CC744A2888AE40CAA232946C5E7E1)
+    a, b = PP.g1mul(rng.randrange(PP.R), gen), PP.g1mul(rng.randrange(PP.R), gen)
+
+    def put3(st, at, p):
+        z = rng.randrange(1, P)
+        st[at:at + 3] = (0, z, 0) if p is None else (p[0] * z % P, p[1] * z % P, z)
+
+    cases = [(a, b), (a, a), (a, PP.g1neg(a)), (None, b), (a, None), (None, None)]
+    for x, y in zip(cases, cases[1:] + cases[:1]):
+        st = state(progs, 7)
+        for j, (p, q) in enumerate((x, y)):
+            put3(st, G.VA + 3 * j, p)
+            put3(st, G.VQ + 3 * j, q)
+        run(progs, st, "VADD")
+        for j, (p, q) in enumerate((x, y)):
+            assert g1_jac(st, G.VA + 3 * j) == PP.g1add(p, q)
+        run(progs, st, "VDBL")
+        for j, (p, q) in enumerate((x, y)):
+            s = PP.g1add(p, q)
+            assert g1_jac(st, G.VA + 3 * j) == PP.g1add(s, s)
