@@ -99,7 +99,8 @@ int fk20_ctx_msm(fk20_ctx *ctx, g1p_t *hext_fft, const fr_t *tc_fft, unsigned ro
  * `polys`) and m_j proofs written at out_off[j] (in g1p_t units from `h_fft`).
  * All offset arrays are HOST arrays (read before the call returns).  The
  * instances are grouped into one segment per length, and all segments run in
- * ONE fixed-base MSM launch and ONE persistent stage-fused G1 FFT launch.
+ * ONE fixed-base MSM launch and ONE persistent launch of the map from hext_fft
+ * to h_fft.
  * No reference counterpart (the reference proves one length per call). */
 int fk20_ctx_batch(fk20_ctx *ctx, g1p_t *h_fft, const fr_t *polys, unsigned count, const unsigned *n,
                    const size_t *poly_off, const size_t *out_off, void *stream);
@@ -132,15 +133,15 @@ typedef struct {
 int fk20_ctx_autotune(fk20_ctx *ctx, unsigned n, unsigned rows, size_t max_table_bytes, fk20_tune_result *result,
                       void *stream);
 
-/* Options.  FK20_OPT_FUSED_FFT (default 1): run the inverse and forward G1
- * FFT stages of the pipeline as one persistent launch whose warps take
- * butterfly tasks in stage order and wait (bounded) for their inputs, instead
- * of one launch per stage. */
+/* Options.  FK20_OPT_FUSED_FFT (default 1): run the pipeline's map from hext_fft
+ * to h_fft (inverse G1 FFT, upper half to infinity, forward FFT) as one
+ * persistent launch whose warps take tasks in dependency order and wait
+ * (bounded) for their inputs, instead of one launch per level of tasks. */
 #define FK20_OPT_FUSED_FFT 1
 /* FK20_OPT_MSM_THREADS: MSM block size, 64, 128 (default) or 256 threads. */
 #define FK20_OPT_MSM_THREADS 2
-/* FK20_OPT_FFT_BLOCKS_PER_SM: persistent FFT grid, blocks per SM (0 =
- * default: as many as fit). */
+/* FK20_OPT_FFT_BLOCKS_PER_SM: grid of that launch, blocks per SM (0 = default:
+ * four, or six where the number of products pays for them). */
 #define FK20_OPT_FFT_BLOCKS_PER_SM 3
 /* FK20_OPT_WAIT_LIMIT: polls a readiness wait of the persistent FFT makes
  * before it gives up and the launch reports FK20_ETIMEOUT (0 = default 2^24). */
