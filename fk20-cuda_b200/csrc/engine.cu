@@ -2027,7 +2027,7 @@ void CUDART_CB pack_done_cb(void *p) {
 }
 
 // inputs to pinned staging, one H2D copy, the segment pipeline, one D2H copy
-int enqueue_pack(fk20_server *s, Slot &sl, bool latency) {
+int enqueue_pack(fk20_server *s, Slot &sl) {
     const size_t cnt = sl.reqs.size();
     std::vector<unsigned> ns(cnt);
     std::vector<size_t> poly_off(cnt), out_off(cnt);
@@ -2053,17 +2053,10 @@ int enqueue_pack(fk20_server *s, Slot &sl, bool latency) {
         Seg sg[3];
         int nseg = 0;
         CKR(batch_segments(ctx, sl.ws, (unsigned)cnt, ns.data(), poly_off.data(), out_off.data(), sg, &nseg, sl.st));
-        // The persistent FFT's blocks per SM.  Adaptive by default: a
-        // latency-mode pack may fill the GPU, and the next pack's blocks take
-        // over as its own retire (a pack alone finishes in about half the
-        // time); a throughput-mode pack takes 1/slots of the SMs, so packs of
-        // different slots run side by side and hide each other's dependency
-        // waits.
-        int share = 0;  // by the number of products
-        if (s->cfg.fft_blocks_per_sm)
-            share = std::min((int)s->cfg.fft_blocks_per_sm, ctx->proj_occupancy);
-        else if (!latency)
-            share = std::max(1, ctx->proj_occupancy / (int)s->slots.size());
+        // Blocks per SM of the pack's projection: the caller's, or by its number of
+        // products.  (Halving them for packs of two slots, so that they run side
+        // by side, idled the chip while the other pack was in its MSM.)
+        const int share = s->cfg.fft_blocks_per_sm ? std::min((int)s->cfg.fft_blocks_per_sm, ctx->proj_occupancy) : 0;
         CKR(run_segments(ctx, sl.ws, sg, nseg, (const fr_t *)sl.dpoly.p, (g1p_t *)sl.dout.p, true, sl.st, false,
                          share));
     }
@@ -2213,7 +2206,7 @@ void server_main(fk20_server *s) {
                 for (const Req &r : fs->reqs)
                     s->sum_wait_ms += std::chrono::duration<double, std::milli>(fs->t_form - r.t0).count();
                 lk.unlock();
-                fs->rc = enqueue_pack(s, *fs, latency);
+                fs->rc = enqueue_pack(s, *fs);
                 fs->t_enq = Clock::now();
                 lk.lock();
                 s->sum_enqueue_ms += std::chrono::duration<double, std::milli>(fs->t_enq - fs->t_form).count();
