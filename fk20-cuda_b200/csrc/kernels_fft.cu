@@ -1,5 +1,6 @@
-// kernels_fft.cu -- G1 FFT stages on row-interleaved tiles, and the
-// reference <-> tile conversions.
+// kernels_fft.cu -- radix-2 G1 FFT stages on row-interleaved tiles (setup, the
+// no-allocation transforms, the cohort engine), and the reference <-> tile
+// conversions.
 //
 // One warp per (butterfly, group of 32 rows): the twiddle of a butterfly is
 // the same for all 32 rows, so its GLV/NAF program (scalar_prog.cuh) runs
@@ -95,8 +96,9 @@ __global__ void __launch_bounds__(FFT_THREADS, FK_FFT_MINB) k_g1_stage(uint4 *__
 }
 
 // ------------------------------------------------------------------ fused stages
-// One persistent launch runs the whole hext -> h_fft sequence of the plain
-// pipeline -- inverse DIF stages 0..L-2, the middle stage, forward DIT stages
+// The radix-2 persistent launch of the server's cohort engine, whose launches
+// advance by stage windows (the plain pipeline's is kernels_proj.cu): the
+// hext -> h_fft sequence -- inverse DIF stages 0..L-2, the middle stage, forward DIT stages
 // 1..L-1 -- for every segment of the plan (segments may differ in length).
 // Work is a stream of warp tasks (one butterfly of 32 rows) taken in order
 // from a global counter; the stream is cut into blocks of (segment, stage) in

@@ -25,8 +25,8 @@
 // kernel the interpolation falls on the constants: beta solves the dual
 // Vandermonde system of the points.
 //
-// Scalar products per instance: 867 for m = 512, 402 for 256, 177 for 128 --
-// 1,734 / 804 / 354 a row, against 3,586 / 1,538 / 642 twiddle products in the
+// Scalar products per instance: 865 for m = 512, 400 for 256, 175 for 128 --
+// 1,730 / 800 / 350 a row, against 3,586 / 1,538 / 642 twiddle products in the
 // two FFTs -- and they are independent of each other: one product deep instead
 // of 2 log m - 2, which is what bounds a small batch.
 #pragma once
