@@ -19,10 +19,11 @@ cudaError_t upload_consts_fr() { return upload_module_consts(); }
 //
 // The multiply pipe's share at m = 512 is 1,793 products a transform (0.13 ms
 // for 4,000); one stage at a time through sm[m][8] took 0.35 ms, its eight-word
-// stride an eight-way bank conflict on every access; this takes 0.21 ms.
+// stride an eight-way bank conflict on every access; this takes 0.21 ms (128-thread blocks at 134
+// registers 0.22; for 4,000 transforms of 128 values 0.055 against 0.072).
 //
 // Load: fn(natural index) -> value, store: fn(index, value).
-constexpr int FR_THREADS = 128;  // threads of a block: 128 / (m / 8) transforms
+constexpr int FR_THREADS = 64;  // threads of a block: 64 / (m / 8) transforms
 constexpr int FR_STRIDE = FR_THREADS * 9;
 constexpr int FR_SMEM_WORDS = 8 * FR_STRIDE;
 
@@ -133,7 +134,7 @@ __device__ __forceinline__ void store_scalar(uint4 *dst, const uint32_t v[8]) {
 
 // transform (row, i) = 16 row + i of the launch: toeplitz -> FFT -> scalar
 // tiles S[g][c][i][q][lane], group g at S + g * stride
-__global__ void __launch_bounds__(FR_THREADS) k_tc_fft(uint4 *__restrict__ S, size_t stride, const uint64_t *__restrict__ poly,
+__global__ void __launch_bounds__(FR_THREADS, 8) k_tc_fft(uint4 *__restrict__ S, size_t stride, const uint64_t *__restrict__ poly,
                                                       const size_t *__restrict__ row_off, int n, int log_m, unsigned rows) {
     __shared__ uint32_t sm[FR_SMEM_WORDS];
     const int m8 = 1 << (log_m - 3), sub = threadIdx.x / m8, t = threadIdx.x % m8;
@@ -156,7 +157,7 @@ __global__ void __launch_bounds__(FR_THREADS) k_tc_fft(uint4 *__restrict__ S, si
 // batched Fr FFT on reference arrays, natural order in and out (fr_fft_wrapper /
 // fr_ift_wrapper, fr_fft.cu:318-363); the inverse includes 1/m.  Each block
 // reads its whole transforms before writing, so in-place calls are safe.
-__global__ void __launch_bounds__(FR_THREADS) k_fr_fft_ref(uint64_t *out, const uint64_t *in, int log_m, unsigned count,
+__global__ void __launch_bounds__(FR_THREADS, 8) k_fr_fft_ref(uint64_t *out, const uint64_t *in, int log_m, unsigned count,
                                                           int inverse) {
     __shared__ uint32_t sm[FR_SMEM_WORDS];
     const int m8 = 1 << (log_m - 3), sub = threadIdx.x / m8, t = threadIdx.x % m8;
