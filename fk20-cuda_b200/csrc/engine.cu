@@ -7,7 +7,7 @@
 //   - contexts: fixed-base MSM tables per polynomial length, commitment
 //     tables, options, a workspace;
 //   - the segment pipeline (run_segments): toeplitz Fr FFTs, one MSM launch
-//     and one persistent G1 FFT launch over up to 8 segments, outputs;
+//     and one persistent projection launch over up to 8 segments, outputs;
 //   - batch plans (CUDA graphs of that pipeline), the autotuner, and the
 //     continuous-batching request server (a worker thread and its slots);
 //   - the launch sequence of every entry point.
@@ -177,12 +177,24 @@ const HostPlan &host_plan(PlanKind kind, int log_m) {
     return h;
 }
 
+// builds the plan if it is not there yet (no exception leaves the library)
+int plan_ready(PlanKind kind, int log_m) {
+    try {
+        (void)host_plan(kind, log_m);
+    } catch (...) {
+        return FK20_ENOMEM;
+    }
+    return 0;
+}
+
 std::mutex g_plan_mu;
 DevPlan g_dev_plan[64][PLAN_KINDS][MAX_LOG_M + 1];
 
 // the plan on the current device `dev`
 int device_plan(int dev, PlanKind kind, int log_m, DevPlan *out) {
     if (dev < 0 || dev >= 64) return FK20_ENODEV;
+    const int built = plan_ready(kind, log_m);
+    if (built) return built;
     const HostPlan &h = host_plan(kind, log_m);
     std::lock_guard<std::mutex> lk(g_plan_mu);
     DevPlan &d = g_dev_plan[dev][kind][log_m];
@@ -326,6 +338,7 @@ struct Workspace {
     cudaEvent_t offs_done = nullptr;   // the last copy out of offs_host
     int init() {
         if (err_host) return 0;
+        OutsideCapture outside;
         if (cudaMallocHost(&err_host, sizeof(int)) != cudaSuccess) {
             cudaGetLastError();
             err_host = nullptr;
@@ -471,6 +484,7 @@ struct fk20_ctx {
         int n = 0, cb = 0, W = 0;
     } commit;
     Workspace ws;   // the context's own calls
+    Workspace pts;  // transforms of points: apart, so that they may run beside a pipeline call on another stream
     DevBuf D2, scratch, xext, fp_dev;
     DevBuf verify;  // check_proof_multi intermediates
     Profiler prof;
@@ -1039,9 +1053,13 @@ int setup2xext(fk20_ctx *ctx, g1p_t *xext_fft, const g1p_t *setup, unsigned n, c
 int run_points(fk20_ctx *ctx, PlanKind kind, g1p_t *out, const g1p_t *in, int log_m, unsigned rows, cudaStream_t st) {
     const size_t m = (size_t)1 << log_m;
     const int two = kind == PLAN_PROJ_HALF;
-    Workspace &ws = ctx->ws;
+    Workspace &ws = ctx->pts;
     CKR(ws.init());
-    if (*ws.err_host) return launch_error(*ws.err_host);
+    if (*ws.err_host) {  // the previous call's launch gave up: reported once
+        const int rc = launch_error(*ws.err_host);
+        *ws.err_host = 0;
+        return rc;
+    }
     DevPlan d;
     CKR(device_plan(ctx->device, kind, log_m, &d));
     const int slots = host_plan(kind, log_m).plan.slots;
@@ -1170,6 +1188,7 @@ int fk20_ctx_destroy(fk20_ctx *ctx) {
         ctx->commit.table.release();
         ctx->commit.part.release();
         ctx->ws.release();
+        ctx->pts.release();
         ctx->D2.release();
         ctx->scratch.release();
         ctx->xext.release();
@@ -1219,7 +1238,7 @@ int fk20_program_cost(int index, int *dbl, int *add) {
 
 size_t fk20_ctx_device_bytes(const fk20_ctx *ctx) {
     if (!ctx) return 0;
-    size_t b = ctx->ws.bytes() + ctx->D2.bytes + ctx->scratch.bytes + ctx->xext.bytes;
+    size_t b = ctx->ws.bytes() + ctx->pts.bytes() + ctx->D2.bytes + ctx->scratch.bytes + ctx->xext.bytes;
     for (auto &t : ctx->tab) b += t.table.bytes + t.xext.bytes;
     b += ctx->commit.table.bytes + ctx->commit.part.bytes;
     return b;
@@ -2582,6 +2601,7 @@ int fk20_server_create(fk20_server **out, fk20_ctx *ctx, const fk20_server_confi
     if (!c.burst_rows) c.burst_rows = std::min(4096u, c.max_rows + c.max_rows * 2 / 5);
     if (c.burst_rows < c.max_rows || c.burst_rows > 4096) return FK20_EINVAL;
     if (c.engine > 1) return FK20_EINVAL;
+    for (int log_m = 7; log_m <= 9; log_m++) CKR(plan_ready(PLAN_PROJ, log_m));  // pack sizes need their slots
     if (!c.cohort_rows) c.cohort_rows = 64;
     if (!c.cohorts) c.cohorts = 16;
     if (!c.form_ms) c.form_ms = 25;
