@@ -183,6 +183,66 @@ __global__ void __launch_bounds__(FR_THREADS, 8) k_fr_fft_ref(uint64_t *out, con
         });
 }
 
+// Few transforms: a butterfly a thread and a barrier a stage, grid (count),
+// block m / 2.  A call that leaves the chip idle costs its chain of products: one
+// a stage here, up to twelve a pass in registers above (a small call 18 us
+// against 35).  4,000 transforms of 512 values take 0.35 ms here (bank
+// conflicts of the eight-word stride) and 0.20 above.  So this serves what is
+// resident at once, 12 blocks of 16 KB to an SM, up to 1,024 values to an SM;
+// at 296 transforms of 512 the rates of the full chip would give 26 us here,
+// while 500 take 45 us above.
+constexpr unsigned FR_FEW_COUNT = 148 * 12, FR_FEW_VALUES = 148 * 1024;
+__global__ void __launch_bounds__(256) k_fr_fft_few(uint64_t *out, const uint64_t *in, int log_m, int inverse) {
+    __shared__ uint32_t sm[512][8];
+    const int m = 1 << log_m, tid = threadIdx.x;
+    const uint64_t *src = in + 4 * (size_t)blockIdx.x * m;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int p = tid + h * (m >> 1);
+        Fr v;
+        fr_from_ref(v, src + 4 * (size_t)p);
+        const int d = (int)bitrev((unsigned)p, log_m);
+#pragma unroll
+        for (int k = 0; k < 8; k++) sm[d][k] = v.w[k];
+    }
+    __syncthreads();
+    for (int s = 0; s < log_m; s++) {
+        const int half = 1 << s, j = tid & (half - 1), i0 = ((tid >> s) << (s + 1)) | j, i1 = i0 + half;
+        Fr u, v, t;
+#pragma unroll
+        for (int k = 0; k < 8; k++) { u.w[k] = sm[i0][k]; v.w[k] = sm[i1][k]; }
+        const int texp = j << (log_m - 1 - s);  // power of w_m
+        if (texp != 0) {
+            int tix = (texp << (MAX_LOG_M - log_m)) & 511;  // power of w_512
+            if (inverse) tix = (512 - tix) & 511;
+#pragma unroll
+            for (int k = 0; k < 8; k++) t.w[k] = g_fr_tw[tix][k];
+            f_mul(v, v, t);
+        }
+        Fr x, y;
+        f_add(x, u, v);
+        f_sub(y, u, v);
+#pragma unroll
+        for (int k = 0; k < 8; k++) { sm[i0][k] = x.w[k]; sm[i1][k] = y.w[k]; }
+        __syncthreads();
+    }
+    uint64_t *dst = out + 4 * (size_t)blockIdx.x * m;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int c = tid + h * (m >> 1);
+        Fr v;
+#pragma unroll
+        for (int k = 0; k < 8; k++) v.w[k] = sm[c][k];
+        if (inverse) {
+            Fr s;
+#pragma unroll
+            for (int k = 0; k < 8; k++) s.w[k] = g_fr_inv2[log_m][k];
+            f_mul(v, v, s);
+        }
+        fr_to_ref(dst + 4 * (size_t)c, v);
+    }
+}
+
 // transforms of 2 and 4 points, one thread each
 __global__ void k_fr_fft_tiny(uint64_t *out, const uint64_t *in, int log_m, unsigned count, int inverse) {
     const unsigned tr = blockIdx.x * blockDim.x + threadIdx.x;
@@ -251,6 +311,10 @@ void launch_tc_fft(uint4 *S, size_t stride, const uint64_t *poly, const size_t *
 void launch_fr_fft_ref(uint64_t *out, const uint64_t *in, int log_m, unsigned count, int inverse, cudaStream_t st) {
     if (log_m < 3) {
         k_fr_fft_tiny<<<blocks_for(count, 64), 64, 0, st>>>(out, in, log_m, count, inverse);
+        return;
+    }
+    if (count <= FR_FEW_COUNT && ((size_t)count << log_m) <= FR_FEW_VALUES) {
+        k_fr_fft_few<<<count, 1u << (log_m - 1), 0, st>>>(out, in, log_m, inverse);
         return;
     }
     const unsigned per = FR_THREADS >> (log_m - 3);

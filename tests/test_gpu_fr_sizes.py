@@ -22,3 +22,17 @@ def test_fr_fft_every_size(engine, log_m, inverse):
     assert np.array_equal(engine.to_host(out), exp)
     engine.call("fr_fft_n", engine._ptr(d), engine._ptr(d), log_m, count, inverse, engine._stream())
     assert np.array_equal(engine.to_host(d), exp)
+
+
+@pytest.mark.parametrize("log_m", range(3, 10))
+@pytest.mark.parametrize("past", [0, 1])
+def test_fr_fft_around_the_line(engine, log_m, past):
+    """The largest count of the kernel for few transforms, and one more."""
+    m = 1 << log_m
+    count = min(148 * 12, 148 * 1024 // m) + past
+    x = O.seeded_fr(60 + log_m, count * m).reshape(count, m, 4)
+    d = engine.to_device(x)
+    for inverse in (0, 1):
+        out = engine.empty(x.shape)
+        engine.call("fr_fft_n", engine._ptr(out), engine._ptr(d), log_m, count, inverse, engine._stream())
+        assert np.array_equal(engine.to_host(out), O.fr_fft(x, inverse=bool(inverse)))
