@@ -332,7 +332,7 @@ struct Tables {
 // they can run on different streams at once against the same tables.
 struct Workspace {
     DevBuf S, D, offs, sync;           // sync: [task counter | error flag | pad][readiness counters]
-    int *err_host = nullptr;           // pinned copy of the last persistent launch's error flag
+    int *err_host = nullptr;           // pinned: the code of a persistent launch that gave up, until it is reported
     size_t *offs_host = nullptr;       // pinned staging of offset arrays
     size_t offs_cap = 0;               // entries of offs_host
     cudaEvent_t offs_done = nullptr;   // the last copy out of offs_host
@@ -806,6 +806,7 @@ int run_plan(fk20_ctx *ctx, Workspace &ws, const SegLayout &lay, const int *log_
     p.nseg = nseg;
     p.next = (unsigned *)ws.sync.p;
     p.err = (int *)((char *)ws.sync.p + 128);
+    p.report = ws.err_host;
     p.spin_limit = ctx->wait_limit;
     p.unpublished = ctx->unpublished;
     // persistent grid: the context's setting, or the caller's share of the SMs (server packs)
@@ -838,7 +839,6 @@ int run_plan(fk20_ctx *ctx, Workspace &ws, const SegLayout &lay, const int *log_
         }
     }
     ctx->prof.end(st);
-    CK(cudaMemcpyAsync(ws.err_host, p.err, sizeof(int), cudaMemcpyDeviceToHost, st));
     return 0;
 }
 
@@ -1055,11 +1055,6 @@ int run_points(fk20_ctx *ctx, PlanKind kind, g1p_t *out, const g1p_t *in, int lo
     const int two = kind == PLAN_PROJ_HALF;
     Workspace &ws = ctx->pts;
     CKR(ws.init());
-    if (*ws.err_host) {  // the previous call's launch gave up: reported once
-        const int rc = launch_error(*ws.err_host);
-        *ws.err_host = 0;
-        return rc;
-    }
     DevPlan d;
     CKR(device_plan(ctx->device, kind, log_m, &d));
     const int slots = host_plan(kind, log_m).plan.slots;
@@ -1171,10 +1166,21 @@ int fk20_ctx_status(fk20_ctx *ctx) {
     std::lock_guard<std::mutex> lk(ctx->mu);
     DeviceGuard dg(ctx->device);
     CK(cudaDeviceSynchronize());
-    if (ctx->ws.err_host && *ctx->ws.err_host) {
-        const int rc = launch_error(*ctx->ws.err_host);
-        *ctx->ws.err_host = 0;
-        return rc;
+    int rc = 0;
+    for (Workspace *w : {&ctx->ws, &ctx->pts})
+        if (w->err_host && *w->err_host) {
+            if (!rc) rc = launch_error(*w->err_host);
+            *w->err_host = 0;
+        }
+    return rc;
+}
+
+int fk20_default_status(int device) {
+    if (device < 0 || device >= 64) return FK20_EINVAL;
+    fk20_ctx *c = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_default_mu);
+        c = g_default[device];
     }
     return 0;
 }
@@ -1196,7 +1202,15 @@ int fk20_ctx_destroy(fk20_ctx *ctx) {
         ctx->verify.release();
     }
     delete ctx;
-    return 0;
+    return c ? fk20_ctx_status(c) : 0;
+}
+
+int fk20_default_set(int device, int option, int value) {
+    if (device < 0 || device >= 64) return FK20_EINVAL;
+    DeviceGuard dg(device);
+    fk20_ctx *c;
+    CKR(default_ctx(&c));
+    return fk20_ctx_set(c, option, value);
 }
 
 int fk20_ctx_profile(fk20_ctx *ctx, int enable) {

@@ -89,6 +89,16 @@ struct TileU {
     }
 };
 
+// The launch gives up: the other warps stop at their next task, and the host
+// learns of it from a word of its own.  That word is written only here, so a
+// later launch that succeeds does not take the report away.
+FK_D void proj_stop(const ProjArgs &P, int code) {
+    if (atomicCAS(P.err, 0, code) == 0) {
+        *(volatile int *)P.report = code;
+        __threadfence_system();
+    }
+}
+
 }  // namespace
 
 // Six blocks (12 warps) an SM, 168 registers: with three warps a scheduler the
@@ -122,7 +132,7 @@ __global__ void __launch_bounds__(FFT_THREADS, 6) k_proj(const __grid_constant__
                                         (t.d1 == PROJ_NONE || t.d1 < A.slots),
                       FK20_CHECK_FFT_TASK) ||
             !FK_CHECK(g_check_proj, t.op != PROJ_MUL || t.prog < S.nprog, FK20_CHECK_FFT_PROGRAM)) {
-            if (lane == 0) atomicCAS(P.err, 0, 2000);
+            if (lane == 0) proj_stop(P, 2000);
             return;
         }
         unsigned *rg = S.ready + (size_t)g * (A.slots + 1);
@@ -154,7 +164,7 @@ __global__ void __launch_bounds__(FFT_THREADS, 6) k_proj(const __grid_constant__
         ok = __all_sync(0xffffffffu, ok);
         __threadfence();
         if (!ok) {
-            if (lane == 0) atomicCAS(P.err, 0, 1000 + t.phase);
+            if (lane == 0) proj_stop(P, 1000 + t.phase);
             return;
         }
         const uint4 *pa = S.D + proj_tile(A, g, t.a);

@@ -73,6 +73,7 @@ struct ProjArgs {
     unsigned first, last;  // launch indices to run
     unsigned *next;        // task counter (zeroed before the launch)
     int *err;              // 0 = ok, else 1000 + phase that timed out, 2000 a failed check
+    int *report;           // pinned host word: gets err when it is set, and keeps it until the host clears it
     unsigned spin_limit;   // polls before a wait gives up
     unsigned unpublished;  // as FusedPlan::unpublished
 };

@@ -43,7 +43,7 @@ ABI_SYMBOLS = (
     "fk20_g1p_compress_n", "fk20_h_fft2proofs", "fk20_ctx_poly2proofs", "fk20_ctx_batch_proofs",
     "fk20_ctx_load_commit", "fk20_ctx_commit", "fk20_pairing_check_n", "fk20_pairing_n", "g2p_op_n",
     "fk20_ctx_check_proof_multi", "fk20_default_release", "fk20_check_status", "fk20_server_cancel",
-    "fk20_test_fail_allocations",
+    "fk20_test_fail_allocations", "fk20_default_status", "fk20_default_set",
 )
 
 # kernel kinds of the per-launch profiler (FK20_K_* in the header)
@@ -176,6 +176,8 @@ def lib() -> ctypes.CDLL:
             "fk20_pairing_n": ([vp, vp, vp, sz, vp], i),
             "g2p_op_n": ([i, vp, vp, vp, sz, vp], i),
             "fk20_default_release": ([i], i),
+            "fk20_default_status": ([i], i),
+            "fk20_default_set": ([i, i, i], i),
             "fk20_check_status": ([ctypes.POINTER(i)], i),
             "fk20_server_cancel": ([vp, ctypes.c_uint64], i),
             "fk20_test_fail_allocations": ([i], i),

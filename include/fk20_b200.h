@@ -367,6 +367,15 @@ int fk20_poly2h_fft(g1p_t *h_fft, const fr_t *polynomial, const g1p_t *xext_fft,
  * that device builds them again.  No call may be in flight on it. */
 int fk20_default_release(int device);
 
+/* fk20_ctx_status and fk20_ctx_set of `device`'s default context.  The
+ * transforms of points (g1p_fft and its relatives, fk20_hext_fft2h_fft) run
+ * persistent launches with bounded waits on it: one that gives up leaves its
+ * output invalid, later calls run as usual, and fk20_default_status returns
+ * FK20_ETIMEOUT once.  With FK20_OPT_FUSED_FFT 0 they run one launch per level
+ * of tasks instead, in which nothing waits. */
+int fk20_default_status(int device);
+int fk20_default_set(int device, int option, int value);
+
 /* No counterpart in the reference (it has no checked build; its debug build
  * asserts).  In the checked build (libfk20b200_checked.so, `make checked`)
  * the MSM and the persistent G1 FFT check their task decoding, tile and table
