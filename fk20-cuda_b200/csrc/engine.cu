@@ -891,7 +891,7 @@ int run_pass(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, const fr_t *
         CKR(run_plan(ctx, ws, lay, log_m, rows, nseg, PLAN_PROJ, first, fft_bps, st));
     }
     for (int k = 0; k < nseg; k++) {
-        TileView v{D + lay.d_off[k] / U, nullptr, lay.arena[k], 1};
+        TileView v{D + lay.d_off[k] / U, nullptr, lay.arena[k], 1, 0};
         if (full) {
             DevPlan d;
             CKR(device_plan(ctx->device, PLAN_PROJ, sg[k].log_m, &d));
@@ -1043,15 +1043,36 @@ int setup2xext(fk20_ctx *ctx, g1p_t *xext_fft, const g1p_t *setup, unsigned n, c
         launch_g1_stage(D, 1, log_m, s, 1, st);
         CKL();
     }
-    launch_tile_to_ref((uint64_t *)xext_fft, TileView{D, nullptr, {}, 0}, nullptr, L_COLS, log_m, 0, st);
+    launch_tile_to_ref((uint64_t *)xext_fft, TileView{D, nullptr, {}, 0, 0}, nullptr, L_COLS, log_m, 0, st);
     CKL();
     return 0;
 }
 
+// Transforms that keep the radix-2 stages: those whose stages are no deeper in
+// products than their plan, two points, and four forward.  What a plan adds to
+// them, its task queue and normalised outputs (an inversion a point), is most of
+// such a call, and the bandwidth of a large one.  B200, two points forward: one
+// transform 62 us by stages and 118 by plan, 100,000 229 and 10,385; inverse, one
+// 1.12 and 1.15 ms.  Four points forward, one: 0.63 and 0.69 ms.  Four inverse, with
+// stages two products deep, 1.70 and 1.20 ms: the plan.
+bool by_stages(PlanKind kind, int log_m) { return log_m == 1 || (log_m == 2 && kind == PLAN_DFT); }
+
+int run_stages(fk20_ctx *ctx, PlanKind kind, g1p_t *out, const g1p_t *in, int log_m, unsigned rows, int raw,
+               cudaStream_t st) {
+    CKR(ctx->D2.reserve(tile_bytes((int)((rows + 31) / 32), 1 << log_m)));
+    return (int)launch_g1_transform((uint64_t *)out, (const uint64_t *)in, (uint4 *)ctx->D2.p, log_m, (int)rows,
+                                    kind == PLAN_IDFT, raw, st);
+}
+
 // A plan on `rows` rows of m = 2^log_m points (reference layout, natural order
-// in and out; out may be in), at most PASS_ROWS rows at a time
+// in and out; out may be in), at most PASS_ROWS rows of 512 points, or as many
+// more as they are shorter, at a time.  (Passes of 1024 rows whatever their length
+// paid the depth of a plan, 0.7 to 1.7 ms, for each: 30,000 transforms of 8 points
+// 50.9 ms.)
 int run_points(fk20_ctx *ctx, PlanKind kind, g1p_t *out, const g1p_t *in, int log_m, unsigned rows, cudaStream_t st) {
+    if (by_stages(kind, log_m)) return run_stages(ctx, kind, out, in, log_m, rows, 1, st);
     const size_t m = (size_t)1 << log_m;
+    const unsigned pass = PASS_ROWS << (MAX_LOG_M - log_m);
     const int two = kind == PLAN_PROJ_HALF;
     Workspace &ws = ctx->pts;
     CKR(ws.init());
@@ -1062,11 +1083,11 @@ int run_points(fk20_ctx *ctx, PlanKind kind, g1p_t *out, const g1p_t *in, int lo
         const int G = (int)((n + 31) / 32);
         return two ? proj_arena(slots, n) : ProjArena{slots, G, G, 0};
     };
-    const ProjArena most = arena(std::min(rows, PASS_ROWS));
+    const ProjArena most = arena(std::min(rows, pass));
     CKR(ws.D.reserve(arena_bytes(most)));
     CKR(ws.sync.reserve(SYNC_HDR + ready_bytes(most)));
-    for (unsigned r0 = 0; r0 < rows; r0 += PASS_ROWS) {
-        const unsigned n = std::min(rows - r0, PASS_ROWS);
+    for (unsigned r0 = 0; r0 < rows; r0 += pass) {
+        const unsigned n = std::min(rows - r0, pass);
         SegLayout lay;
         lay.arena[0] = arena(n);
         lay.d_off[0] = lay.r_off[0] = 0;
@@ -1074,7 +1095,7 @@ int run_points(fk20_ctx *ctx, PlanKind kind, g1p_t *out, const g1p_t *in, int lo
         launch_ref_to_arena((uint4 *)ws.D.p, lay.arena[0], (const uint64_t *)(in + r0 * m), (int)n, log_m, two, st);
         CKL();
         CKR(run_plan(ctx, ws, lay, &log_m, &n, 1, kind, r0 == 0, 0, st));
-        const TileView v{(const uint4 *)ws.D.p, d.out, lay.arena[0], two};
+        const TileView v{(const uint4 *)ws.D.p, d.out, lay.arena[0], two, 0};
         launch_tile_to_ref((uint64_t *)(out + r0 * m), v, nullptr, (int)n, log_m, 0, st);
         CKL();
     }
@@ -1182,7 +1203,15 @@ int fk20_default_status(int device) {
         std::lock_guard<std::mutex> lk(g_default_mu);
         c = g_default[device];
     }
-    return 0;
+    return c ? fk20_ctx_status(c) : 0;
+}
+
+int fk20_default_set(int device, int option, int value) {
+    if (device < 0 || device >= 64) return FK20_EINVAL;
+    DeviceGuard dg(device);
+    fk20_ctx *c;
+    CKR(default_ctx(&c));
+    return fk20_ctx_set(c, option, value);
 }
 
 int fk20_ctx_destroy(fk20_ctx *ctx) {
@@ -1202,15 +1231,7 @@ int fk20_ctx_destroy(fk20_ctx *ctx) {
         ctx->verify.release();
     }
     delete ctx;
-    return c ? fk20_ctx_status(c) : 0;
-}
-
-int fk20_default_set(int device, int option, int value) {
-    if (device < 0 || device >= 64) return FK20_EINVAL;
-    DeviceGuard dg(device);
-    fk20_ctx *c;
-    CKR(default_ctx(&c));
-    return fk20_ctx_set(c, option, value);
+    return 0;
 }
 
 int fk20_ctx_profile(fk20_ctx *ctx, int enable) {
@@ -1326,7 +1347,7 @@ int fk20_ctx_msm(fk20_ctx *ctx, g1p_t *hext_fft, const fr_t *tc_fft, unsigned ro
     launch_ref_to_scalars((uint4 *)ctx->ws.S.p, (const uint64_t *)tc_fft, (int)rows, log_m, st);
     CKL();
     CKR(msm_launch(ctx, T, (uint4 *)ctx->ws.D.p, (const uint4 *)ctx->ws.S.p, G, (int)rows, 1, st));
-    CKR(output_launch(ctx->prof, (uint64_t *)hext_fft, TileView{(const uint4 *)ctx->ws.D.p, nullptr, {}, 0}, nullptr, (int)rows,
+    CKR(output_launch(ctx->prof, (uint64_t *)hext_fft, TileView{(const uint4 *)ctx->ws.D.p, nullptr, {}, 0, 0}, nullptr, (int)rows,
                       log_m, 0, st));
     return 0;
 }
@@ -2352,7 +2373,7 @@ int cohort_launch(fk20_server *s, const std::vector<int> &act) {
         c.stage = p.blk.s_hi[k];
         if (c.stage < 2 * c.log_m - 1) continue;
         const int m = 1 << c.log_m;
-        launch_tile_to_ref((uint64_t *)b.dout.p, TileView{(const uint4 *)b.D.p, nullptr, {}, 0}, nullptr, c.rows, c.log_m, 0, st);
+        launch_tile_to_ref((uint64_t *)b.dout.p, TileView{(const uint4 *)b.D.p, nullptr, {}, 0, 0}, nullptr, c.rows, c.log_m, 0, st);
         CKL();
         CK(cudaMemcpyAsync(b.hout, b.dout.p, (size_t)c.rows * m * sizeof(g1p_t), cudaMemcpyDeviceToHost, st));
         CK(cudaEventRecord(b.out_done, st));

@@ -278,9 +278,9 @@ __global__ void k_ref_to_tile(uint4 *__restrict__ D, const uint64_t *__restrict_
     }
 }
 
-// tiles -> reference g1p_t rows, natural order, normalised (x, y, 1): the
-// words do not depend on the order of additions that led to a point.  Row r is
-// written at dst + 18 * (row_off ? row_off[r] : r * m).
+// tiles -> reference g1p_t rows, natural order, normalised (x, y, 1), so that the
+// words do not depend on the order of additions that led to a point, unless the
+// view is raw.  Row r is written at dst + 18 * (row_off ? row_off[r] : r * m).
 __global__ void k_tile_to_ref(uint64_t *__restrict__ dst, const TileView V, const size_t *__restrict__ row_off,
                               int rows, int log_m, int bitrev_out) {
     const int m = 1 << log_m;
@@ -290,7 +290,7 @@ __global__ void k_tile_to_ref(uint64_t *__restrict__ dst, const TileView V, cons
         const int pos = bitrev_out ? (int)bitrev((unsigned)i, log_m) : i;
         G1P p;
         view_load(p, V, row, pos, m);
-        g1_normalize(p);
+        if (!V.raw) g1_normalize(p);
         const size_t base = row_off ? row_off[row] : (size_t)row * m;
         g1p_to_ref(dst + 18 * (base + i), p);
     }
@@ -340,6 +340,16 @@ void launch_ref_to_tile(uint4 *D, const uint64_t *src, int rows, int G, int log_
 void launch_tile_to_ref(uint64_t *dst, const TileView &v, const size_t *row_off, int rows, int log_m, int bitrev_out,
                         cudaStream_t st) {
     k_tile_to_ref<<<blocks_for((size_t)rows << log_m, 64), 64, 0, st>>>(dst, v, row_off, rows, log_m, bitrev_out);
+}
+cudaError_t launch_g1_transform(uint64_t *out, const uint64_t *in, uint4 *D, int log_m, int count, int inverse, int raw,
+                                cudaStream_t st) {
+    const int G = (count + 31) / 32;
+    // forward: bit-reversed load, DIT stages; inverse: natural load, DIF stages, times 1/m, reorder on store
+    launch_ref_to_tile(D, in, count, G, log_m, !inverse, 0, st);
+    for (int s = 0; s < log_m; s++) launch_g1_stage(D, G, log_m, s, !inverse, st);
+    if (inverse) launch_g1_scale(D, G, log_m, 512 + log_m, st);
+    launch_tile_to_ref(out, TileView{D, nullptr, {}, 0, raw}, nullptr, count, log_m, inverse, st);
+    return cudaGetLastError();
 }
 void launch_hext2h_ref(uint64_t *h, int rows, int log_m, cudaStream_t st) {
     k_hext2h_ref<<<grid_stride_blocks((size_t)rows << (log_m - 1)), 256, 0, st>>>(h, rows, log_m);

@@ -85,11 +85,12 @@ void launch_ref_to_arena(uint4 *D, const ProjArena &A, const uint64_t *src, int 
 // Points read by the output kernels: natural tiles [G][m], or (out != null) an
 // arena.  Entry slot | neg << 16 | phi << 17 of out: position i is out[i], or
 // with two instances out[i / 2] of instance i mod 2, times (-1)^neg phi^phi.
+// raw: reference points are written as they are stored instead of normalised.
 struct TileView {
     const uint4 *D;
     const uint32_t *out;
     ProjArena arena;
-    int two;
+    int two, raw;
 };
 
 // per-module constant upload (one per translation unit)
@@ -141,6 +142,9 @@ void launch_ref_to_tile(uint4 *D, const uint64_t *src, int rows, int G, int log_
                         cudaStream_t st);
 void launch_tile_to_ref(uint64_t *dst, const TileView &v, const size_t *row_off, int rows, int log_m, int bitrev_out,
                         cudaStream_t st);
+// `count` radix-2 transforms, natural order in and out (out may be in), through the tiles D[(count + 31) / 32][m]
+cudaError_t launch_g1_transform(uint64_t *out, const uint64_t *in, uint4 *D, int log_m, int count, int inverse, int raw,
+                                cudaStream_t st);
 void launch_hext2h_ref(uint64_t *h, int rows, int log_m, cudaStream_t st);
 void launch_setup_to_tile(uint4 *D, const uint64_t *setup, int n, int log_m, cudaStream_t st);
 

@@ -52,3 +52,25 @@ def test_abandoned_transform_is_reported_and_refuses_nothing(engine, call):
     assert lib.fk20_default_status(dev) == 0
     assert lib.fk20_default_status(-1) == engine.FK20_EINVAL
     assert lib.fk20_default_set(dev, 99, 0) == engine.FK20_EINVAL
+
+
+@pytest.mark.parametrize("inverse", [0, 1])
+@pytest.mark.parametrize("log_m,count", [(1, 1), (1, 33), (1, 5000), (2, 1), (2, 40), (2, 5000), (3, 4097), (3, 65536 + 40),
+                                         (4, 2050)])
+def test_short_transforms_by_stages_and_in_passes(engine, log_m, count, inverse):
+    """Two points, and four forward, go by radix-2 stages; longer ones by plans, 2^19
+    points of rows a pass.  Blocks of distinct transforms repeat, so that only the
+    first needs the oracle."""
+    import torch
+    m, distinct = 1 << log_m, min(count, 24)
+    x = points(40 + log_m, distinct * m).reshape(distinct, m, 18)
+    src = engine.to_device(x).repeat((count + distinct - 1) // distinct, 1, 1)[:count].contiguous()
+    out = engine.empty((count, m, 18))
+    engine.call("g1p_fft_n", engine._ptr(out), engine._ptr(src), log_m, count, inverse, engine._stream())
+    torch.cuda.synchronize()
+    whole = count // distinct * distinct
+    blocks = out[:whole].reshape(-1, distinct, m, 18)
+    assert (blocks == blocks[0]).all() and (out[whole:] == blocks[0][:count - whole]).all()
+    assert np.array_equal(normalized(engine, out[:distinct]), O.g1_fft(x, inverse=bool(inverse)))
+    engine.call("g1p_fft_n", engine._ptr(src), engine._ptr(src), log_m, count, inverse, engine._stream())
+    assert torch.equal(src, out)  # in place
