@@ -1048,15 +1048,6 @@ int setup2xext(fk20_ctx *ctx, g1p_t *xext_fft, const g1p_t *setup, unsigned n, c
     return 0;
 }
 
-// Transforms that keep the radix-2 stages: those whose stages are no deeper in
-// products than their plan, two points, and four forward.  What a plan adds to
-// them, its task queue and normalised outputs (an inversion a point), is most of
-// such a call, and the bandwidth of a large one.  B200, two points forward: one
-// transform 62 us by stages and 118 by plan, 100,000 229 and 10,385; inverse, one
-// 1.12 and 1.15 ms.  Four points forward, one: 0.63 and 0.69 ms.  Four inverse, with
-// stages two products deep, 1.70 and 1.20 ms: the plan.
-bool by_stages(PlanKind kind, int log_m) { return log_m == 1 || (log_m == 2 && kind == PLAN_DFT); }
-
 int run_stages(fk20_ctx *ctx, PlanKind kind, g1p_t *out, const g1p_t *in, int log_m, unsigned rows, int raw,
                cudaStream_t st) {
     CKR(ctx->D2.reserve(tile_bytes((int)((rows + 31) / 32), 1 << log_m)));
@@ -1070,7 +1061,7 @@ int run_stages(fk20_ctx *ctx, PlanKind kind, g1p_t *out, const g1p_t *in, int lo
 // paid the depth of a plan, 0.7 to 1.7 ms, for each: 30,000 transforms of 8 points
 // 50.9 ms.)
 int run_points(fk20_ctx *ctx, PlanKind kind, g1p_t *out, const g1p_t *in, int log_m, unsigned rows, cudaStream_t st) {
-    if (by_stages(kind, log_m)) return run_stages(ctx, kind, out, in, log_m, rows, 1, st);
+    if (kind != PLAN_PROJ_HALF && g1_by_stages(log_m, kind == PLAN_IDFT)) return run_stages(ctx, kind, out, in, log_m, rows, 1, st);
     const size_t m = (size_t)1 << log_m;
     const unsigned pass = PASS_ROWS << (MAX_LOG_M - log_m);
     const int two = kind == PLAN_PROJ_HALF;

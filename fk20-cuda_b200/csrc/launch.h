@@ -142,6 +142,14 @@ void launch_ref_to_tile(uint4 *D, const uint64_t *src, int rows, int G, int log_
                         cudaStream_t st);
 void launch_tile_to_ref(uint64_t *dst, const TileView &v, const size_t *row_off, int rows, int log_m, int bitrev_out,
                         cudaStream_t st);
+// Transforms that keep the radix-2 stages, and points as these leave them: those whose stages are no deeper in
+// products than their plan, two points, and four forward.  What a plan adds to
+// them, its task queue and normalised outputs (an inversion a point), is most of
+// such a call, and the bandwidth of a large one.  B200, two points forward: one
+// transform 62 us by stages and 118 by plan, 100,000 229 and 10,385; inverse, one
+// 1.12 and 1.15 ms.  Four points forward, one: 0.63 and 0.69 ms.  Four inverse, with
+// stages two products deep, 1.70 and 1.20 ms: the plan.
+inline bool g1_by_stages(int log_m, int inverse) { return log_m == 1 || (log_m == 2 && !inverse); }
 // `count` radix-2 transforms, natural order in and out (out may be in), through the tiles D[(count + 31) / 32][m]
 cudaError_t launch_g1_transform(uint64_t *out, const uint64_t *in, uint4 *D, int log_m, int count, int inverse, int raw,
                                 cudaStream_t st);

@@ -79,19 +79,9 @@ extern "C" int g1p_fft_noalloc(g1p_t *output, const g1p_t *input, unsigned log_m
     uint4 *D = nullptr;
     rc = noalloc_tiles(&D);
     if (rc) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
-    const int G = (int)((count + 31) / 32);
-    const int L = (int)log_m;
-    if (!inverse) {  // bit-reversed load, forward DIT stages -> natural order
-        launch_ref_to_tile(D, (const uint64_t *)input, (int)count, G, L, 1, 0, st);
-        for (int s = 0; s < L; s++) launch_g1_stage(D, G, L, s, 1, st);
-        launch_tile_to_ref((uint64_t *)output, TileView{D, nullptr, {}, 0}, nullptr, (int)count, L, 0, st);
-    } else {  // natural load, inverse DIF stages -> bit-reversed, times 1/m
-        launch_ref_to_tile(D, (const uint64_t *)input, (int)count, G, L, 0, 0, st);
-        for (int s = 0; s < L; s++) launch_g1_stage(D, G, L, s, 0, st);
-        launch_g1_scale(D, G, L, 512 + L, st);
-        launch_tile_to_ref((uint64_t *)output, TileView{D, nullptr, {}, 0}, nullptr, (int)count, L, 1, st);
-    }
-    const cudaError_t e = cudaGetLastError();
+    // the same words as g1p_fft_n's; normalising the points of a two-point transform
+    // too would make it 104 us instead of 58 (B200)
+    const cudaError_t e = launch_g1_transform((uint64_t *)output, (const uint64_t *)input, D, (int)log_m, (int)count,
+                                              inverse, g1_by_stages((int)log_m, inverse), (cudaStream_t)stream);
     return e == cudaSuccess ? 0 : (int)e;
 }

@@ -74,3 +74,18 @@ def test_short_transforms_by_stages_and_in_passes(engine, log_m, count, inverse)
     assert np.array_equal(normalized(engine, out[:distinct]), O.g1_fft(x, inverse=bool(inverse)))
     engine.call("g1p_fft_n", engine._ptr(src), engine._ptr(src), log_m, count, inverse, engine._stream())
     assert torch.equal(src, out)  # in place
+
+
+@pytest.mark.parametrize("log_m,inverse", [(1, 0), (1, 1), (2, 0), (2, 1), (3, 0)])
+def test_no_allocation_entry_gives_the_same_words(engine, log_m, inverse):
+    """Also where the points of both are not normalised."""
+    import torch
+    m = 1 << log_m
+    src = engine.to_device(points(50 + log_m, 37 * m).reshape(37, m, 18))
+    a, b = engine.empty(src.shape), engine.empty(src.shape)
+    for call, out in (("g1p_fft_n", a), ("g1p_fft_noalloc", b)):
+        engine.call(call, engine._ptr(out), engine._ptr(src), log_m, 37, inverse, engine._stream())
+    torch.cuda.synchronize()
+    assert torch.equal(a, b)
+    raw = log_m == 1 or (log_m == 2 and not inverse)
+    assert raw == bool((a.reshape(-1, 18)[:, 12] != 1).any())
