@@ -475,6 +475,7 @@ struct fk20_ctx {
     int fft_blocks_per_sm = 0;  // persistent FFT grid: blocks per SM (0 = as many as fit)
     int fused_occupancy = 1;    // blocks of the cohorts' persistent FFT kernel that fit on one SM
     int proj_occupancy = 1;     // blocks of the persistent projection kernel that fit on one SM
+    int commit_warps = 4;       // warps of the commitments' first pass that the device holds
     unsigned wait_limit = FUSED_SPIN_LIMIT;  // polls before a persistent wait gives up
     unsigned unpublished = 0xffffffffu;      // test hook: a task whose completion is not published
     std::mutex mu;
@@ -690,7 +691,7 @@ int msm_launch(fk20_ctx *ctx, Tables *T, uint4 *D, const uint4 *S, int G, int ro
     a.warps = (unsigned)G << T->log_m;
     const Work w = msm_products(T->W, T->log_m, times_m != 0) * ((double)rows * (1 << T->log_m));
     ctx->prof.begin(FK20_K_MSM, w.alg, w.exe, st);
-    launch_msm(a, ctx->msm_threads, st);
+    launch_msm(a, ctx->msm_threads, ctx->sms, st);
     ctx->prof.end(st);
     CKL();
     return 0;
@@ -881,7 +882,7 @@ int run_pass(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, const fr_t *
     a.test_check = ctx->test_check;
     a.warps = warps;
     ctx->prof.begin(FK20_K_MSM, prod.alg, prod.exe, st);
-    launch_msm(a, ctx->msm_threads, st);
+    launch_msm(a, ctx->msm_threads, ctx->sms, st);
     ctx->prof.end(st);
     CKL();
     if (full) {
@@ -1134,6 +1135,7 @@ int fk20_ctx_create(fk20_ctx **out, int device, int window) {
         DeviceGuard dg(device);
         c->fused_occupancy = std::max(1, fused_blocks_per_sm());
         c->proj_occupancy = std::max(1, proj_blocks_per_sm());
+        c->commit_warps = c->sms * 4 * std::max(1, commit_blocks_per_sm());
         const int rc = c->ws.init();
         if (rc) {
             delete c;
@@ -1637,12 +1639,12 @@ int fk20_ctx_commit(fk20_ctx *ctx, g1p_t *commitment, const fr_t *polynomial, un
     std::lock_guard<std::mutex> lk(ctx->mu);
     DeviceGuard dg(ctx->device);
     if (!ctx->commit.n || (int)n > ctx->commit.n) return FK20_ENOSETUP;
-    const CommitCut cut = commit_cut((int)rows, (int)n, ctx->commit.W);
+    const CommitCut cut = commit_cut((int)rows, (int)n, ctx->commit.W, ctx->commit_warps);
     CKR(ctx->commit.part.reserve(tile_bytes(1, cut.tiles())));
     const double terms = (double)rows * n * ctx->commit.W, sums = (double)rows * (cut.full ? cut.P : cut.Pr) * ADD_P;
     ctx->prof.begin(FK20_K_MSM, terms * MADD_A + sums, terms * MADD_X + sums, S_(stream));
     launch_commit((uint64_t *)commitment, (uint4 *)ctx->commit.part.p, (const uint64_t *)polynomial,
-                  (const uint4 *)ctx->commit.table.p, (int)rows, (int)n, ctx->commit.W, ctx->commit.cb, S_(stream));
+                  (const uint4 *)ctx->commit.table.p, (int)rows, (int)n, ctx->commit.W, ctx->commit.cb, cut, S_(stream));
     ctx->prof.end(S_(stream));
     CKL();
     return 0;
@@ -1827,7 +1829,8 @@ int fk20_ctx_check_proof_multi(fk20_ctx *ctx, uint8_t *ok, const g1p_t *commitme
     const size_t poly_b = (size_t)count * COMMIT_CHUNK * sizeof(fr_t), xl_b = (size_t)count * sizeof(fr_t),
                  pt_b = (size_t)count * sizeof(g1p_t);
     CKR(ctx->verify.reserve(poly_b + xl_b + 2 * pt_b));
-    CKR(ctx->commit.part.reserve(tile_bytes(1, commit_cut((int)count, (int)COMMIT_CHUNK, ctx->commit.W).tiles())));
+    const CommitCut cut = commit_cut((int)count, (int)COMMIT_CHUNK, ctx->commit.W, ctx->commit_warps);
+    CKR(ctx->commit.part.reserve(tile_bytes(1, cut.tiles())));
     char *base = (char *)ctx->verify.p;
     uint64_t *poly = (uint64_t *)base, *xl = (uint64_t *)(base + poly_b);
     uint64_t *I = (uint64_t *)(base + poly_b + xl_b), *A = I + 18 * (size_t)count;
@@ -1835,7 +1838,7 @@ int fk20_ctx_check_proof_multi(fk20_ctx *ctx, uint8_t *ok, const g1p_t *commitme
     // I(X) over the coset and x^l; [I(s)]G1 with the commitment tables
     launch_interp(poly, xl, (const uint64_t *)x, (const uint64_t *)ys, log_l, count, st);
     launch_commit(I, (uint4 *)ctx->commit.part.p, poly, (const uint4 *)ctx->commit.table.p, (int)count,
-                  (int)COMMIT_CHUNK, ctx->commit.W, ctx->commit.cb, st);
+                  (int)COMMIT_CHUNK, ctx->commit.W, ctx->commit.cb, cut, st);
     // e(C - [I(s)] + [x^l] proof, G2) == e(proof, [s^l]G2)
     launch_verify_points(A, (const uint64_t *)commitment, I, (const uint64_t *)proof, xl, count, st);
     launch_pairing(1, nullptr, ok, A, (const uint64_t *)setup_g2, (const uint64_t *)proof,
@@ -2318,7 +2321,7 @@ int cohort_msm(fk20_server *s, const std::vector<int> &fresh) {
     a.times_m = 0;
     a.test_check = ctx->test_check;
     a.warps = warps;
-    launch_msm(a, ctx->msm_threads, st);
+    launch_msm(a, ctx->msm_threads, ctx->sms, st);
     CKL();
     CK(cudaEventRecord(s->msm_done, st));
     CK(cudaLaunchHostFunc(st, pack_done_cb, s));

@@ -355,22 +355,20 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_commit_reduce(uint64_t *__re
     if (threadIdx.x == 0) g1p_to_ref(out + 18 * (size_t)row, acc);
 }
 
+int commit_blocks_per_sm() {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_commit_partial, 128, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
 // Pass 1 as one wave of the warps the device holds at once, every lane group
 // with a run of the same length (at least 4 digits): the last group's rows,
 // packed, take a share of the warps like their share of the lanes.  B200, 48
 // commitments of 4096 at window 10: 2.47 ms; with whole bases and whole groups 2.96.
-CommitCut commit_cut(int rows, int n, int W) {
-    static int resident = 0;  // warps of k_commit_partial resident on the device
-    if (!resident) {
-        int dev = 0, sms = 1, bps = 1;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_commit_partial, 128, 0) != cudaSuccess || bps < 1) {
-            cudaGetLastError();
-            bps = 1;
-        }
-        resident = sms * bps * 4;
-    }
+CommitCut commit_cut(int rows, int n, int W, int resident) {
     CommitCut c{};
     const int rest = rows & 31, lanes = rest ? 32 >> msm_row_lanes(rest) : 32;
     const double groups = (rows >> 5) + (rest ? 1.0 / lanes : 0.0);
@@ -383,8 +381,7 @@ CommitCut commit_cut(int rows, int n, int W) {
 }
 
 void launch_commit(uint64_t *out, uint4 *part, const uint64_t *poly, const uint4 *table, int rows, int n, int W,
-                   int cb, cudaStream_t st) {
-    const CommitCut cut = commit_cut(rows, n, W);
+                   int cb, const CommitCut &cut, cudaStream_t st) {
     k_commit_partial<<<blocks_for((size_t)cut.tiles(), 4), 128, 0, st>>>(part, poly, table, rows, n, W, cb, cut);
     k_commit_reduce<<<(unsigned)rows, REDUCE_THREADS, 0, st>>>(out, part, cut);
 }
@@ -399,7 +396,7 @@ void launch_commit(uint64_t *out, uint4 *part, const uint64_t *poly, const uint4
 // 1.33, 160 of 4096 15.1 -> 13.5; at 512 rows of 4096 (4.6 waves) splitting
 // costs 1 %, 40.7 -> 41.1, hence the line at 4 waves.  48 commitments of 4096:
 // 10.5 -> 3.0 ms, most of it the partial sums, which one thread per row added.
-void launch_msm(const MsmArgs &in, int threads, cudaStream_t st) {
+void launch_msm(const MsmArgs &in, int threads, int sms, cudaStream_t st) {
     if (threads != 64 && threads != 128 && threads != 256) threads = 128;
     if (threads > MSM_MAX_THREADS) threads = MSM_MAX_THREADS;
     MsmArgs a = in;
@@ -424,7 +421,7 @@ void launch_msm(const MsmArgs &in, int threads, cudaStream_t st) {
             a.seg[a.nseg++] = s;
         }
     }
-    const unsigned resident = 148 * 12;
+    const unsigned resident = (unsigned)sms * 12;
     int rl_max = 0;
     for (int k = 0; k < a.nseg; k++) rl_max = std::max(rl_max, a.seg[k].rl);
     a.split = 1;

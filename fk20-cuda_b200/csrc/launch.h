@@ -115,7 +115,8 @@ inline int msm_row_lanes(int rows) {
 }
 
 // kernels_msm.cu
-void launch_msm(const MsmArgs &a, int threads, cudaStream_t st);  // threads: 64, 128 or 256
+// threads: 64, 128 or 256; sms: the device's SMs
+void launch_msm(const MsmArgs &a, int threads, int sms, cudaStream_t st);
 // checked build (check.cuh): take and clear the first failing check site of the
 // MSM / persistent-FFT translation units (0: none)
 int check_take_msm();
@@ -129,9 +130,10 @@ struct CommitCut {
     int full, P, Pr, rl;
     FK_HD int tiles() const { return full * P + Pr; }
 };
-CommitCut commit_cut(int rows, int n, int W);
+int commit_blocks_per_sm();  // blocks of pass 1 resident on an SM
+CommitCut commit_cut(int rows, int n, int W, int resident);  // resident: warps of pass 1 on the device
 void launch_commit(uint64_t *out, uint4 *part, const uint64_t *poly, const uint4 *table, int rows, int n, int W,
-                   int cb, cudaStream_t st);
+                   int cb, const CommitCut &cut, cudaStream_t st);
 
 // kernels_fft.cu
 void launch_g1_stage(uint4 *D, int G, int log_m, int s, int kind, cudaStream_t st);
