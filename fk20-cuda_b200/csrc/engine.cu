@@ -1639,7 +1639,7 @@ int fk20_ctx_commit(fk20_ctx *ctx, g1p_t *commitment, const fr_t *polynomial, un
     std::lock_guard<std::mutex> lk(ctx->mu);
     DeviceGuard dg(ctx->device);
     if (!ctx->commit.n || (int)n > ctx->commit.n) return FK20_ENOSETUP;
-    const CommitCut cut = commit_cut((int)rows, (int)n, ctx->commit.W, ctx->commit_warps);
+    const CommitCut cut = commit_cut((int)rows, (int)n, ctx->commit.W, ctx->commit_warps, ctx->sms);
     CKR(ctx->commit.part.reserve(tile_bytes(1, cut.tiles())));
     const double terms = (double)rows * n * ctx->commit.W, sums = (double)rows * (cut.full ? cut.P : cut.Pr) * ADD_P;
     ctx->prof.begin(FK20_K_MSM, terms * MADD_A + sums, terms * MADD_X + sums, S_(stream));
@@ -1829,7 +1829,7 @@ int fk20_ctx_check_proof_multi(fk20_ctx *ctx, uint8_t *ok, const g1p_t *commitme
     const size_t poly_b = (size_t)count * COMMIT_CHUNK * sizeof(fr_t), xl_b = (size_t)count * sizeof(fr_t),
                  pt_b = (size_t)count * sizeof(g1p_t);
     CKR(ctx->verify.reserve(poly_b + xl_b + 2 * pt_b));
-    const CommitCut cut = commit_cut((int)count, (int)COMMIT_CHUNK, ctx->commit.W, ctx->commit_warps);
+    const CommitCut cut = commit_cut((int)count, (int)COMMIT_CHUNK, ctx->commit.W, ctx->commit_warps, ctx->sms);
     CKR(ctx->commit.part.reserve(tile_bytes(1, cut.tiles())));
     char *base = (char *)ctx->verify.p;
     uint64_t *poly = (uint64_t *)base, *xl = (uint64_t *)(base + poly_b);

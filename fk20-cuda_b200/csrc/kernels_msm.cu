@@ -21,6 +21,7 @@
 #define FK_FP_MUL_OUTLINE 1
 #endif
 #include <algorithm>
+#include <cmath>
 
 #include "../../include/fk20_b200.h"
 #include "check.cuh"
@@ -355,6 +356,25 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_commit_reduce(uint64_t *__re
     if (threadIdx.x == 0) g1p_to_ref(out + 18 * (size_t)row, acc);
 }
 
+// The same for many rows: 2^ll lanes a row, rows on the low lane bits.
+__global__ void __launch_bounds__(REDUCE_THREADS) k_commit_reduce_rows(uint64_t *__restrict__ out, const uint4 *__restrict__ part,
+                                                                       int rows, const CommitCut cut, int ll) {
+    const int lane = threadIdx.x & 31, per = 32 >> ll;
+    const unsigned warp = blockIdx.x * (REDUCE_THREADS / 32) + (threadIdx.x >> 5);
+    const int row = (int)(warp * (unsigned)per) + (lane & (per - 1)), sub = lane >> (5 - ll), g = row >> 5;
+    const int P = row >= rows ? 0 : g < cut.full ? cut.P : cut.Pr;
+    G1P acc, q;
+    g1_set_inf(acc);
+    if (sub < P) tile_load(acc, part + tile_index(0, 0, g * cut.P + sub), row & 31);
+    for (int c = sub + (1 << ll); c < P; c += 1 << ll) {
+        tile_load(q, part + tile_index(0, 0, g * cut.P + c), row & 31);
+        g1_add(acc, acc, q);
+    }
+    __syncwarp();
+    g1_sum_lanes(acc, per);
+    if (P > 0 && sub == 0) g1p_to_ref(out + 18 * (size_t)row, acc);
+}
+
 int commit_blocks_per_sm() {
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_commit_partial, 128, 0) != cudaSuccess) {
@@ -368,22 +388,49 @@ int commit_blocks_per_sm() {
 // with a run of the same length (at least 4 digits): the last group's rows,
 // packed, take a share of the warps like their share of the lanes.  B200, 48
 // commitments of 4096 at window 10: 2.47 ms; with whole bases and whole groups 2.96.
-CommitCut commit_cut(int rows, int n, int W, int resident) {
+// Where a group's share is few warps, rounding it down would leave much of the chip
+// idle: several waves, by the least count of waves times digits of a run (a run's
+// own sum and conversion taken as 4).
+CommitCut commit_cut(int rows, int n, int W, int resident, int sms) {
     CommitCut c{};
+    c.lanes = sms * 256;
     const int rest = rows & 31, lanes = rest ? 32 >> msm_row_lanes(rest) : 32;
     const double groups = (rows >> 5) + (rest ? 1.0 / lanes : 0.0);
     c.full = rows >> 5;
     c.rl = rest ? msm_row_lanes(rest) : 5;
     const int most = std::max(1, n * W / 4);
-    c.P = c.full ? std::max(1, std::min(most, (int)(resident / groups))) : 0;
-    c.Pr = rest ? std::max(1, std::min(most / lanes, (int)(resident / groups / lanes))) : 0;
+    const double share = resident / groups;
+    // the last group's runs are no longer than the others'
+    const auto part = [&](int p) { return rest ? (p + lanes - 1) / lanes : 0; };
+    const auto warps = [&](int p) { return (double)c.full * p + part(p); };
+    int P = std::max(1, (int)std::min<double>(most, share));
+    while (P > 1 && warps(P) > resident) P--;
+    if (share < 16) {
+        double least = 0;
+        for (int p = 1; p <= std::min(most, std::max(8, (int)(4 * share))); p++) {
+            const double cost = std::ceil(warps(p) / resident) * ((double)n * W / p + 4);
+            if (p == 1 || cost < least) least = cost, P = p;
+        }
+    }
+    c.P = c.full ? P : 0;
+    c.Pr = part(P);
     return c;
 }
 
 void launch_commit(uint64_t *out, uint4 *part, const uint64_t *poly, const uint4 *table, int rows, int n, int W,
                    int cb, const CommitCut &cut, cudaStream_t st) {
     k_commit_partial<<<blocks_for((size_t)cut.tiles(), 4), 128, 0, st>>>(part, poly, table, rows, n, W, cb, cut);
-    k_commit_reduce<<<(unsigned)rows, REDUCE_THREADS, 0, st>>>(out, part, cut);
+    // as many lanes a row as two warps a scheduler give, at most one a partial sum: a
+    // block, or a part of a warp.  A block for each of many rows would add mostly
+    // points at infinity: 10,000 commitments of 32 7.6 ms with blocks, 3.35 with lanes.
+    const int lanes = cut.lanes / rows;
+    if (lanes >= REDUCE_THREADS) {
+        k_commit_reduce<<<(unsigned)rows, REDUCE_THREADS, 0, st>>>(out, part, cut);
+        return;
+    }
+    int ll = 0;
+    while (ll < 5 && (2 << ll) <= lanes && (2 << ll) <= std::max(cut.P, cut.Pr)) ll++;
+    k_commit_reduce_rows<<<blocks_for((size_t)rows << ll, REDUCE_THREADS), REDUCE_THREADS, 0, st>>>(out, part, rows, cut, ll);
 }
 
 // How a launch is cut.  A segment's last rows % 32 rows form one or two segments

@@ -128,10 +128,11 @@ int check_take_proj();
 constexpr int COMMIT_CHUNK = 32;
 struct CommitCut {
     int full, P, Pr, rl;
+    int lanes;  // of the device with two warps on each scheduler: for the sums of the partial sums
     FK_HD int tiles() const { return full * P + Pr; }
 };
 int commit_blocks_per_sm();  // blocks of pass 1 resident on an SM
-CommitCut commit_cut(int rows, int n, int W, int resident);  // resident: warps of pass 1 on the device
+CommitCut commit_cut(int rows, int n, int W, int resident, int sms);  // resident: warps of pass 1 on the device
 void launch_commit(uint64_t *out, uint4 *part, const uint64_t *poly, const uint4 *table, int rows, int n, int W,
                    int cb, const CommitCut &cut, cudaStream_t st);
 

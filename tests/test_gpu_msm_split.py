@@ -51,3 +51,24 @@ def test_commitments_of_every_packing(engine, ctx, rows, n):
         ks.append(acc)
     exp = O.g1_op("mul", np.repeat(O.g1_generator().reshape(1, 18), rows, 0), O.ints_to_array(ks, 4))
     assert np.array_equal(O.g1_normalize(engine.to_host(out)), O.g1_normalize(exp))
+
+
+@pytest.mark.parametrize("rows,n", [(296, 32), (297, 32), (1183, 64), (2100, 32), (9000, 32), (18000, 64), (40001, 32)])
+def test_many_commitments(engine, ctx, rows, n):
+    """The partial sums of a row added by a block, or by 32 down to one lanes;
+    several waves of the first pass.  Rows repeat 61 polynomials."""
+    tau = O.limbs_to_int(fk20_setup_data(1024)[0])
+    poly = O.seeded_fr(77, 61 * n).reshape(61, n, 4)
+    ks = []
+    for p in poly:
+        acc = 0
+        for v in reversed(p):
+            acc = (acc * tau + O.limbs_to_int(v)) % O.R
+        ks.append(acc)
+    exp = O.g1_normalize(O.g1_op("mul", np.repeat(O.g1_generator().reshape(1, 18), 61, 0), O.ints_to_array(ks, 4)))
+    out, aff = engine.empty((rows, 18)), engine.empty((rows, 18))
+    d = engine.to_device(poly).repeat((rows + 60) // 61, 1, 1)[:rows].contiguous()
+    ctx.commit(out, d, rows, n)
+    engine.call("g1p_op_n", engine.G1_OPS["normalize"], engine._ptr(aff), engine._ptr(out), None, rows, engine._stream())
+    got = engine.to_host(aff)
+    assert np.array_equal(got, np.tile(exp, ((rows + 60) // 61, 1))[:rows])
