@@ -100,6 +100,7 @@ namespace {
 
 std::mutex g_dev_mu;
 bool g_dev_ready[64];
+int g_dev_sms[64];  // set before g_dev_ready
 
 int ensure_device(int dev) {
     if (dev < 0 || dev >= 64) return FK20_ENODEV;
@@ -119,14 +120,17 @@ int ensure_device(int dev) {
     if (err == cudaSuccess) err = upload_consts_misc();
     if (cur != dev) cudaSetDevice(cur);
     if (err != cudaSuccess) return (int)err;
+    g_dev_sms[dev] = prop.multiProcessorCount;
     g_dev_ready[dev] = true;
     return 0;
 }
 
-int current_device_ready() {
+int current_device_ready(int *sms = nullptr) {
     int dev;
     if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return FK20_ENODEV; }
-    return ensure_device(dev);
+    const int rc = ensure_device(dev);
+    if (!rc && sms) *sms = g_dev_sms[dev];
+    return rc;
 }
 
 }  // namespace
@@ -1797,8 +1801,9 @@ int fr_fft_n(fr_t *output, const fr_t *input, unsigned log_m, unsigned count, in
     if (log_m < 1 || log_m > 9) return FK20_EINVAL;
     CKR(check_call(output, input, count ? 1 : 0));
     if (count == 0) return FK20_EINVAL;
-    CKR(current_device_ready());
-    launch_fr_fft_ref((uint64_t *)output, (const uint64_t *)input, (int)log_m, count, inverse, S_(stream));
+    int sms = 0;
+    CKR(current_device_ready(&sms));
+    launch_fr_fft_ref((uint64_t *)output, (const uint64_t *)input, (int)log_m, count, inverse, sms, S_(stream));
     CKL();
     return 0;
 }

@@ -19,8 +19,9 @@ cudaError_t upload_consts_fr() { return upload_module_consts(); }
 //
 // The multiply pipe's share at m = 512 is 1,793 products a transform (0.13 ms
 // for 4,000); one stage at a time through sm[m][8] took 0.35 ms, its eight-word
-// stride an eight-way bank conflict on every access; this takes 0.21 ms (128-thread blocks at 134
-// registers 0.22; for 4,000 transforms of 128 values 0.055 against 0.072).
+// stride an eight-way bank conflict on every access; this takes 0.20 ms
+// (128-thread blocks at 134 registers 0.22; for 4,000 transforms of 128 values
+// 0.055 against 0.072).
 //
 // Load: fn(natural index) -> value, store: fn(index, value).
 constexpr int FR_THREADS = 64;  // threads of a block: 64 / (m / 8) transforms
@@ -185,13 +186,7 @@ __global__ void __launch_bounds__(FR_THREADS, 8) k_fr_fft_ref(uint64_t *out, con
 
 // Few transforms: a butterfly a thread and a barrier a stage, grid (count),
 // block m / 2.  A call that leaves the chip idle costs its chain of products: one
-// a stage here, up to twelve a pass in registers above (a small call 18 us
-// against 35).  4,000 transforms of 512 values take 0.35 ms here (bank
-// conflicts of the eight-word stride) and 0.20 above.  So this serves what is
-// resident at once, 12 blocks of 16 KB to an SM, up to 1,024 values to an SM;
-// at 296 transforms of 512 the rates of the full chip would give 26 us here,
-// while 500 take 45 us above.
-constexpr unsigned FR_FEW_COUNT = 148 * 12, FR_FEW_VALUES = 148 * 1024;
+// a stage here, up to twelve a pass in registers above.
 __global__ void __launch_bounds__(256) k_fr_fft_few(uint64_t *out, const uint64_t *in, int log_m, int inverse) {
     __shared__ uint32_t sm[512][8];
     const int m = 1 << log_m, tid = threadIdx.x;
@@ -243,7 +238,7 @@ __global__ void __launch_bounds__(256) k_fr_fft_few(uint64_t *out, const uint64_
     }
 }
 
-// transforms of 2 and 4 points, one thread each
+// many transforms of 2 and 4 values, one thread each
 __global__ void k_fr_fft_tiny(uint64_t *out, const uint64_t *in, int log_m, unsigned count, int inverse) {
     const unsigned tr = blockIdx.x * blockDim.x + threadIdx.x;
     if (tr >= count) return;
@@ -308,13 +303,24 @@ void launch_tc_fft(uint4 *S, size_t stride, const uint64_t *poly, const size_t *
     const unsigned per = FR_THREADS >> (log_m - 3);
     k_tc_fft<<<blocks_for((size_t)rows * L_COLS, per), FR_THREADS, 0, st>>>(S, stride, poly, row_off, n, log_m, rows);
 }
-void launch_fr_fft_ref(uint64_t *out, const uint64_t *in, int log_m, unsigned count, int inverse, cudaStream_t st) {
-    if (log_m < 3) {
-        k_fr_fft_tiny<<<blocks_for(count, 64), 64, 0, st>>>(out, in, log_m, count, inverse);
+// Values an SM up to which k_fr_fft_few is the faster one, for forward and inverse
+// transforms (of which k_fr_fft_ref pays more for the factor 1/m) of 2^1 .. 2^9
+// values.  Its time is that of one transform and then grows with every block that
+// an SM gets: the others' is flat up to about 2,000 values an SM.  B200, us, few and
+// other, at the line and at twice it: 2 values inverse 4.6 and 6.3, 6.3 and 6.2; 4:
+// 6.6 and 6.8, 10.5 and 7.2; 8: 10.5 and 10.6, 14.6 and 10.6; 16: 14.6 and 14.7, 23.0
+// and 15.6; 32: 16.9 and 17.1, 28.0 and 18.9; 64: 22.9 and 22.9, 37.5 and 26.0; 128:
+// 31.1 and 31.0, 58.0 and 39.0; 256: 34.0 and 35.2, 62.0 and 45.5; 512: 29.0 and 33.2,
+// 47.6 and 40.9.
+constexpr unsigned short FR_FEW[2][MAX_LOG_M + 1] = {{0, 8, 80, 176, 400, 672, 944, 1472, 1536, 1024},
+                                                     {0, 8, 64, 176, 400, 816, 1312, 1648, 1600, 1536}};
+void launch_fr_fft_ref(uint64_t *out, const uint64_t *in, int log_m, unsigned count, int inverse, int sms, cudaStream_t st) {
+    if (((size_t)count << log_m) <= (size_t)sms * FR_FEW[inverse != 0][log_m]) {
+        k_fr_fft_few<<<count, 1u << (log_m - 1), 0, st>>>(out, in, log_m, inverse);
         return;
     }
-    if (count <= FR_FEW_COUNT && ((size_t)count << log_m) <= FR_FEW_VALUES) {
-        k_fr_fft_few<<<count, 1u << (log_m - 1), 0, st>>>(out, in, log_m, inverse);
+    if (log_m < 3) {
+        k_fr_fft_tiny<<<blocks_for(count, 64), 64, 0, st>>>(out, in, log_m, count, inverse);
         return;
     }
     const unsigned per = FR_THREADS >> (log_m - 3);

@@ -36,3 +36,21 @@ def test_fr_fft_around_the_line(engine, log_m, past):
         out = engine.empty(x.shape)
         engine.call("fr_fft_n", engine._ptr(out), engine._ptr(d), log_m, count, inverse, engine._stream())
         assert np.array_equal(engine.to_host(out), O.fr_fft(x, inverse=bool(inverse)))
+
+
+# values an SM that each size leaves to the kernel for few transforms, forward and inverse
+LINES = [[8, 80, 176, 400, 672, 944, 1472, 1536, 1024], [8, 64, 176, 400, 816, 1312, 1648, 1600, 1536]]
+
+
+@pytest.mark.parametrize("log_m", range(1, 10))
+@pytest.mark.parametrize("inverse", [0, 1])
+def test_fr_fft_on_both_sides_of_its_line(engine, log_m, inverse):
+    import torch
+    m = 1 << log_m
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for count in (sms * LINES[inverse][log_m - 1] // m + k for k in (0, 1)):
+        x = O.seeded_fr(80 + log_m, count * m).reshape(count, m, 4)
+        d = engine.to_device(x)
+        exp = O.fr_fft(x, inverse=bool(inverse))
+        engine.call("fr_fft_n", engine._ptr(d), engine._ptr(d), log_m, count, inverse, engine._stream())
+        assert np.array_equal(engine.to_host(d), exp)
