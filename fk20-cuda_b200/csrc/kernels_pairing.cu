@@ -836,13 +836,15 @@ __global__ void __launch_bounds__(64) k_g2_op(int op, uint64_t *out, const uint6
     g2_store(out + 36 * i, xr, yr, ir);
 }
 
-// Checks one warp each up to here, one thread each beyond.  B200: the warp kernel
-// 2.8 ms to 300 checks, then 409 k checks/s (23.8 ms at 9,472); the thread kernel
-// 26 ms to 10^4 checks, 37.6 ms at 37,888 (1.0 M/s).
-constexpr size_t PAIRING_WARP_MAX = 10240;
+// One warp each up to here, one thread each beyond: pairings (op 0) and checks (op
+// 1).  B200: the warp kernel 2.8 ms to 300 of either (it runs both Miller loops'
+// rounds for one pairing too), then 409 k/s: 20.8 ms at 8,288, 25.1 at 10,000; the
+// thread kernel 26.2 ms to 10^4 checks, 20.4 to 20.8 to 10^4 pairings, 37.5 and 29.5
+// at 37,888.
+constexpr size_t PAIRING_WARP_MAX[2] = {8192, 10240};
 void launch_pairing(int op, uint64_t *out, uint8_t *ok, const uint64_t *a, const uint64_t *b, const uint64_t *c,
                     const uint64_t *d, size_t count, cudaStream_t st, int bcast) {
-    if (count <= PAIRING_WARP_MAX)
+    if (count <= PAIRING_WARP_MAX[op])
         k_pairing<<<blocks_for(count, PV_WARPS), 32 * PV_WARPS, 0, st>>>(op, out, ok, a, b, c, d, count, bcast);
     else
         k_pairing_threads<<<blocks_for(count, 64), 64, 0, st>>>(op, out, ok, a, b, c, d, count, bcast);

@@ -83,3 +83,23 @@ def test_check_proof_multi_on_both_point_kernels(engine, count):
     c.close()
     # at x = 0 the interpolation keeps coefficient 0 only, as before: ys[0] alone moves the mean
     assert got == [rows[i][4] for i in idx]
+
+
+@pytest.mark.parametrize("count", [8192, 8193])
+def test_pairing_values_on_both_sides_of_their_line(engine, count):
+    """The same words from a warp and from a thread a pairing, infinities and a
+    point off the curve among the inputs."""
+    g1, g2 = O.g1_generator().reshape(1, 18), PP.g2_generator()
+    a = O.g1_op("mul", np.repeat(g1, 6, 0), O.ints_to_array([3, 5, 0, 7, O.R - 1, 11], 4))
+    b = g2_rows([PP.g2mul(k, g2) if k else None for k in (1, 9, 4, 0, 2, 6)])
+    b[5, :12] = b[1, 12:24]  # no point of the twist
+    idx = np.arange(count) % 6
+    few, many = engine.empty((6, 72)), engine.empty((count, 72))
+    d = [engine.to_device(np.ascontiguousarray(v)) for v in (a, b, a[idx], b[idx])]
+    engine.call("fk20_pairing_n", engine._ptr(few), engine._ptr(d[0]), engine._ptr(d[1]), 6, engine._stream())
+    engine.call("fk20_pairing_n", engine._ptr(many), engine._ptr(d[2]), engine._ptr(d[3]), count, engine._stream())
+    ref = engine.to_host(few)
+    assert np.array_equal(engine.to_host(many), ref[idx])
+    one = np.zeros(72, np.uint64)
+    one[0] = 1
+    assert [bool(np.array_equal(v, one)) for v in ref] == [False, False, True, True, False, False]
