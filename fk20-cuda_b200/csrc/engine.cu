@@ -1071,17 +1071,26 @@ int run_points(fk20_ctx *ctx, PlanKind kind, g1p_t *out, const g1p_t *in, int lo
     const unsigned pass = PASS_ROWS << (MAX_LOG_M - log_m);
     const int two = kind == PLAN_PROJ_HALF;
     Workspace &ws = ctx->pts;
-    CKR(ws.init());
     DevPlan d;
-    CKR(device_plan(ctx->device, kind, log_m, &d));
+    CKR(plan_ready(kind, log_m));
     const int slots = host_plan(kind, log_m).plan.slots;
     const auto arena = [&](unsigned n) {
         const int G = (int)((n + 31) / 32);
         return two ? proj_arena(slots, n) : ProjArena{slots, G, G, 0};
     };
     const ProjArena most = arena(std::min(rows, pass));
-    CKR(ws.D.reserve(arena_bytes(most)));
-    CKR(ws.sync.reserve(SYNC_HDR + ready_bytes(most)));
+    int rc = ws.init();
+    if (!rc) rc = device_plan(ctx->device, kind, log_m, &d);
+    if (!rc) rc = ws.D.reserve(arena_bytes(most));
+    if (!rc) rc = ws.sync.reserve(SYNC_HDR + ready_bytes(most));
+    if (rc == FK20_ENOMEM) {
+        // no room for the arena (13.8 MB for 32 rows of 512 points): by stages, which take 2.4
+        if (!two) return run_stages(ctx, kind, out, in, log_m, rows, 0, st);
+        CKR(run_stages(ctx, PLAN_IDFT, out, in, log_m, rows, 0, st));
+        launch_hext2h_ref((uint64_t *)out, (int)rows, log_m, st);
+        return run_stages(ctx, PLAN_DFT, out, out, log_m, rows, 0, st);
+    }
+    if (rc) return rc;
     for (unsigned r0 = 0; r0 < rows; r0 += pass) {
         const unsigned n = std::min(rows - r0, pass);
         SegLayout lay;

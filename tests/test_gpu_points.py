@@ -89,3 +89,36 @@ def test_no_allocation_entry_gives_the_same_words(engine, log_m, inverse):
     assert torch.equal(a, b)
     raw = log_m == 1 or (log_m == 2 and not inverse)
     assert raw == bool((a.reshape(-1, 18)[:, 12] != 1).any())
+
+
+def test_transforms_without_room_for_their_arena(engine):
+    """The device allocations of the arena fail (injected): the transforms go by
+    stages and give the same words; only when those fail too do they refuse."""
+    import torch
+    dev, lib = torch.cuda.current_device(), engine.lib()
+    x = points(61, 40 * 512).reshape(40, 512, 18)
+    src = engine.to_device(x)
+    calls = [("g1p_fft", 512, 40, ()), ("g1p_ift", 512, 40, ()), ("fk20_hext_fft2h_fft", 512, 33, ()),
+             ("g1p_fft_n", 8, 700, (3, 0)), ("g1p_fft_n", 4, 700, (2, 1))]
+
+    def run(name, m, count, first):
+        out = engine.empty((count, m, 18))
+        args = first and (first[0], count, first[1]) or (count,)
+        engine.call(name, engine._ptr(out), engine._ptr(src), *args, engine._stream())
+        torch.cuda.synchronize()
+        return out
+
+    try:
+        for c in calls:
+            good = run(*c)
+            assert lib.fk20_default_release(dev) == 0
+            assert lib.fk20_test_fail_allocations(1) == 0
+            assert torch.equal(run(*c), good), c
+            assert lib.fk20_default_release(dev) == 0
+            assert lib.fk20_test_fail_allocations(2) == 0
+            with pytest.raises(engine.Fk20Error) as err:
+                run(*c)
+            assert err.value.code == engine.FK20_ENOMEM
+            assert torch.equal(run(*c), good), c
+    finally:
+        lib.fk20_test_fail_allocations(0)
