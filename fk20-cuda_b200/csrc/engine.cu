@@ -755,23 +755,42 @@ int segment_layout(fk20_ctx *ctx, const Seg *sg, int nseg, bool full, SegLayout 
     return 0;
 }
 
-// Rows of one segment that one pass takes: an arena holds 24 MB for every 32
+// Rows of one segment that one pass takes: an arena holds 20.8 MB for every 32
 // rows of 4096 coefficients, so longer batches run in passes through one
-// workspace.  1024 rows (780 MB) fill the chip 55 times over in the products.
+// workspace.  1024 rows (665 MB) fill the chip 93 times over in the products.
 constexpr unsigned PASS_ROWS = 1024;
 
-// device buffers of a segment call (a no-op once they are large enough)
-int reserve_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, bool full) {
-    SegLayout lay;
-    Seg part[MAX_SEGS];
+// true if the device has `need` bytes left, and a little more for the allocator's rounding
+bool device_has(size_t need) {
+    OutsideCapture outside;
+    size_t fr = 0, tot = 0;
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return fr >= need + ((size_t)64 << 20);
+}
+
+// Device buffers of a segment call (a no-op once they are large enough), and the
+// rows of a pass that they hold: PASS_ROWS, or where the device has no room for
+// that arena half of it and so on down to 16, whose arena is no larger than the
+// point and scalar tiles of one group of 32 rows.
+int reserve_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, bool full, unsigned *pass) {
+    Seg part[MAX_PROJ_SEGS];
     if (nseg < 1 || nseg > MAX_PROJ_SEGS) return FK20_EINVAL;
-    for (int k = 0; k < nseg; k++) part[k] = sg[k], part[k].rows = std::min(sg[k].rows, PASS_ROWS);
-    CKR(segment_layout(ctx, part, nseg, full, lay));
     CKR(ws.init());
-    if (!full) CKR(ws.S.reserve(lay.s_bytes));
-    CKR(ws.D.reserve(lay.d_bytes));
-    if (full) CKR(ws.sync.reserve(SYNC_HDR + lay.r_bytes));
-    return 0;
+    for (*pass = PASS_ROWS;; *pass /= 2) {
+        SegLayout lay;
+        for (int k = 0; k < nseg; k++) part[k] = sg[k], part[k].rows = std::min(sg[k].rows, *pass);
+        CKR(segment_layout(ctx, part, nseg, full, lay));
+        if (!full) {
+            CKR(ws.S.reserve(lay.s_bytes));
+            return ws.D.reserve(lay.d_bytes);
+        }
+        int rc = ws.D.reserve(lay.d_bytes);
+        if (!rc) rc = ws.sync.reserve(SYNC_HDR + lay.r_bytes);
+        if (rc != FK20_ENOMEM || *pass <= 16 || device_has(lay.d_bytes + lay.r_bytes)) return rc;
+    }
 }
 
 // Blocks per SM for `products` product tasks.  Two warps a scheduler share the
@@ -917,14 +936,15 @@ int run_pass(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, const fr_t *
     return 0;
 }
 
-// run_pass over at most PASS_ROWS rows of each segment at a time
+// run_pass over as many rows of each segment at a time as the workspace holds (at most PASS_ROWS)
 int run_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, const fr_t *polys, void *out, bool full,
                  cudaStream_t st, bool proofs = false, int fft_bps = 0) {
-    CKR(reserve_segments(ctx, ws, sg, nseg, full));
+    unsigned pass = 0;
+    CKR(reserve_segments(ctx, ws, sg, nseg, full, &pass));
     if (*ws.err_host) return launch_error(*ws.err_host);  // a previous persistent launch stopped: results invalid
     unsigned most = 0;
     for (int k = 0; k < nseg; k++) most = std::max(most, sg[k].rows);
-    for (unsigned r0 = 0; r0 < most; r0 += PASS_ROWS) {
+    for (unsigned r0 = 0; r0 < most; r0 += pass) {
         Seg part[MAX_PROJ_SEGS];
         int np = 0;
         const fr_t *in = polys;
@@ -932,7 +952,7 @@ int run_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, const fr
         for (int k = 0; k < nseg; k++) {
             if (r0 >= sg[k].rows) continue;
             Seg s = sg[k];
-            s.rows = std::min(s.rows - r0, PASS_ROWS);
+            s.rows = std::min(s.rows - r0, pass);
             const size_t m = (size_t)1 << s.log_m;
             // contiguous rows come as the only segment of a call
             if (s.poly_off) s.poly_off += r0;
@@ -1084,7 +1104,7 @@ int run_points(fk20_ctx *ctx, PlanKind kind, g1p_t *out, const g1p_t *in, int lo
     if (!rc) rc = ws.D.reserve(arena_bytes(most));
     if (!rc) rc = ws.sync.reserve(SYNC_HDR + ready_bytes(most));
     if (rc == FK20_ENOMEM) {
-        // no room for the arena (13.8 MB for 32 rows of 512 points): by stages, which take 2.4
+        // no room for the arena (14.3 MB for 32 rows of 512 points): by stages, which take 2.4
         if (!two) return run_stages(ctx, kind, out, in, log_m, rows, 0, st);
         CKR(run_stages(ctx, PLAN_IDFT, out, in, log_m, rows, 0, st));
         launch_hext2h_ref((uint64_t *)out, (int)rows, log_m, st);
@@ -1411,7 +1431,8 @@ namespace {
 // the batch's launch sequence (offsets already on the device) captured into plan->graph
 int capture_plan(fk20_plan *plan, g1p_t *h_fft, const fr_t *polys, const Seg *sg, int nseg) {
     fk20_ctx *ctx = plan->ctx;
-    CKR(reserve_segments(ctx, plan->ws, sg, nseg, true));
+    unsigned pass = 0;
+    CKR(reserve_segments(ctx, plan->ws, sg, nseg, true, &pass));
     const bool prof_on = ctx->prof.on;
     ctx->prof.on = false;  // timing events cannot be replayed
     CK(cudaStreamBeginCapture(plan->capture, cudaStreamCaptureModeThreadLocal));

@@ -112,3 +112,35 @@ def test_cancel_before_packing(engine, ctx1024):
             assert np.array_equal(engine.to_host(h)[0], outs[j]), j
     finally:
         srv.close()
+
+
+def test_batches_without_room_for_a_full_pass(engine):
+    """With less device memory left than the arena of 1024 rows takes (665 MB), a
+    batch runs in shorter passes; transforms of points go by stages."""
+    import torch
+    n, rows, m = 4096, 1100, 512
+    c = engine.Context(0, 8)
+    lib, dev = engine.lib(), torch.cuda.current_device()
+    hold = []
+    try:
+        c.load_xext_fft(n, engine.to_device(fk20_setup_data(n)[2]))
+        poly = engine.to_device(O.seeded_fr(91, 50 * n).reshape(50, n, 4)).repeat(22, 1, 1).contiguous()
+        small, h, g = engine.empty((50, m, 18)), engine.empty((rows, m, 18)), engine.empty((rows, m, 18))
+        ref = engine.empty((50, m, 18))
+        assert lib.fk20_default_release(dev) == 0
+        c.poly2h_fft(small, poly, 50, n)  # also sizes the kernels' local memory
+        engine.call("g1p_fft", engine._ptr(ref), engine._ptr(small), 50, engine._stream())
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        hold.append(torch.empty(free - (448 << 20), dtype=torch.uint8, device="cuda"))
+        assert torch.cuda.mem_get_info()[0] < 600 << 20
+        c.poly2h_fft(h, poly, rows, n)
+        engine.call("g1p_fft", engine._ptr(g), engine._ptr(h), rows, engine._stream())
+        assert c.status() == 0 and lib.fk20_default_status(dev) == 0
+        for k in range(0, rows, 50):
+            assert torch.equal(h[k:k + 50], small) and torch.equal(g[k:k + 50], ref)
+    finally:
+        hold.clear()
+        torch.cuda.empty_cache()
+        c.close()
