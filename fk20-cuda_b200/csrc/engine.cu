@@ -2205,9 +2205,8 @@ void server_main(fk20_server *s) {
             // in the pack keeps a multiple of 32 (a warp proves 32 rows of one
             // length; a partial group idles lanes): its youngest extra
             // requests go back to the head of the queue for the next pack.
-            const bool latency = s->queue.size() <= s->cfg.latency_rows;
+            const bool whole = s->queue.size() > s->cfg.latency_rows;
             const size_t cap = s->queue.size() > 2 * (size_t)s->cfg.max_rows ? s->cfg.burst_rows : s->cfg.max_rows;
-            const bool more = s->queue.size() > cap;
             // Admission by device memory: the packs in flight and this one stay
             // within the budget, and whatever this pack adds to its slot's
             // buffers must be free on the device now (less a reserve for the
@@ -2243,7 +2242,7 @@ void server_main(fk20_server *s) {
                 fs->reqs.push_back(r);
             }
             s->queue.erase(s->queue.begin(), s->queue.begin() + (long)q);
-            if (more) {
+            if (whole) {
                 unsigned keep[3];
                 for (int k = 0; k < 3; k++) keep[k] = cnt[k] >= 32 ? cnt[k] & ~31u : cnt[k];
                 std::vector<Req> kept, back;

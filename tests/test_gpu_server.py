@@ -155,3 +155,37 @@ def test_server_full_queue_refuses_with_eagain(engine, served_ctx):
         h = engine.empty((1, 512, 18))
         served_ctx.poly2h_fft(h, engine.to_device(polys[j].reshape(1, 4096, 4)), 1, 4096)
         assert np.array_equal(engine.to_host(h)[0], outs[j]), j
+
+
+@pytest.mark.parametrize("latency_rows,packs", [(8, 3), (64, 2)])
+def test_server_latency_rows_decides_whole_groups(engine, served_ctx, latency_rows, packs):
+    """40 requests wait while the one slot is busy: at most latency_rows, they make
+    one pack; beyond it a pack keeps whole groups of 32, and the other 8 make the
+    next.  A status call on the context holds the first pack back meanwhile."""
+    import threading
+    n, rows = 1024, 4000
+    poly = engine.to_device(O.seeded_fr(70, 100 * n).reshape(100, n, 4)).repeat(40, 1, 1)
+    h = engine.empty((rows, n // 8, 18))
+    served_ctx.poly2h_fft(h, poly, rows, n)  # sizes the workspace
+    assert served_ctx.status() == 0
+    polys = [O.seeded_fr(7100 + j, n) for j in range(41)]
+    outs = [np.zeros((n // 8, 18), np.uint64) for _ in polys]
+    srv = engine.Server(served_ctx, max_rows=64, slots=1, latency_rows=latency_rows)
+    try:
+        served_ctx.poly2h_fft(h, poly, rows, n)  # 160 ms of work
+        holder = threading.Thread(target=served_ctx.status)
+        holder.start()
+        time.sleep(0.01)
+        tickets = [srv.submit(polys[0], outs[0])]
+        time.sleep(0.02)
+        tickets += [srv.submit(p, o) for p, o in zip(polys[1:], outs[1:])]
+        assert holder.is_alive()  # all 40 wait
+        holder.join()
+        for t in tickets:
+            assert srv.wait(t, 60000) == 0
+        assert srv.stats()["packs"] == packs
+    finally:
+        srv.close()
+    one = engine.empty((41, n // 8, 18))
+    served_ctx.poly2h_fft(one, engine.to_device(np.stack(polys)), 41, n)
+    assert np.array_equal(engine.to_host(one), np.stack(outs))
