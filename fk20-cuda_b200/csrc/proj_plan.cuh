@@ -508,7 +508,9 @@ inline ProjPlan finish_plan(const ProjBuilder &g, int inputs, const std::vector<
     // ---- slots.  A task may write over a value all of whose readers are above
     // it in the dependency graph (or are the task itself): they have finished
     // when it runs.  Tasks of the last phase wait until every product of their
-    // group is done, so all readers of the first two phases are above them.
+    // group is done, so the products and all that is above one of them count too;
+    // a task of the first phase that feeds no product (a diagonal term's doublings)
+    // does not.
     ProjPlan P;
     std::vector<int> slot(N, -1), ver(N, 0), pos(NT, 0);
     std::vector<std::vector<int>> readers(N);
@@ -521,6 +523,11 @@ inline ProjPlan finish_plan(const ProjBuilder &g, int inputs, const std::vector<
     const auto under = [&](int i, int o) {  // task i runs after task o
         for (size_t k = 0; k < words; k++) above[i][k] |= above[o][k];
         above[i][(size_t)o / 64] |= 1ull << (o % 64);
+    };
+    std::vector<uint64_t> produced(words, 0);  // the products and the tasks above them (complete before the last phase)
+    const auto finished = [&](int r, int i) {  // reader r has finished when task i runs
+        const auto has = [&](const std::vector<uint64_t> &set) { return ((set[(size_t)r / 64] >> (r % 64)) & 1) != 0; };
+        return r == i || has(above[i]) || (phase[i] == 2 && has(produced));
     };
     struct Dead { int slot, ver; std::vector<int> readers; };
     std::vector<Dead> dead;
@@ -549,18 +556,15 @@ inline ProjPlan finish_plan(const ProjBuilder &g, int inputs, const std::vector<
             int pick = -1;
             for (int k = (int)dead.size() - 1; k >= 0 && pick < 0; k--) {
                 bool ok = true;
-                for (int r : dead[k].readers)
-                    ok &= r == i || (phase[i] == 2 && phase[r] < 2) || ((above[i][(size_t)r / 64] >> (r % 64)) & 1);
+                for (int r : dead[k].readers) ok &= finished(r, i);
                 if (ok) pick = k;
             }
             // or one whose only other reader is a task of an earlier level: this
             // task then waits for that reader's result as well (b2)
             for (int k = (int)dead.size() - 1; k >= 0 && pick < 0 && t.op != PROJ_OUT && o.b2 == PROJ_NONE; k--) {
                 int other = -1, n = 0;
-                for (int r : dead[k].readers) {
-                    const bool ok = r == i || (phase[i] == 2 && phase[r] < 2) || ((above[i][(size_t)r / 64] >> (r % 64)) & 1);
-                    if (!ok) other = r, n++;
-                }
+                for (int r : dead[k].readers)
+                    if (!finished(r, i)) other = r, n++;
                 if (n != 1 || phase[i] == 1 || phase[other] != phase[i] || tasks[other].level >= t.level) continue;
                 pick = k;
                 o.b2 = wrote[other].first, o.vb2 = wrote[other].second;
@@ -577,6 +581,10 @@ inline ProjPlan finish_plan(const ProjBuilder &g, int inputs, const std::vector<
         place(t.d0, o.d0, o.w0);
         wrote[i] = {o.d0, o.w0};
         if (t.d1 >= 0) place(t.d1, o.d1, o.w1);
+        if (phase[i] == 1) {
+            for (size_t k = 0; k < words; k++) produced[k] |= above[i][k];
+            produced[(size_t)i / 64] |= 1ull << (i % 64);
+        }
         if (t.op == PROJ_MUL) {
             o.prog = (uint16_t)P.scalars.size();
             Fr s;
