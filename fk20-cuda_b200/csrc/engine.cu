@@ -1111,15 +1111,18 @@ int run_points(fk20_ctx *ctx, PlanKind kind, g1p_t *out, const g1p_t *in, int lo
         return run_stages(ctx, PLAN_DFT, out, out, log_m, rows, 0, st);
     }
     if (rc) return rc;
-    for (unsigned r0 = 0; r0 < rows; r0 += pass) {
-        const unsigned n = std::min(rows - r0, pass);
+    // a pass reads its rows before it writes any; where the output lies over later rows
+    // of the input, the last pass comes first
+    const unsigned passes = (rows + pass - 1) / pass;
+    for (unsigned p = 0; p < passes; p++) {
+        const unsigned r0 = (out > in ? passes - 1 - p : p) * pass, n = std::min(rows - r0, pass);
         SegLayout lay;
         lay.arena[0] = arena(n);
         lay.d_off[0] = lay.r_off[0] = 0;
         lay.r_bytes = ready_bytes(lay.arena[0]);
         launch_ref_to_arena((uint4 *)ws.D.p, lay.arena[0], (const uint64_t *)(in + r0 * m), (int)n, log_m, two, st);
         CKL();
-        CKR(run_plan(ctx, ws, lay, &log_m, &n, 1, kind, r0 == 0, 0, st));
+        CKR(run_plan(ctx, ws, lay, &log_m, &n, 1, kind, p == 0, 0, st));
         const TileView v{(const uint4 *)ws.D.p, d.out, lay.arena[0], two, 0};
         launch_tile_to_ref((uint64_t *)(out + r0 * m), v, nullptr, (int)n, log_m, 0, st);
         CKL();

@@ -89,3 +89,21 @@ def test_points_in_passes(engine, ctx, call, rows):
     engine.call(call, engine._ptr(small), engine._ptr(src), DISTINCT, engine._stream())
     engine.call(call, engine._ptr(large), engine._ptr(large), rows, engine._stream())
     assert torch.equal(small[index], large)
+
+
+@pytest.mark.parametrize("shift", [-3, 3])
+def test_points_over_a_shifted_input(engine, ctx, shift):
+    """Output and input share a buffer, the output some rows before or behind."""
+    import torch
+    rows, k = 1060, DISTINCT * 512
+    gen = engine.to_device(np.repeat(O.g1_generator().reshape(1, 18), k, 0))
+    src, small = words(engine.empty((DISTINCT, 512, 18))), words(engine.empty((DISTINCT, 512, 18)))
+    scal = engine.to_device(O.seeded_fr(10, k))
+    engine.call("g1p_op_n", engine.G1_OPS["mul"], engine._ptr(src), engine._ptr(gen), engine._ptr(scal), k, engine._stream())
+    engine.call("g1p_fft", engine._ptr(small), engine._ptr(src), DISTINCT, engine._stream())
+    index = torch.arange(rows, device="cuda") % DISTINCT
+    buf = torch.zeros((rows + 3, 512, 18), dtype=torch.int64, device="cuda")
+    a, b = buf[max(0, -shift):][:rows], buf[max(0, shift):][:rows]
+    a.copy_(src[index])
+    engine.call("g1p_fft", engine._ptr(b), engine._ptr(a), rows, engine._stream())
+    assert torch.equal(small[index], b)
