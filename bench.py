@@ -396,7 +396,7 @@ def run_ours(args, ws, rank, dev):
     all_prod = sum(prof_exe.values())
     launches = sum(v[1] for v in prof.values())
     roofline = {
-        "bound": "imad", "kernel": f"k_g1_stage ({kind})" if kind.startswith("stage") else kind,
+        "bound": "imad", "kernel": f"k_proj ({kind})" if kind.startswith("stage") or kind == "middle" else kind,
         "achieved": achieved / 1e9, "peak": peak_products / 1e9, "unit": "Gprod/s",
         "frac": achieved / peak_products, "traffic": traffic_from_profiles(kind),
         "peak_source": "measured live: fk20_bench_imad (8 independent IMAD chains/thread), IMAD/s / 2",

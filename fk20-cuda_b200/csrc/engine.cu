@@ -592,20 +592,25 @@ Work msm_products(int W, int log_m, bool times_m) {
 // One row of a plan.  Algorithmically the radix-2 transforms it stands for
 // (projection: inverse DIF stages 0..L-2, last inverse butterfly + zeroing +
 // first forward one, forward DIT stages 1..L-1); executed, the plan's products
-// and additions (for a projection, of two instances).
-Work plan_products(PlanKind kind, int log_m) {
-    Work w;
+// and additions (for a projection, of two instances).  One phase of it (0: before
+// the products, 1: the products, 2: after) has its executed share of both.
+Work plan_products(PlanKind kind, int log_m, int phase = -1) {
+    double alg = 0;
     const bool proj = kind == PLAN_PROJ || kind == PLAN_PROJ_HALF;
     if (proj) {
-        for (int s = 0; s < log_m - 1; s++) w += stage_products(1, log_m, s, 0) + stage_products(1, log_m, s + 1, 1);
-        w += Work(ADD_P) * (double)(1 << (log_m - 1));
+        for (int s = 0; s < log_m - 1; s++)
+            alg += (stage_products(1, log_m, s, 0) + stage_products(1, log_m, s + 1, 1)).alg;
+        alg += ADD_P * (double)(1 << (log_m - 1));
     } else {
-        for (int s = 0; s < log_m; s++) w += stage_products(1, log_m, s, kind == PLAN_IDFT ? 0 : 1);
+        for (int s = 0; s < log_m; s++) alg += stage_products(1, log_m, s, kind == PLAN_IDFT ? 0 : 1).alg;
     }
     const HostPlan &h = host_plan(kind, log_m);
-    w.exe = (proj ? 2 : 1) * (h.programs * (37.0 * MP + 16.0 * MS_X) + (h.alg_dbl - h.programs) * (2 * MP + 5 * MS_X) +
-                              (h.alg_add - 3 * h.programs) * (8 * MP + 3 * MS_X) + h.plan.lin_products * MP);
-    return w;
+    double exe[3], all = 0;
+    for (int k = 0; k < 3; k++) exe[k] = h.plan.lin_products[k] * MP;
+    exe[1] += h.programs * (37.0 * MP + 16.0 * MS_X) + (h.alg_dbl - h.programs) * (2 * MP + 5 * MS_X) +
+              (h.alg_add - 3 * h.programs) * (8 * MP + 3 * MS_X);
+    for (double &x : exe) x *= proj ? 2 : 1, all += x;
+    return phase < 0 ? Work(alg, all) : Work(alg * exe[phase] / all, exe[phase]);
 }
 
 size_t arena_bytes(const ProjArena &a) { return (size_t)a.G * a.slots * TILE_Q * 32 * sizeof(uint4); }
@@ -847,22 +852,32 @@ int run_plan(fk20_ctx *ctx, Workspace &ws, const SegLayout &lay, const int *log_
         CK(cudaMemsetAsync(ws.sync.p, 0, 128, st));
         CK(cudaMemsetAsync((char *)ws.sync.p + SYNC_HDR, 0, lay.r_bytes, st));
     }
-    ctx->prof.begin(FK20_K_FFT_FUSED, prod.alg, prod.exe, st);
     if (ctx->fused_fft) {
         p.first = 0;
         p.last = p.runs.total;
+        ctx->prof.begin(FK20_K_FFT_FUSED, prod.alg, prod.exe, st);
         launch_proj(p, blocks(p.runs.total), st);
+        ctx->prof.end(st);
         CKL();
-    } else {
-        for (int r = 0; r < p.runs.n; r++) {
-            p.first = p.runs.run[r].start;
-            p.last = r + 1 < p.runs.n ? p.runs.run[r + 1].start : p.runs.total;
-            CK(cudaMemsetAsync(p.next, 0, sizeof(unsigned), st));
-            launch_proj(p, blocks(p.last - p.first), st);
-            CKL();
-        }
+        return 0;
     }
-    ctx->prof.end(st);
+    double tasks[MAX_PROJ_SEGS][3] = {};  // of a phase, all groups
+    for (int k = 0; k < nseg; k++)
+        for (const ProjLevel &l : plans[k]->levels) tasks[k][l.phase] += (double)l.count * G[k];
+    for (int r = 0; r < p.runs.n; r++) {
+        const ProjRun &run = p.runs.run[r];
+        p.first = run.start;
+        p.last = r + 1 < p.runs.n ? p.runs.run[r + 1].start : p.runs.total;
+        CK(cudaMemsetAsync(p.next, 0, sizeof(unsigned), st));
+        const int phase = plans[run.seg]->tasks[run.first].phase;
+        Work w;
+        if (ctx->prof.on)
+            w = plan_products(kind, log_m[run.seg], phase) * (rows[run.seg] * (double)(p.last - p.first) / tasks[run.seg][phase]);
+        ctx->prof.begin(phase == 0 ? FK20_K_STAGE_INV : phase == 1 ? FK20_K_MIDDLE : FK20_K_STAGE_FWD, w.alg, w.exe, st);
+        launch_proj(p, blocks(p.last - p.first), st);
+        ctx->prof.end(st);
+        CKL();
+    }
     return 0;
 }
 

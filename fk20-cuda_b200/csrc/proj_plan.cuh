@@ -52,7 +52,7 @@ struct ProjPlan {
     std::vector<ProjLevel> levels;
     std::vector<uint32_t> out;                                // output k: slot | neg << 16 | phi << 17
     std::vector<std::array<uint64_t, 4>> scalars;             // the products' constants (standard form)
-    double lin_products = 0;                                  // Fp products of the additions and doublings
+    double lin_products[3] = {0, 0, 0};                       // Fp products of a phase's additions and doublings
 };
 
 namespace host {
@@ -593,7 +593,7 @@ inline ProjPlan finish_plan(const ProjBuilder &g, int inputs, const std::vector<
             for (int q = 0; q < 4; q++) k[q] = (uint64_t)s.w[2 * q] | ((uint64_t)s.w[2 * q + 1] << 32);
             P.scalars.push_back(k);
         } else {
-            P.lin_products += 8.0 * t.sh + (t.phi ? 1 : 0) + (t.op == PROJ_SHL ? 0 : t.d1 >= 0 ? 18 : 12);
+            P.lin_products[phase[i]] += 8.0 * t.sh + (t.phi ? 1 : 0) + (t.op == PROJ_SHL ? 0 : t.d1 >= 0 ? 18 : 12);
         }
         const int ph = phase[i], lv = ph == 1 ? 0 : t.level;
         o.phase = (uint8_t)ph;

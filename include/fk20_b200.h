@@ -190,11 +190,12 @@ size_t fk20_ctx_device_bytes(const fk20_ctx *ctx);
  * additions of 8 M + 2 S, Jacobian twiddle programs on an isomorphic curve). */
 #define FK20_K_TC_FFT 0    /* toeplitz + Fr FFTs */
 #define FK20_K_MSM 1       /* fixed-base MSM */
-#define FK20_K_STAGE_INV 2 /* inverse G1 FFT stages */
-#define FK20_K_STAGE_FWD 3 /* forward G1 FFT stages */
-#define FK20_K_MIDDLE 4    /* last inverse + zeroing + first forward stage */
+/* the map from hext_fft to h_fft, with FK20_OPT_FUSED_FFT 0 a launch per level of tasks: */
+#define FK20_K_STAGE_INV 2 /* additions before the fixed-scalar products */
+#define FK20_K_STAGE_FWD 3 /* additions after them */
+#define FK20_K_MIDDLE 4    /* the products */
 #define FK20_K_OUTPUT 5    /* tiles -> reference g1p_t */
-#define FK20_K_FFT_FUSED 6 /* all G1 FFT stages in one persistent launch */
+#define FK20_K_FFT_FUSED 6 /* the same map in one persistent launch */
 #define FK20_NKINDS 7
 int fk20_ctx_profile(fk20_ctx *ctx, int enable);
 int fk20_ctx_profile_read(fk20_ctx *ctx, int kind, double *ms, long *launches, double *products);

@@ -450,3 +450,28 @@ def test_bounded_wait_reports_timeout_and_context_recovers(engine):
     torch.cuda.synchronize()
     assert torch.equal(again, good)
     c.close()
+
+
+def test_profiler_kinds_of_the_unfused_map(engine):
+    """With FK20_OPT_FUSED_FFT 0 the three phases of the map have a kind each, and
+    together the fused launch's work."""
+    n, rows = 1024, 40
+    c = engine.Context(0, 8)
+    c.load_xext_fft(n, engine.to_device(fk20_setup_data(n)[2]))
+    poly = engine.to_device(O.seeded_fr(8900, rows * n).reshape(rows, n, 4))
+    h = engine.empty((rows, n // 8, 18))
+    work = {}
+    for fused in (1, 0):
+        c.set(engine.FK20_OPT_FUSED_FFT, fused)
+        c.profile(True)
+        c.poly2h_fft(h, poly, rows, n)
+        alg, exe = c.profile_read(), c.profile_read_executed()
+        c.profile(False)
+        kinds = ("fft_fused",) if fused else ("stage_inv", "middle", "stage_fwd")
+        for k in ("stage_inv", "middle", "stage_fwd", "fft_fused"):
+            assert (alg[k][1] > 0) == (k in kinds) == (exe[k] > 0)
+        work[fused] = sum(alg[k][2] for k in kinds), sum(exe[k] for k in kinds)
+        if not fused:
+            assert exe["middle"] > max(exe["stage_inv"], exe["stage_fwd"]) and all(alg[k][0] > 0 for k in kinds)
+    assert work[0] == pytest.approx(work[1], rel=1e-9)
+    c.close()
