@@ -2285,12 +2285,16 @@ void server_main(fk20_server *s) {
                 // they are given back first
                 bool held = false;
                 if (!busy)
+                    for (Slot &sl : s->slots) held |= sl.bytes() > 0;
+                if (held) {
+                    lk.unlock();  // submit must not wait on the driver; only this thread touches the slots
                     for (Slot &sl : s->slots) {
-                        held |= sl.bytes() > 0;
                         sl.ws.D.release(), sl.ws.offs.release(), sl.ws.sync.release();
                         sl.dpoly.release(), sl.dout.release();
                     }
-                if (held) continue;
+                    lk.lock();
+                    continue;
+                }
                 if (!busy) {
                     s->finished[s->queue.front().ticket] = FK20_ENOMEM;
                     s->nomem++;
