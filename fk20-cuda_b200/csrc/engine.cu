@@ -1638,8 +1638,11 @@ int autotune(fk20_ctx *ctx, int log_m, unsigned rows, size_t max_table_bytes, fk
     // 2. MSM block size, 3. persistent FFT grid, 4. fused vs staged FFT
     for (int t : {64, 128, 256})
         if (!rc && t != best.threads) rc = consider(Cfg{best.window, t, best.bps, best.fused});
+    // (a default of 0 is the grid that a call of these rows would take)
+    const double products = (double)host_plan(PLAN_PROJ, log_m).plan.muls * proj_arena(0, std::min(rows, PASS_ROWS)).G;
+    const int by_count = proj_grid(products, ctx->sms, ctx->proj_occupancy);
     for (int b = 1; b <= ctx->proj_occupancy && !rc; b++)
-        if (b != (best.bps ? best.bps : ctx->proj_occupancy)) rc = consider(Cfg{best.window, best.threads, b, 1});
+        if (b != (best.bps ? best.bps : by_count)) rc = consider(Cfg{best.window, best.threads, b, 1});
     if (!rc) rc = consider(Cfg{best.window, best.threads, best.bps, best.fused ? 0 : 1});
     apply(best);
     cudaStreamSynchronize(st);
