@@ -58,18 +58,62 @@ struct ProjPlan {
 namespace host {
 
 // ---------------------------------------------------------------- Fr on the host
+// The Montgomery product in 64-bit words.  A plan of 512 points takes some 550,000
+// products, and the 32-bit form, written for the GPU, 0.3 us each on a host core: the
+// first hext_fft -> h_fft of a process waited 0.29 s for its plan, now 0.06, its first
+// transform of 512 points 0.16 and 0.09 s.
+inline Fr operator*(const Fr &a, const Fr &b) {
+    using u128 = unsigned __int128;
+    const auto word = [](const uint32_t *w, int i) { return (uint64_t)w[2 * i] | (uint64_t)w[2 * i + 1] << 32; };
+    constexpr auto mod = [](int i) { return (uint64_t)FrDesc::mod(2 * i) | (uint64_t)FrDesc::mod(2 * i + 1) << 32; };
+    constexpr uint64_t m[4] = {mod(0), mod(1), mod(2), mod(3)};
+    constexpr uint64_t inv = [](uint64_t m0) {  // 1 / m mod 2^64, by Newton's iteration: 1, 2, 4, .. 64 bits
+        uint64_t v = 1;
+        for (int k = 0; k < 6; k++) v *= 2 - m0 * v;
+        return v;
+    }(m[0]);
+    uint64_t t[5] = {0, 0, 0, 0, 0};
+    for (int i = 0; i < 4; i++) {
+        const uint64_t bi = word(b.w, i);
+        u128 c = 0;
+        for (int j = 0; j < 4; j++) {
+            c += (u128)word(a.w, j) * bi + t[j];
+            t[j] = (uint64_t)c;
+            c >>= 64;
+        }
+        c += t[4];
+        t[4] = (uint64_t)c;  // t < 2^256 + 2^319 (a, m < 2^255): five words hold it, and q m too
+        const uint64_t q = 0 - t[0] * inv;
+        c = (u128)q * m[0] + t[0];
+        c >>= 64;
+        for (int j = 1; j < 4; j++) {
+            c += (u128)q * m[j] + t[j];
+            t[j - 1] = (uint64_t)c;
+            c >>= 64;
+        }
+        c += t[4];
+        t[3] = (uint64_t)c;
+        t[4] = (uint64_t)(c >> 64);
+    }
+    Fr s, r;
+    for (int i = 0; i < 4; i++) s.w[2 * i] = (uint32_t)t[i], s.w[2 * i + 1] = (uint32_t)(t[i] >> 32);
+    f_reduce_once<FrDesc>(r.w, s.w);  // t < 2 m < 2^256
+    return r;
+}
+inline Fr fr_mont(const Fr &a) {  // standard form -> Montgomery form
+    Fr r2;
+    for (int i = 0; i < 8; i++) r2.w[i] = FrDesc::r2(i);
+    return a * r2;
+}
 inline Fr fr_from_u64(uint64_t v) {
-    Fr t, r;
+    Fr t;
     f_set_zero(t);
     t.w[0] = (uint32_t)v;
     t.w[1] = (uint32_t)(v >> 32);
-    f_to_mont(r, t);
-    return r;
+    return v ? fr_mont(t) : t;
 }
-inline Fr operator*(const Fr &a, const Fr &b) { Fr r; f_mul(r, a, b); return r; }
 inline Fr operator+(const Fr &a, const Fr &b) { Fr r; f_add(r, a, b); return r; }
 inline Fr operator-(const Fr &a, const Fr &b) { Fr r; f_sub(r, a, b); return r; }
-inline Fr fr_inv(const Fr &a) { Fr r; f_inv(r, a); return r; }
 inline Fr fr_pow(const Fr &a, unsigned e) {
     Fr r;
     f_set_one(r);
@@ -80,17 +124,31 @@ inline Fr fr_pow(const Fr &a, unsigned e) {
     }
     return r;
 }
+inline Fr fr_pow(const Fr &a, const uint32_t e[8]) {
+    Fr v;
+    f_set_one(v);
+    for (int i = 254; i >= 0; i--) {
+        v = v * v;
+        if ((e[i >> 5] >> (i & 31)) & 1) v = v * a;
+    }
+    return v;
+}
+inline Fr fr_inv(const Fr &a) {  // a^(r - 2)
+    uint32_t e[8];
+    for (int i = 0; i < 8; i++) e[i] = FrDesc::mod(i);
+    e[0] -= 2, e[1] -= 1;  // r's low word is 1
+    return fr_pow(a, e);
+}
 inline int log2_of(int v) {
     int l = 0;
     while ((1 << l) < v) l++;
     return l;
 }
 inline Fr fr_lambda() {  // z^2 - 1
-    Fr t, r;
+    Fr t;
     f_set_zero(t);
     t.w[0] = 0xffffffffu, t.w[1] = 0, t.w[2] = 0x0001a402u, t.w[3] = 0xac45a401u;
-    f_to_mont(r, t);
-    return r;
+    return fr_mont(t);
 }
 inline Fr fr_root(int log_order) {  // 5^((r-1) / 2^log_order)
     uint32_t e[8];
@@ -98,9 +156,7 @@ inline Fr fr_root(int log_order) {  // 5^((r-1) / 2^log_order)
     e[0] -= 1;
     for (int k = 0; k < log_order; k++)
         for (int i = 0; i < 8; i++) e[i] = (e[i] >> 1) | (i < 7 ? e[i + 1] << 31 : 0);
-    Fr r;
-    f_pow(r, fr_from_u64(5), e, 8);
-    return r;
+    return fr_pow(fr_from_u64(5), e);
 }
 
 // ---------------------------------------------------------------- evaluation points
