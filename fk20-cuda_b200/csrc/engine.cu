@@ -618,7 +618,8 @@ size_t ready_bytes(const ProjArena &a) { return (size_t)a.G * (a.slots + 1) * si
 
 int output_launch(Profiler &pf, uint64_t *dst, const TileView &D, const size_t *row_off, int rows, int log_m,
                   int bitrev_out, cudaStream_t st) {
-    pf.begin(FK20_K_OUTPUT, (double)rows * (1 << log_m) * 3 * MP, (double)rows * (1 << log_m) * 3 * MP, st);
+    const double out = (double)rows * (1 << log_m) * 5 * MP;  // two products to affine, three conversions
+    pf.begin(FK20_K_OUTPUT, out, out, st);
     launch_tile_to_ref(dst, D, row_off, rows, log_m, bitrev_out, st);
     pf.end(st);
     CKL();
@@ -717,9 +718,9 @@ struct Seg {
 };
 
 constexpr size_t SYNC_HDR = 256;  // persistent-launch header: task counter at 0, error flag at 128
-// Fp products per compressed proof: inversion by Fermat (381 squarings + 190
-// products), two products to affine, two conversions out of Montgomery form
-constexpr double PROOF_OUT_MP = 575.0;
+// Fp products per compressed proof: two to affine, two conversions out of
+// Montgomery form (the inversion is division steps: additions and shifts)
+constexpr double PROOF_OUT_MP = 4.0;
 
 // Arena slots of the pipeline's plan: the scalar tiles of a row group lie
 // behind the input slots of its (first) group, where nothing is written

@@ -441,8 +441,7 @@ void launch_commit(uint64_t *out, uint4 *part, const uint64_t *poly, const uint4
 // would only add sums.  B200, window 10, MSM alone, before (a row per lane, a
 // warp per unit) and after: 1 row of 4096 4.41 -> 0.21 ms, 19 of 2048 4.64 ->
 // 1.33, 160 of 4096 15.1 -> 13.5; at 512 rows of 4096 (4.6 waves) splitting
-// costs 1 %, 40.7 -> 41.1, hence the line at 4 waves.  48 commitments of 4096:
-// 10.5 -> 3.0 ms, most of it the partial sums, which one thread per row added.
+// costs 1 %, 40.7 -> 41.1, hence the line at 4 waves.
 void launch_msm(const MsmArgs &in, int threads, int sms, cudaStream_t st) {
     if (threads != 64 && threads != 128 && threads != 256) threads = 128;
     if (threads > MSM_MAX_THREADS) threads = MSM_MAX_THREADS;

@@ -735,7 +735,7 @@ __global__ void __launch_bounds__(32 * PV_WARPS) k_verify_points_warp(uint64_t *
 // a P with a part outside the order-r subgroup the two halves differ from
 // [k] P by a point of the cofactor's order, which the pairing does not see.
 // The element-wise product's 256 doublings and ~128 additions are 2.5 times as
-// deep.  With the warp kernels of this file, 300 checks 40.6 -> 5.2 ms.
+// deep.  With the warp kernels of this file, 300 checks 40.6 -> 3.9 ms.
 __global__ void __launch_bounds__(64) k_verify_points(uint64_t *out, const uint64_t *C, const uint64_t *I,
                                                       const uint64_t *P, const uint64_t *k, size_t count) {
     const size_t i = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 1;

@@ -17,9 +17,9 @@
 // Bound by the integer multiply pipe, as the butterflies it replaces, with
 // about half their products; a small batch is bound by the depth, one product
 // (~1,300 dependent Fp products) and ~35 additions instead of 14-16 products.
-// Measured against the persistent radix-2 FFT over whole calls (MSM included):
-// one blob of 4096 34.8 -> 9.3 ms, 160 blobs 68.6 -> 44.2, 512 blobs at window
-// 13 172.8 -> 116.1.
+// Whole calls (MSM included, whose own cuts and products became faster too) with
+// the persistent radix-2 FFT and now: one blob of 4096 34.8 and 3.2 ms, 160 blobs
+// 68.6 and 31.5, 512 blobs at window 13 172.8 and 86.0.
 #define FK_FP_MUL_OUTLINE 1
 #include "../../include/fk20_b200.h"
 #include "check.cuh"
@@ -103,7 +103,9 @@ FK_D void proj_stop(const ProjArgs &P, int code) {
 
 // Six blocks (12 warps) an SM, 168 registers: with three warps a scheduler the
 // pipe stays busier than with two (512 blobs of 4096: 54.7 ms at 228 registers
-// and four blocks, 52.6 here); small launches use fewer of them (proj_grid).
+// and four blocks, 52.6 here); small launches use fewer of them (proj_grid).  What
+// 168 registers spill (524 bytes stored, 800 loaded a thread) is 0.14 % of the
+// instructions.
 __global__ void __launch_bounds__(FFT_THREADS, 6) k_proj(const __grid_constant__ ProjArgs P) {
     __shared__ uint32_t slots[PROG_POINT_WORDS][FFT_THREADS];
     const int lane = threadIdx.x & 31;

@@ -844,7 +844,7 @@ inline std::vector<ProjRef> odd_sums(ProjBuilder &g, const std::vector<ProjRef> 
 // in slot j, output k in out[k].  1,388 products at m = 512 (the inverse 1,398,
 // its factor on every product and on the few values that meet none), one deep;
 // radix 2 takes 1,793 (2,305), nine (ten) deep.  B200: 32 inverse transforms of
-// 512 points 12.8 -> 4.9 ms.
+// 512 points by stages 12.6 ms, by plan 4.3.
 inline ProjPlan build_dft_plan(int log_m, bool inverse) {
     const int m = 1 << log_m;
     ProjBuilder g;
