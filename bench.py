@@ -64,7 +64,7 @@ def parse():
     ap.add_argument("--serve-max-rows", type=int, default=160)
     ap.add_argument("--serve-slots", type=int, default=2)
     ap.add_argument("--serve-fft-blocks", type=int, default=0,
-                    help="persistent-FFT blocks per SM of each pack (0: adaptive to the backlog)")
+                    help="blocks per SM of each pack's persistent launch (0: by its number of products)")
     ap.add_argument("--serve-engine", type=int, default=0,
                     help="server engine: 0 packs on slots, 1 cohorts (continuous batching at FFT-stage granularity)")
     ap.add_argument("--serve-cohort-rows", type=int, default=0, help="engine 1: rows per cohort (0 = 64)")

@@ -100,7 +100,7 @@ int fk20_ctx_msm(fk20_ctx *ctx, g1p_t *hext_fft, const fr_t *tc_fft, unsigned ro
  * All offset arrays are HOST arrays (read before the call returns).  The
  * instances are grouped into one segment per length, and all segments run in
  * ONE fixed-base MSM launch and ONE persistent launch of the map from hext_fft
- * to h_fft.
+ * to h_fft; more than 1024 instances of a length run in passes of that many.
  * No reference counterpart (the reference proves one length per call). */
 int fk20_ctx_batch(fk20_ctx *ctx, g1p_t *h_fft, const fr_t *polys, unsigned count, const unsigned *n,
                    const size_t *poly_off, const size_t *out_off, void *stream);

@@ -27,9 +27,9 @@ def served_ctx(engine):
                          ids=["adaptive", "latency-rows-4", "one-fft-block-per-sm", "cohorts",
                               "cohorts-1-stage-per-launch", "cohorts-whole-fft-per-launch"])
 def test_server_results_same_alone_and_in_the_mix(engine, served_ctx, mode):
-    """Latency-mode packs (the whole queue, the whole GPU) and throughput-mode
-    packs (whole 32-row groups, the SMs split between slots) both occur here:
-    bursts of 10 submissions against 16-request packs."""
+    """Bursts of 10 submissions against packs of at most 16 requests on two slots, so
+    that packs overlap with each other and with new arrivals (whole groups of 32:
+    test_server_latency_rows_decides_whole_groups)."""
     rng = np.random.default_rng(5)
     sizes = [int(x) for x in rng.choice([1024, 2048, 4096], 90, p=[0.2, 0.3, 0.5])]
     polys = [O.seeded_fr(4000 + j, n) for j, n in enumerate(sizes)]
