@@ -1253,6 +1253,11 @@ int fk20_default_status(int device) {
 
 int fk20_default_set(int device, int option, int value) {
     if (device < 0 || device >= 64) return FK20_EINVAL;
+    int ndev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || device >= ndev) {
+        cudaGetLastError();
+        return FK20_ENODEV;
+    }
     DeviceGuard dg(device);
     fk20_ctx *c;
     CKR(default_ctx(&c));

@@ -52,6 +52,7 @@ def test_abandoned_transform_is_reported_and_refuses_nothing(engine, call):
     assert lib.fk20_default_status(dev) == 0
     assert lib.fk20_default_status(-1) == engine.FK20_EINVAL
     assert lib.fk20_default_set(dev, 99, 0) == engine.FK20_EINVAL
+    assert lib.fk20_default_set(63, engine.FK20_OPT_FUSED_FFT, 1) == engine.FK20_ENODEV
 
 
 @pytest.mark.parametrize("inverse", [0, 1])
@@ -122,3 +123,21 @@ def test_transforms_without_room_for_their_arena(engine):
             assert torch.equal(run(*c), good), c
     finally:
         lib.fk20_test_fail_allocations(0)
+
+
+@pytest.mark.parametrize("log_m,inverse", [(3, 0), (6, 1), (9, 0)])
+def test_transforms_level_by_level_give_the_same_words(engine, log_m, inverse):
+    """FK20_OPT_FUSED_FFT 0 on the default context: a launch per level, 300 rows in
+    chunks of groups."""
+    import torch
+    dev, lib, m = torch.cuda.current_device(), engine.lib(), 1 << log_m
+    src = engine.to_device(points(70 + log_m, 6 * m).reshape(6, m, 18)).repeat(50, 1, 1)
+    a, b = engine.empty(src.shape), engine.empty(src.shape)
+    try:
+        for fused, out in ((1, a), (0, b)):
+            assert lib.fk20_default_set(dev, engine.FK20_OPT_FUSED_FFT, fused) == 0
+            engine.call("g1p_fft_n", engine._ptr(out), engine._ptr(src), log_m, 300, inverse, engine._stream())
+    finally:
+        lib.fk20_default_set(dev, engine.FK20_OPT_FUSED_FFT, 1)
+    assert lib.fk20_default_status(dev) == 0
+    assert torch.equal(a, b)
