@@ -710,11 +710,12 @@ int msm_launch(fk20_ctx *ctx, Tables *T, uint4 *D, const uint4 *S, int G, int ro
 // One segment of a pipeline call: `rows` polynomials of length n = 8m
 // (m = 2^log_m); polynomial r starts at word 4 * poly_off[r] of the input and
 // its outputs at word 18 * out_off[r] of the output (device arrays; null =
-// contiguous rows).
+// contiguous rows).  The offsets lie in [in_lo, in_hi) and [out_lo, out_hi).
 struct Seg {
     int log_m;
     unsigned rows;
     const size_t *poly_off, *out_off;
+    size_t in_lo = 0, in_hi = 0, out_lo = 0, out_hi = 0;
 };
 
 constexpr size_t SYNC_HDR = 256;  // persistent-launch header: task counter at 0, error flag at 128
@@ -777,15 +778,33 @@ bool device_has(size_t need) {
     return fr >= need + ((size_t)64 << 20);
 }
 
+// A pass reads its rows' coefficients before it writes any output.  True if an
+// output would be written over coefficients that a later pass reads: all rows then
+// go in one pass.  (Contiguous outputs that begin at or before the coefficients
+// stay behind them, a row of outputs being the shorter one.)
+bool output_over_input(const Seg *sg, int nseg, const fr_t *polys, const void *out, size_t point) {
+    const uintptr_t in0 = (uintptr_t)polys, out0 = (uintptr_t)out;
+    for (int a = 0; a < nseg; a++)
+        for (int b = 0; b < nseg; b++) {
+            const bool rows = !sg[a].poly_off;  // contiguous: the only segment
+            const size_t n = (size_t)L_COLS / 2 << sg[a].log_m, m = (size_t)1 << sg[b].log_m;
+            const uintptr_t ilo = in0 + sg[a].in_lo * sizeof(fr_t), olo = out0 + sg[b].out_lo * point;
+            const uintptr_t ihi = in0 + (rows ? sg[a].rows * n : sg[a].in_hi) * sizeof(fr_t);
+            const uintptr_t ohi = out0 + (rows ? sg[b].rows * m : sg[b].out_hi) * point;
+            if (ilo < ohi && olo < ihi && !(rows && olo <= ilo)) return true;
+        }
+    return false;
+}
+
 // Device buffers of a segment call (a no-op once they are large enough), and the
-// rows of a pass that they hold: PASS_ROWS, or where the device has no room for
-// that arena half of it and so on down to 16, whose arena is no larger than the
-// point and scalar tiles of one group of 32 rows.
-int reserve_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, bool full, unsigned *pass) {
+// rows of a pass that they hold: all (one_pass), or PASS_ROWS, or where the device
+// has no room for that arena half of it and so on down to 16, whose arena is no
+// larger than the point and scalar tiles of one group of 32 rows.
+int reserve_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, bool full, bool one_pass, unsigned *pass) {
     Seg part[MAX_PROJ_SEGS];
     if (nseg < 1 || nseg > MAX_PROJ_SEGS) return FK20_EINVAL;
     CKR(ws.init());
-    for (*pass = PASS_ROWS;; *pass /= 2) {
+    for (*pass = one_pass ? MAX_ROWS / 2 : PASS_ROWS;; *pass /= 2) {
         SegLayout lay;
         for (int k = 0; k < nseg; k++) part[k] = sg[k], part[k].rows = std::min(sg[k].rows, *pass);
         CKR(segment_layout(ctx, part, nseg, full, lay));
@@ -795,7 +814,7 @@ int reserve_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, bool
         }
         int rc = ws.D.reserve(lay.d_bytes);
         if (!rc) rc = ws.sync.reserve(SYNC_HDR + lay.r_bytes);
-        if (rc != FK20_ENOMEM || *pass <= 16 || device_has(lay.d_bytes + lay.r_bytes)) return rc;
+        if (rc != FK20_ENOMEM || one_pass || *pass <= 16 || device_has(lay.d_bytes + lay.r_bytes)) return rc;
     }
 }
 
@@ -956,7 +975,8 @@ int run_pass(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, const fr_t *
 int run_segments(fk20_ctx *ctx, Workspace &ws, const Seg *sg, int nseg, const fr_t *polys, void *out, bool full,
                  cudaStream_t st, bool proofs = false, int fft_bps = 0) {
     unsigned pass = 0;
-    CKR(reserve_segments(ctx, ws, sg, nseg, full, &pass));
+    const bool one_pass = output_over_input(sg, nseg, polys, out, proofs ? 48 : sizeof(g1p_t));
+    CKR(reserve_segments(ctx, ws, sg, nseg, full, one_pass, &pass));
     if (*ws.err_host) return launch_error(*ws.err_host);  // a previous persistent launch stopped: results invalid
     unsigned most = 0;
     for (int k = 0; k < nseg; k++) most = std::max(most, sg[k].rows);
@@ -991,13 +1011,18 @@ int batch_segments(fk20_ctx *ctx, Workspace &ws, unsigned count, const unsigned 
     CKR(ws.stage_offsets(2 * (size_t)count));
     size_t *h = ws.offs_host;
     size_t at = 0;
-    struct Part { int log_m; size_t first; unsigned rows; } parts[3];
+    struct Part { int log_m; size_t first; unsigned rows; size_t in_lo = ~(size_t)0, in_hi = 0, out_lo = ~(size_t)0, out_hi = 0; } parts[3];
     int np = 0;
     for (int log_m = 9; log_m >= 7; log_m--) {
         const unsigned nn = (unsigned)(L_COLS << (log_m - 1));
         Part pt{log_m, at, 0};
         for (unsigned j = 0; j < count; j++)
-            if (n[j] == nn) { h[at++] = poly_off[j]; pt.rows++; }
+            if (n[j] == nn) {
+                h[at++] = poly_off[j];
+                pt.rows++;
+                pt.in_lo = std::min(pt.in_lo, poly_off[j]), pt.in_hi = std::max(pt.in_hi, poly_off[j] + nn);
+                pt.out_lo = std::min(pt.out_lo, out_off[j]), pt.out_hi = std::max(pt.out_hi, out_off[j] + nn / 8);
+            }
         for (unsigned j = 0; j < count; j++)
             if (n[j] == nn) h[at++] = out_off[j];
         if (pt.rows) {
@@ -1010,7 +1035,8 @@ int batch_segments(fk20_ctx *ctx, Workspace &ws, unsigned count, const unsigned 
     CK(cudaEventRecord(ws.offs_done, st));
     const size_t *d = (const size_t *)ws.offs.p;
     for (int k = 0; k < np; k++)
-        sg[k] = Seg{parts[k].log_m, parts[k].rows, d + parts[k].first, d + parts[k].first + parts[k].rows};
+        sg[k] = Seg{parts[k].log_m, parts[k].rows, d + parts[k].first, d + parts[k].first + parts[k].rows,
+                    parts[k].in_lo, parts[k].in_hi, parts[k].out_lo, parts[k].out_hi};
     *nseg = np;
     return 0;
 }
@@ -1456,7 +1482,7 @@ namespace {
 int capture_plan(fk20_plan *plan, g1p_t *h_fft, const fr_t *polys, const Seg *sg, int nseg) {
     fk20_ctx *ctx = plan->ctx;
     unsigned pass = 0;
-    CKR(reserve_segments(ctx, plan->ws, sg, nseg, true, &pass));
+    CKR(reserve_segments(ctx, plan->ws, sg, nseg, true, output_over_input(sg, nseg, polys, h_fft, sizeof(g1p_t)), &pass));
     const bool prof_on = ctx->prof.on;
     ctx->prof.on = false;  // timing events cannot be replayed
     CK(cudaStreamBeginCapture(plan->capture, cudaStreamCaptureModeThreadLocal));

@@ -107,3 +107,24 @@ def test_points_over_a_shifted_input(engine, ctx, shift):
     a.copy_(src[index])
     engine.call("g1p_fft", engine._ptr(b), engine._ptr(a), rows, engine._stream())
     assert torch.equal(small[index], b)
+
+
+@pytest.mark.parametrize("shape", ["rows behind", "rows at the start", "ragged"])
+def test_proofs_over_their_coefficients(engine, ctx, shape):
+    """1,060 rows' proofs written into the buffer of the coefficients."""
+    import torch
+    n, rows, m = 1024, 1060, 128
+    base = words(engine.to_device(O.seeded_fr(777, DISTINCT * n).reshape(DISTINCT, n, 4)))
+    small = forms(engine, ctx, base, DISTINCT, n)[0]
+    index = torch.arange(rows, device="cuda") % DISTINCT
+    buf = base[index].reshape(-1).clone()
+    at = {"rows behind": buf.numel() - rows * m * 18, "rows at the start": 0, "ragged": 18 * m}[shape]
+    at -= at % 18
+    out = buf[at:at + rows * m * 18].reshape(rows, m, 18)
+    if shape == "ragged":
+        order = list(range(rows))[::-1]  # of coefficients and proofs alike
+        ctx.batch(buf, buf, [n] * rows, [r * n for r in order], [at // 18 + r * m for r in order])
+    else:
+        ctx.poly2h_fft(out, buf, rows, n)
+    assert ctx.status() == 0
+    assert torch.equal(out, small[index])
